@@ -78,11 +78,12 @@ typedef struct nbx_params {
                              src/cuda/CudaNaive.cu:17-57); no tree is built,
                              use_mlp must be 0 */
   int32_t force_block;    /* threads per block of the default force walk:
-                             128, 256 or 512 (0 = 256) */
-  int32_t leaf_pairs;     /* default force walk: 1 takes a leaf's bodies two
-                             at a time with paired FP32 instructions, 0 one
-                             at a time (default 1); the same terms either
-                             way, summed in another order */
+                             128, 256 or 512 (0 = 128) */
+  int32_t leaf_pairs;     /* default force walk: 1 walks the tree once per
+                             group of 32 bodies and sums the group's terms
+                             with paired FP32 instructions, 0 one record and
+                             one body at a time (default 1); the same terms
+                             either way, summed in another order */
 } nbx_params;
 
 typedef struct nbx_handle nbx_handle;

@@ -227,6 +227,7 @@ struct nbx_handle {
   nbx_params params{};
   uint32_t n = 0, nseg = 0;
   std::vector<uint32_t> segStart, segCount;
+  std::vector<uint32_t> groupFirst; // DevState::groupFirst
   std::vector<void *> allocs;
   DevState base{};       // buffer set A current
   int cur = 0;           // 0: state in set A (pv), 1: in set B (pv2)
@@ -404,10 +405,12 @@ int allocate(nbx_handle *h) {
   A(S.groupStart, (size_t)ns * kLevelSlots);
   A(S.groupEnd, (size_t)ns * kLevelSlots);
   A(S.levelStart, (size_t)ns * (kLevelSlots + 1));
-  A(S.comX, nodes);
-  A(S.comY, nodes);
-  A(S.mass, nodes);
-  A(S.centerX, nodes);
+  // one block: the upward pass of the traversal records uses it as float4s
+  A(S.tUp, nodes);
+  S.comX = reinterpret_cast<float *>(S.tUp);
+  S.comY = S.comX + nodes;
+  S.mass = S.comY + nodes;
+  S.centerX = S.mass + nodes;
   A(S.centerY, nodes);
   A(S.size, nodes);
   A(S.children, nodes);
@@ -422,6 +425,22 @@ int allocate(nbx_handle *h) {
   A(S.arrive, nodes);
   A(S.tN, nodes); // cudaMalloc: 256-byte aligned, so every record is 32
   A(S.tM, nodes);
+  { // written by every build before it is read: not cleared
+    void *v = nullptr;
+    if (cudaError_t e = cudaMalloc(&v, ((size_t)n + ns) * sizeof(QuadRec)))
+      return cuda_fail(h, e, "cudaMalloc S.tQ");
+    h->allocs.push_back(v);
+    S.tQ = static_cast<QuadRec *>(v);
+  }
+  h->groupFirst.clear();
+  S.nGroups = (n + 31) / 32; // one instance: group g starts at 32 g
+  if (ns > 1) {
+    for (uint32_t s = 0; s < ns; ++s)
+      for (uint32_t b = 0; b < h->segCount[s]; b += 32)
+        h->groupFirst.push_back(h->segStart[s] + b);
+    S.nGroups = (uint32_t)h->groupFirst.size();
+    A(S.groupFirst, S.nGroups);
+  }
   // scan / sort scratch
   SortScratch &so = h->sort;
   so.capacity = sortCap;
@@ -450,6 +469,9 @@ int allocate(nbx_handle *h) {
   A(S.attr, 2);
 #undef A
   NBX_CUDA(h, cudaMemcpy(S.attr, h->attrHost, sizeof(h->attrHost), cudaMemcpyHostToDevice));
+  if (!h->groupFirst.empty())
+    NBX_CUDA(h, cudaMemcpy(S.groupFirst, h->groupFirst.data(), S.nGroups * sizeof(uint32_t),
+                           cudaMemcpyHostToDevice));
   // bounds accumulators start empty
   std::vector<uint32_t> b(4 * ns);
   for (uint32_t s = 0; s < ns; ++s) {
@@ -520,16 +542,23 @@ uint32_t io_chunks(const nbx_handle *h) {
 static_assert(sizeof(nbx_body) == 9 * sizeof(uint32_t), "the force pass writes 9-word records");
 void enqueue_forces_io(nbx_handle *h, cudaStream_t s, const DevState &S) {
   const uint32_t n = S.n, chunks = io_chunks(h);
-  const uint32_t per = ((n + chunks - 1) / chunks + 31u) & ~31u;
+  // ranges of whole target groups (DevState::groupFirst)
+  const uint32_t per = (S.nGroups + chunks - 1) / chunks;
+  auto body = [&](uint32_t g) {
+    return g >= S.nGroups ? n : S.nseg == 1 ? g * 32u : h->groupFirst[g];
+  };
   cudaEventRecord(h->ioFork, s);
   for (uint32_t c = 0; c < chunks; ++c) {
-    const uint32_t b = c * per, e = std::min(n, b + per);
-    if (b >= e) break;
+    const uint32_t g0 = c * per, g1 = std::min(S.nGroups, g0 + per);
+    if (g0 >= g1) break;
+    const uint32_t b = body(g0), e = body(g1);
     cudaStream_t cs = h->ioStream[c];
     cudaStreamWaitEvent(cs, h->ioFork, 0);
     DevState R = S;
     R.forceBegin = b;
     R.forceEnd = e;
+    R.tgBegin = g0;
+    R.tgEnd = g1;
     R.recOut = reinterpret_cast<uint32_t *>(h->dAoS);
     launch_forces(cs, R, h->params.exact_math != 0, h->params.force_blocks,
                   h->mlpLoaded ? h->mlpW : nullptr, h->params.mlp_band, h->params.use_mlp,
@@ -2134,9 +2163,9 @@ int nbx_autotune(nbx_handle *h, int allowLeaf, uint32_t steps, nbx_params *best,
     for (int threads : blockShapes)
       for (int pairs : leafWidths) {
         // grids: one warp per 32 bodies, or a half, one or two full SMs'
-        // worth of resident blocks per SM (the paired walk's launch bounds
-        // hold 1536 threads per SM, the single-body walk's 2048)
-        const int perSm = (pairs ? 1536 : 2048) / (threads > 0 ? threads : 256);
+        // worth of resident blocks per SM (the group walk's launch bounds
+        // hold 1024 threads per SM, the single-body walk's 2048)
+        const int perSm = (pairs ? 1024 : 2048) / (threads > 0 ? threads : 128);
         for (int grid : {0, sms * perSm / 2, sms * perSm, sms * perSm * 2})
           trials.push_back({leaf, threads, pairs, grid});
       }

@@ -658,6 +658,43 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
+// Writes record `at` of the default force walk (QuadRec) from the sums, cell
+// and first body of up to four children; returns the link to it.  (px, py):
+// a finite place for absent children.
+__device__ __forceinline__ uint32_t quad_record(const DevState &S, uint32_t at, float px,
+                                                float py, uint32_t children,
+                                                const float4 (&up)[4], const float4 (&ca)[4],
+                                                const int (&first)[4]) {
+  float x[4], y[4], h[4], w[4];
+  uint2 c[4];
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) {
+    const bool have = q < children;
+    x[q] = have ? ca[q].x : px;
+    y[q] = have ? ca[q].y : py;
+    h[q] = have ? 0.5f * ca[q].z : 0.0f;
+    w[q] = have ? up[q].z : 0.0f;
+    c[q] = have ? make_uint2(__float_as_uint(up[q].w), (uint32_t)first[q])
+                : make_uint2(kQuadLeaf, 0u);
+  }
+  QuadRec &Q = S.tQ[at];
+  Q.x = make_float4(x[0], x[1], x[2], x[3]);
+  Q.y = make_float4(y[0], y[1], y[2], y[3]);
+  Q.halfM = make_float4(h[0], h[1], h[2], h[3]);
+  Q.w = make_float4(w[0], w[1], w[2], w[3]);
+  *reinterpret_cast<uint4 *>(&Q.child[0]) = make_uint4(c[0].x, c[0].y, c[1].x, c[1].y);
+  *reinterpret_cast<uint4 *>(&Q.child[2]) = make_uint4(c[2].x, c[2].y, c[3].x, c[3].y);
+  return at;
+}
+
+// The record that holds only the root (up, a) of the instance with body b.
+__device__ __forceinline__ void quad_root(const DevState &S, uint32_t b, float4 up, float4 a) {
+  const uint32_t sg = S.segOf[b];
+  const float4 ups[4] = {up}, as[4] = {a};
+  const int first[4] = {(int)S.seg[sg].start};
+  quad_record(S, S.n + sg, a.x, a.y, 1, ups, as, first);
+}
+
 // Bottom-up sums over the traversal records: each leaf sums its bodies
 // (sumNode's order) and climbs; the last non-empty child to arrive sums its
 // parent's children in digit order, then finishNode's divide; second
@@ -692,10 +729,14 @@ __global__ void __launch_bounds__(kBlock)
       }
       __stcg(&S.tM[p], make_float4(ixx, iyy, ixy, S.tM[p].w));
     }
-    __stcg(&S.sumX[p], px);
-    __stcg(&S.sumY[p], py);
-    __stcg(&S.tN[p].a, make_float4(X, Y, mm, S.tN[p].a.w));
+    const float4 own = S.tN[p].a;
+    const uint32_t leafLink = kQuadLeaf | (uint32_t)(B.w - B.z);
+    __stcg(&S.tUp[p], make_float4(px, py, own.w, __uint_as_float(leafLink)));
+    __stcg(&S.tN[p].a, make_float4(X, Y, mm, own.w));
     int32_t node = S.parent[p];
+    if (node < 0)
+      quad_root(S, b0, make_float4(px, py, own.w, __uint_as_float(leafLink)),
+                make_float4(X, Y, mm, own.w));
     for (int guard = 0; node >= 0 && guard <= kMaxDepth; ++guard) {
       const uint32_t g = (uint32_t)node;
       if (g >= total) {
@@ -713,20 +754,20 @@ __global__ void __launch_bounds__(kBlock)
       if (old + 1 != children) break;
       const uint4 kv = kids[g];
       const uint32_t r[4] = {kv.x, kv.y, kv.z, kv.w};
-      float cxs[4], cys[4];
-      float4 ca[4], mo[4];
+      float4 up[4], ca[4], mo[4];
+      int first[4]; // the children's first bodies
       for (uint32_t q = 0; q < 4; ++q) {
         if (q >= children || r[q] >= total) continue;
-        cxs[q] = __ldcg(&S.sumX[r[q]]);
-        cys[q] = __ldcg(&S.sumY[r[q]]);
+        up[q] = __ldcg(&S.tUp[r[q]]);
         ca[q] = __ldcg(&S.tN[r[q]].a);
+        first[q] = S.tN[r[q]].b.z;
         if (kMoments) mo[q] = __ldcg(&S.tM[r[q]]);
       }
       float sx = 0.0f, sy = 0.0f, sm = 0.0f;
       for (uint32_t q = 0; q < children && q < 4; ++q) {
         if (r[q] >= total) break;
-        sx = q == 0 ? cxs[q] : __fadd_rn(sx, cxs[q]);
-        sy = q == 0 ? cys[q] : __fadd_rn(sy, cys[q]);
+        sx = q == 0 ? up[q].x : __fadd_rn(sx, up[q].x);
+        sy = q == 0 ? up[q].y : __fadd_rn(sy, up[q].y);
         sm = q == 0 ? ca[q].z : __fadd_rn(sm, ca[q].z);
       }
       const float dv = fmaxf(sm, FLT_MIN);
@@ -742,10 +783,20 @@ __global__ void __launch_bounds__(kBlock)
         }
         __stcg(&S.tM[g], make_float4(jxx, jyy, jxy, S.tM[g].w));
       }
-      __stcg(&S.sumX[g], sx);
-      __stcg(&S.sumY[g], sy);
-      __stcg(&S.tN[g].a, make_float4(PX, PY, sm, S.tN[g].a.w));
+      const float ownW = S.tN[g].a.w;
+      // one child: the same bodies under a smaller square, its record goes up
+      float wBot = up[0].z;
+      uint32_t link = __float_as_uint(up[0].w);
+      if (children > 1) {
+        wBot = ownW;
+        link = quad_record(S, (uint32_t)first[1], PX, PY, children, up, ca, first);
+      }
+      const float4 ownUp = make_float4(sx, sy, wBot, __uint_as_float(link));
+      const float4 ownA = make_float4(PX, PY, sm, ownW);
+      __stcg(&S.tUp[g], ownUp);
+      __stcg(&S.tN[g].a, ownA);
       node = S.parent[g];
+      if (node < 0) quad_root(S, b0, ownUp, ownA);
     }
   }
 }

@@ -1,20 +1,22 @@
-// force.cu -- warp-cooperative stackless Barnes-Hut traversal.
+// force.cu -- warp-cooperative Barnes-Hut traversal.
 //
-// Each lane walks the tree for one body exactly as accelerationAt does
+// Every walk here gives each body exactly the terms accelerationAt does
 // (src/cuda/TreeKernels.cuh:197-245; QuadTree::acceleration,
 // src/QuadTree.cpp:264-389): accept a node when size^2 < d^2*theta^2 and
 // add m*d*fastInvSqrt(d^2)/(d^2+eps^2) (clamped to FLT_MAX), otherwise sum
-// a leaf's bodies one by one, otherwise descend.  Per-lane acceptance is
-// kept, so each body opens exactly the nodes the reference opens and sums
-// them in the same order.
+// a leaf's bodies one by one, otherwise descend.
 //
-// The warp cooperates through the depth-first preorder layout (build.cu):
-// along every lane's walk the preorder position only increases (descend =
-// +1, skip = +subtree size), so the warp always serves the smallest
-// position any lane is waiting at.  The node's record is read once per
-// warp (one broadcast load through L1; staging 32-node tiles in shared
-// memory measured 9-11% slower for the extra per-iteration bookkeeping);
-// a leaf's bodies are staged in shared memory with one coalesced load.
+// The default force pass walks the tree once per group of 32 bodies over
+// records of four children (walk_group).  Exact arithmetic, the clamped law,
+// the corrected forms, queries and counting keep a cursor per lane
+// (walk_targets), so that a body's terms are summed in the reference's
+// order: along a lane's walk of the depth-first preorder layout (build.cu)
+// the position only increases (descend = +1, skip = +subtree size), so the
+// warp always serves the smallest position any lane is waiting at.  The
+// node's record is read once per warp (one broadcast load through L1;
+// staging 32-node tiles in shared memory measured 9-11% slower for the extra
+// per-iteration bookkeeping); a leaf's bodies are staged in shared memory
+// with one coalesced load.
 //
 // kExact = true evaluates every float operation as the reference writes
 // it (no FMA contraction, IEEE reciprocal): the result is bit-identical to
@@ -133,7 +135,7 @@ __device__ __forceinline__ void quad_term(float dx, float dy, float dSq,
 template <bool kExact, bool kCount, int kCorr, bool kClamp>
 __device__ __forceinline__ void walk_targets(
     const DevState &S, float tSq, float eSq, float bandSq, float eps, float x, float y,
-    uint32_t cur, float4 *sBodyW, const MlpDev &sW, __nv_bfloat16 (*sStageW)[16],
+    uint32_t cur, float4 *sBodyW, const MlpDev *sW, __nv_bfloat16 (*sStageW)[16],
     float &ax, float &ay, uint32_t &nFar, uint32_t &nNear, uint32_t &nVisit,
     uint32_t &nIter, uint32_t &nChunk) {
   const int lane = threadIdx.x & 31;
@@ -193,7 +195,7 @@ __device__ __forceinline__ void walk_targets(
           if (!ok)
             for (int q = 0; q < 9; ++q) f[q] = 0.0f;
           float o0, o1;
-          mlp_warp(sW, f, sStageW, o0, o1);
+          mlp_warp(*sW, f, sStageW, o0, o1);
           if (ok) {
             // |mono| * ((1 + t0) u + t1 w), w = (-uy, ux)
             const float r = dSq * rsqrtf(dSq);
@@ -269,7 +271,7 @@ __device__ __forceinline__ f2x fma2(f2x a, f2x b, f2x c) {
 }
 
 // The default plain walk (contracted arithmetic, clamp-free law, no
-// correction, no counting) with paired FP32 instructions: the cell term's
+// correction, no counting) with a cursor per lane and paired FP32 instructions: the cell term's
 // {dx, dy} and its accumulation are one pair each, and a leaf's bodies are
 // taken two at a time (structure-of-arrays staging, so one 64-bit shared
 // load gives two bodies' x, y or mass).  Each body accepts, opens and skips
@@ -355,6 +357,449 @@ __device__ __forceinline__ void walk_plain_x2(const DevState &S, float tSq, floa
   ayOut = ay + (ly0 + ly1);
 }
 
+// The law's factor m * fastInvSqrt(d^2) / (d^2 + eps^2) of two terms, from
+// half masses.  With g the magic guess, the Newton step g (1.5 - 0.5 d^2 g g)
+// is half of gn (d^2 gn gn - 3), gn = -g (the sign bit set in the guess's
+// constant); negations and factors of two are exact, so every rounding is
+// that of (m * g (1.5 - (0.5 d^2) g g)) * rcp, one operation less.
+__device__ __forceinline__ f2x law_pair(f2x d2, f2x halfM, f2x e2, f2x neg3) {
+  float d0, d1, q0, q1;
+  upk2(d2, d0, d1);
+  const f2x gn = pk2(u2f(0xdf3759dfu - (f2u(d0) >> 1)), u2f(0xdf3759dfu - (f2u(d1) >> 1)));
+  const f2x is2 = mul2(gn, fma2(mul2(d2, gn), gn, neg3));
+  upk2(add2(d2, e2), q0, q1);
+  return mul2(mul2(halfM, is2), pk2(rcp_approx(q0), rcp_approx(q1)));
+}
+
+// acc += a * b where on != 0.
+__device__ __forceinline__ void fma2_if(uint32_t on, f2x a, f2x b, f2x &acc) {
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\t@p fma.rn.f32x2 %0, %2, %3, %0;\n\t}"
+      : "+l"(acc)
+      : "r"(on), "l"(a), "l"(b));
+}
+__device__ __forceinline__ void fma_if(uint32_t on, float dx, float dy, float f, float &ax,
+                                       float &ay) {
+  asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p fma.rn.f32 %0, %3, %5, %0;\n\t"
+      "@p fma.rn.f32 %1, %4, %5, %1;\n\t}"
+      : "+f"(ax), "+f"(ay)
+      : "r"(on), "f"(dx), "f"(dy), "f"(f));
+}
+
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// One warp's scratch of walk_group.
+constexpr int kTake = 16;     // records tested at once, four children each
+constexpr int kSlots = 192;   // opened records (slots are bytes)
+constexpr int kParts = 400;   // children that some lanes accept
+constexpr int kCells = 704;   // cell terms
+constexpr int kLeaves = 128;  // opened leaves
+constexpr int kPairs = 448;   // pairs of their bodies
+struct alignas(16) WalkStage {
+  union {
+    struct { // children the lanes disagree on, their lanes, those that accept
+      float cx[64], cy[64], cw[64];
+      uint32_t cm[64], ca[64];
+    };
+    uint32_t count[kSlots]; // terms of a record's subtree, later its first
+                            // place: cells | leaves << 10 | leaf pairs << 20
+    struct { // terms being summed: place, half mass, lanes (of each / a pair)
+      float x[64], y[64], h[64];
+      uint32_t m[64];
+    };
+  };
+  uint32_t rec[kSlots], who[kSlots]; // an opened record and its lanes
+  uint32_t part[kParts];             // lanes that accept a child
+  uint32_t starts[kPairs / 32];      // bit p: pair p is the first of a leaf
+  uint16_t info[kSlots * 4];         // per child: kInfo bits | slot or pairs
+  uint16_t partOf[kSlots * 4];       // per child with kInfoPart: index in part
+  uint16_t cell[kCells];             // cells in order: slot << 2 | child
+  uint16_t leaf[kLeaves];            // leaves in order
+  uint8_t batch[kSlots];             // first slot of each batch
+};
+static_assert(kSlots <= 256 && kSlots * 4 < 1024 && kPairs < 4096, "packed fields");
+// a child's low byte: the slot of its opened record, or an opened leaf's pairs
+constexpr uint32_t kInfoLeaf = 1u << 8, kInfoInner = 1u << 9;
+constexpr uint32_t kInfoTerm = 1u << 10, kInfoPart = 1u << 11; // accepted, by some only
+
+// The default plain walk for a group of targets of instance sg (lanes in
+// `valid`; the others hold a copy of a valid target's place), with the
+// result of walk_plain_x2 bit for bit: a body's cells are summed in preorder
+// into one accumulator, its leaves' bodies in preorder into two.
+// Bounded by instruction issue, so the tree is walked once for the group,
+// with a node to a lane, instead of by every lane at every node:
+//  * records open breadth-first, up to sixteen at a time: lanes 2 r and
+//    2 r + 1 test two children each of record r against the group's box.  A target's own test is
+//    w < fl(fl(dx^2 + dy^2) theta^2) with every rounding monotone in |dx| and
+//    |dy|, so the same expression at the box's nearest (farthest) point is a
+//    lower (upper) bound of every lane's: a child all lanes accept is a
+//    term, one that none accepts is opened, with no test per lane.  The
+//    children in between (a fifth) are tested by every lane, two to a paired
+//    instruction;
+//  * the batches are then passed in reverse to count each subtree's terms and
+//    forwards to place them, which lists the terms in preorder;
+//  * all lanes sum the lists, each term with the mask of the lanes it belongs
+//    to: the law in pairs, the cells' accumulation one by one in order.
+// Returns false, with nothing summed, if the group's records do not fit.
+//
+// Two discs of 2^20 bodies, theta 0.5, per group: 95 records in 12 batches, 229
+// whole cells, 86 children tested by lane, 34 leaves of 329 bodies; 14.3k
+// warp instructions instead of walk_plain_x2's 18.6k.  The force pass takes
+// 617 us there (719 before), 99,991 bodies 78 (131), 10,000 at theta 1 20 (36),
+// 1000 16 (27): with few warps the walk's latency counts, and a group waits
+// for ~12 dependent loads instead of ~400.  Of a group's 87k cycles the opening
+// takes 30k, counting and placing 13k, the cells 19k, the leaves 25k.
+// Measured and dropped: terms in the order the records open (528 us, no
+// counting or placing, but another order of the sums); eight records at a
+// time (630); 24 or 28 warps per SM at fewer registers (620, 640); both
+// loops over terms unrolled twice more (645); the guess as one mad.hi (+13%).
+__device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float eSq, float x,
+                                           float y, uint32_t sg, uint32_t valid,
+                                           WalkStage &st, float &axOut, float &ayOut) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t laneBit = 1u << lane, below = laneBit - 1u;
+  const f2x XX = pk2(x, x), YY = pk2(y, y), E2 = pk2(eSq, eSq), N3 = pk2(-3.0f, -3.0f);
+  const QuadRec *__restrict__ tQ = S.tQ;
+  const uint32_t lastRec = S.n + S.nseg - 1u;
+  uint32_t tail = 1, batches = 0;
+  const int half = lane & 1;
+  {
+    const f2x T2 = pk2(tSq, tSq);
+    f2x LOX, HIX, LOY, HIY;
+    {
+      const float loX = warp_min(x), hiX = warp_max(x), loY = warp_min(y), hiY = warp_max(y);
+      LOX = pk2(loX, loX);
+      HIX = pk2(hiX, hiX);
+      LOY = pk2(loY, loY);
+      HIY = pk2(hiY, hiY);
+    }
+    if (lane == 0) { // the root's record
+      st.rec[0] = S.n + sg;
+      st.who[0] = valid;
+    }
+    if (lane < kPairs / 32) st.starts[lane] = 0u;
+    __syncwarp();
+    uint32_t parts = 0, lanePairs = 0;
+    for (uint32_t head = 0; head < tail;) {
+      const uint32_t take = min((uint32_t)kTake, tail - head);
+      const uint32_t slot = head + (lane >> 1);
+      const bool have = (uint32_t)(lane >> 1) < take;
+      f2x X2 = 0, Y2 = 0;
+      float w[2] = {0.0f, 0.0f};
+      uint32_t link[2] = {kQuadLeaf, kQuadLeaf}, mask = 0;
+      if (have) {
+        const QuadRec *q = tQ + min(st.rec[slot], lastRec);
+        mask = st.who[slot];
+        X2 = __ldg(reinterpret_cast<const f2x *>(&q->x) + half);
+        Y2 = __ldg(reinterpret_cast<const f2x *>(&q->y) + half);
+        const float2 ww = __ldg(reinterpret_cast<const float2 *>(&q->w) + half);
+        const uint4 cc = __ldg(reinterpret_cast<const uint4 *>(&q->child[0]) + half);
+        w[0] = ww.x;
+        w[1] = ww.y;
+        link[0] = cc.x;
+        link[1] = cc.z;
+      }
+      // per axis: how far the box lies beyond the child on either side
+      float ax0[2], ax1[2], ay0[2], ay1[2], near2[2], far2[2];
+      upk2(sub2(LOX, X2), ax0[0], ax0[1]);
+      upk2(sub2(X2, HIX), ax1[0], ax1[1]);
+      upk2(sub2(LOY, Y2), ay0[0], ay0[1]);
+      upk2(sub2(Y2, HIY), ay1[0], ay1[1]);
+      {
+        const f2x NX = pk2(fmaxf(fmaxf(ax0[0], ax1[0]), 0.0f), fmaxf(fmaxf(ax0[1], ax1[1]), 0.0f));
+        const f2x NY = pk2(fmaxf(fmaxf(ay0[0], ay1[0]), 0.0f), fmaxf(fmaxf(ay0[1], ay1[1]), 0.0f));
+        const f2x FX = pk2(fminf(ax0[0], ax1[0]), fminf(ax0[1], ax1[1]));
+        const f2x FY = pk2(fminf(ay0[0], ay1[0]), fminf(ay0[1], ay1[1]));
+        upk2(mul2(fma2(NX, NX, mul2(NY, NY)), T2), near2[0], near2[1]);
+        upk2(mul2(fma2(FX, FX, mul2(FY, FY)), T2), far2[0], far2[1]);
+      }
+      uint32_t accept[2], info[2], lanes[2];
+      bool split[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        lanes[j] = link[j] == kQuadLeaf ? 0u : mask; // absent: no lane
+        const bool all = w[j] < near2[j], none = !(w[j] < far2[j]);
+        accept[j] = all ? lanes[j] : 0u;
+        split[j] = lanes[j] != 0 && !all && !none;
+        info[j] = split[j] ? kInfoPart : 0u;
+      }
+      const uint32_t s0 = __ballot_sync(0xffffffffu, split[0]);
+      const uint32_t s1 = __ballot_sync(0xffffffffu, split[1]);
+      if (s0 | s1) {
+        const uint32_t at0 = __popc(s0 & below) + __popc(s1 & below);
+        const uint32_t at[2] = {at0, at0 + (split[0] ? 1u : 0u)};
+        const uint32_t n = __popc(s0) + __popc(s1);
+        float px[2], py[2];
+        upk2(X2, px[0], px[1]);
+        upk2(Y2, py[0], py[1]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (split[j]) {
+            st.cx[at[j]] = px[j];
+            st.cy[at[j]] = py[j];
+            st.cw[at[j]] = w[j];
+            st.cm[at[j]] = lanes[j];
+          }
+        __syncwarp();
+        for (uint32_t k = 0; k < n; k += 2) { // an odd last one's partner: unused
+          const f2x DX = sub2(*reinterpret_cast<const f2x *>(&st.cx[k]), XX);
+          const f2x DY = sub2(*reinterpret_cast<const f2x *>(&st.cy[k]), YY);
+          const float2 cw2 = *reinterpret_cast<const float2 *>(&st.cw[k]);
+          const uint2 m = *reinterpret_cast<const uint2 *>(&st.cm[k]);
+          float r0, r1;
+          upk2(mul2(fma2(DX, DX, mul2(DY, DY)), T2), r0, r1);
+          const uint32_t a0 = m.x & __ballot_sync(0xffffffffu, cw2.x < r0);
+          const uint32_t a1 = m.y & __ballot_sync(0xffffffffu, cw2.y < r1);
+          if (lane == 0) *reinterpret_cast<uint2 *>(&st.ca[k]) = make_uint2(a0, a1);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+          if (split[j]) {
+            accept[j] = st.ca[at[j]];
+            if (parts + at[j] < kParts) {
+              st.part[parts + at[j]] = accept[j];
+              st.partOf[slot * 4 + 2 * half + j] = (uint16_t)(parts + at[j]);
+            }
+          }
+        parts += n;
+      }
+      bool inner[2];
+      uint32_t open[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        open[j] = lanes[j] & ~accept[j];
+        inner[j] = open[j] != 0 && !(link[j] & kQuadLeaf);
+        if (accept[j]) info[j] |= kInfoTerm;
+        if (open[j] != 0 && !inner[j]) {
+          const uint32_t pairs = ((link[j] & ~kQuadLeaf) + 1u) >> 1;
+          lanePairs += min(pairs, 65536u);
+          info[j] |= (pairs & 255u) | kInfoLeaf;
+          if (pairs > 255u) lanePairs = 65536u; // does not fit the byte
+        }
+      }
+      const uint32_t p0 = __ballot_sync(0xffffffffu, inner[0]);
+      const uint32_t p1 = __ballot_sync(0xffffffffu, inner[1]);
+      uint32_t at = tail + __popc(p0 & below) + __popc(p1 & below);
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        if (inner[j]) {
+          if (at < kSlots) {
+            st.rec[at] = link[j];
+            st.who[at] = open[j];
+          }
+          info[j] |= (at & 255u) | kInfoInner;
+          ++at;
+        }
+      if (have) reinterpret_cast<uint32_t *>(st.info)[slot * 2 + half] = info[0] | info[1] << 16;
+      if (lane == 0) st.batch[batches] = (uint8_t)head;
+      ++batches;
+      head += take;
+      tail += __popc(p0) + __popc(p1);
+      if (tail > kSlots || parts > kParts) return false;
+      __syncwarp();
+    }
+    if (__reduce_add_sync(0xffffffffu, lanePairs) > kPairs) return false;
+  }
+  // subtree counts, from the last batch to the first
+  auto child_terms = [&](uint32_t info) {
+    uint32_t v = info & kInfoTerm ? 1u : 0u;
+    if (info & kInfoLeaf) v += (info & 255u) << 20 | 1u << 10;
+    if (info & kInfoInner) v += st.count[info & 255u];
+    return v;
+  };
+  for (uint32_t b = batches, end = tail; b-- > 0;) {
+    const uint32_t head = st.batch[b], slot = head + (lane >> 1);
+    const bool have = slot < end;
+    const uint32_t info = have ? reinterpret_cast<const uint32_t *>(st.info)[slot * 2 + half] : 0u;
+    uint32_t v = child_terms(info & 0xffffu) + child_terms(info >> 16);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    if (have && half == 0) st.count[slot] = v;
+    end = head;
+    __syncwarp();
+  }
+  const uint32_t total = st.count[0], nCells = total & 1023u, nLeaves = total >> 10 & 1023u;
+  const uint32_t nPairs = total >> 20;
+  if (nCells > kCells || nLeaves > kLeaves) return false;
+  __syncwarp();
+  if (lane == 0) st.count[0] = 0;
+  __syncwarp();
+  // places: a child's term, then its subtree's, then the next child's
+  for (uint32_t b = 0; b < batches; ++b) {
+    const uint32_t head = st.batch[b], end = b + 1 < batches ? st.batch[b + 1] : tail;
+    const uint32_t slot = head + (lane >> 1);
+    const bool have = slot < end;
+    const uint32_t info2 = have ? reinterpret_cast<const uint32_t *>(st.info)[slot * 2 + half] : 0u;
+    const uint32_t info[2] = {info2 & 0xffffu, info2 >> 16};
+    const uint32_t v[2] = {child_terms(info[0]), child_terms(info[1])};
+    const uint32_t before = __shfl_up_sync(0xffffffffu, v[0] + v[1], 1);
+    if (have) {
+      uint32_t at = st.count[slot] + (half ? before : 0u);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const uint16_t code = (uint16_t)(slot << 2 | (2 * half + j));
+        if (info[j] & kInfoTerm) st.cell[at & 1023u] = code;
+        if (info[j] & kInfoInner) st.count[info[j] & 255u] = at + (info[j] & kInfoTerm ? 1u : 0u);
+        if (info[j] & kInfoLeaf) {
+          st.leaf[at >> 10 & 1023u] = code;
+          atomicOr(&st.starts[at >> 25], 1u << (at >> 20 & 31u));
+        }
+        at += v[j];
+      }
+    }
+    __syncwarp();
+  }
+  // lanes of a listed child's record that accept it
+  auto accepts = [&](uint32_t code, uint32_t lanes) {
+    const uint32_t info = st.info[code];
+    return info & kInfoTerm ? (info & kInfoPart ? st.part[st.partOf[code]] : lanes) : 0u;
+  };
+  // the cells, 64 at a time, two to a lane (the next ones' loads under way)
+  float ax = 0.0f, ay = 0.0f;
+  {
+    float qx[2], qy[2], qh[2];
+    uint32_t qm[2];
+    auto fetch = [&](uint32_t k) {
+#pragma unroll
+      for (uint32_t j = 0; j < 2; ++j) {
+        qx[j] = qy[j] = qh[j] = 0.0f;
+        qm[j] = 0;
+        if (k + j < nCells) {
+          const uint32_t code = st.cell[k + j], slot = code >> 2, c = code & 3u;
+          const QuadRec *q = tQ + st.rec[slot];
+          qx[j] = __ldg(reinterpret_cast<const float *>(&q->x) + c);
+          qy[j] = __ldg(reinterpret_cast<const float *>(&q->y) + c);
+          qh[j] = __ldg(reinterpret_cast<const float *>(&q->halfM) + c);
+          qm[j] = accepts(code, st.who[slot]);
+        }
+      }
+    };
+    fetch(2 * lane);
+    for (uint32_t base = 0; base < nCells; base += 64) {
+      *reinterpret_cast<float2 *>(&st.x[2 * lane]) = make_float2(qx[0], qx[1]);
+      *reinterpret_cast<float2 *>(&st.y[2 * lane]) = make_float2(qy[0], qy[1]);
+      *reinterpret_cast<float2 *>(&st.h[2 * lane]) = make_float2(qh[0], qh[1]);
+      *reinterpret_cast<uint2 *>(&st.m[2 * lane]) = make_uint2(qm[0], qm[1]);
+      __syncwarp();
+      fetch(base + 64 + 2 * lane);
+      const uint32_t n = min(64u, nCells - base);
+      for (uint32_t k = 0; k < n; k += 4) { // past n: no lane
+        const ulonglong2 X4 = *reinterpret_cast<const ulonglong2 *>(&st.x[k]);
+        const ulonglong2 Y4 = *reinterpret_cast<const ulonglong2 *>(&st.y[k]);
+        const ulonglong2 H4 = *reinterpret_cast<const ulonglong2 *>(&st.h[k]);
+        const uint4 m = *reinterpret_cast<const uint4 *>(&st.m[k]);
+        const f2x DX0 = sub2(X4.x, XX), DY0 = sub2(Y4.x, YY);
+        const f2x DX1 = sub2(X4.y, XX), DY1 = sub2(Y4.y, YY);
+        const f2x F0 = law_pair(fma2(DX0, DX0, mul2(DY0, DY0)), H4.x, E2, N3);
+        const f2x F1 = law_pair(fma2(DX1, DX1, mul2(DY1, DY1)), H4.y, E2, N3);
+        float dx0, dx1, dx2, dx3, dy0, dy1, dy2, dy3, f0, f1, f2, f3;
+        upk2(DX0, dx0, dx1);
+        upk2(DY0, dy0, dy1);
+        upk2(F0, f0, f1);
+        upk2(DX1, dx2, dx3);
+        upk2(DY1, dy2, dy3);
+        upk2(F1, f2, f3);
+        fma_if(m.x & laneBit, dx0, dy0, f0, ax, ay);
+        fma_if(m.y & laneBit, dx1, dy1, f1, ax, ay);
+        fma_if(m.z & laneBit, dx2, dy2, f2, ax, ay);
+        fma_if(m.w & laneBit, dx3, dy3, f3, ax, ay);
+      }
+      __syncwarp();
+    }
+  }
+  // the leaves' bodies, 32 pairs at a time (an odd leaf's last body has a
+  // massless partner)
+  f2x lx = pk2(0.0f, 0.0f), ly = pk2(0.0f, 0.0f);
+  {
+    float4 q0, q1;
+    uint32_t qm;
+    uint32_t before = 0, last = 0; // leaves that start before the pairs fetched
+                                   // next, and the last one's first pair
+    auto fetch = [&](uint32_t base) {
+      q0 = q1 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      qm = 0;
+      if (base >= nPairs) return;
+      const uint32_t word = st.starts[base >> 5], mine = word & (laneBit | below);
+      if (base + lane < nPairs) {
+        const uint32_t code = st.leaf[before + __popc(mine) - 1u], slot = code >> 2;
+        const uint32_t j = 2u * (base + lane - (mine ? base + 31u - __clz(mine) : last));
+        const uint2 c = __ldg(&tQ[st.rec[slot]].child[code & 3u]);
+        const uint32_t b = c.y + j, lanes = st.who[slot];
+        if (b < S.n) q0 = S.xym[b]; // defensive bounds
+        if (j + 1u < (c.x & ~kQuadLeaf) && b + 1u < S.n) q1 = S.xym[b + 1u];
+        qm = lanes & ~accepts(code, lanes);
+      }
+      before += __popc(word);
+      if (word) last = base + 31u - __clz(word);
+    };
+    fetch(0);
+    for (uint32_t base = 0; base < nPairs; base += 32) {
+      *reinterpret_cast<float2 *>(&st.x[2 * lane]) = make_float2(q0.x, q1.x);
+      *reinterpret_cast<float2 *>(&st.y[2 * lane]) = make_float2(q0.y, q1.y);
+      *reinterpret_cast<float2 *>(&st.h[2 * lane]) = make_float2(0.5f * q0.z, 0.5f * q1.z);
+      st.m[lane] = qm;
+      __syncwarp();
+      fetch(base + 32);
+      const uint32_t n = min(32u, nPairs - base);
+      for (uint32_t k = 0; k < n; k += 2) { // past n: no lane
+        const ulonglong2 X4 = *reinterpret_cast<const ulonglong2 *>(&st.x[2 * k]);
+        const ulonglong2 Y4 = *reinterpret_cast<const ulonglong2 *>(&st.y[2 * k]);
+        const ulonglong2 H4 = *reinterpret_cast<const ulonglong2 *>(&st.h[2 * k]);
+        const uint2 m = *reinterpret_cast<const uint2 *>(&st.m[k]);
+        const f2x DX0 = sub2(X4.x, XX), DY0 = sub2(Y4.x, YY);
+        const f2x DX1 = sub2(X4.y, XX), DY1 = sub2(Y4.y, YY);
+        const f2x F0 = law_pair(fma2(DX0, DX0, mul2(DY0, DY0)), H4.x, E2, N3);
+        const f2x F1 = law_pair(fma2(DX1, DX1, mul2(DY1, DY1)), H4.y, E2, N3);
+        fma2_if(m.x & laneBit, DX0, F0, lx);
+        fma2_if(m.x & laneBit, DY0, F0, ly);
+        fma2_if(m.y & laneBit, DX1, F1, lx);
+        fma2_if(m.y & laneBit, DY1, F1, ly);
+      }
+      __syncwarp();
+    }
+  }
+  if (valid & laneBit) {
+    float lx0, lx1, ly0, ly1;
+    upk2(lx, lx0, lx1);
+    upk2(ly, ly0, ly1);
+    axOut = ax + (lx0 + lx1);
+    ayOut = ay + (ly0 + ly1);
+  }
+  return true;
+}
+
+// Body i's acceleration: the attractor's pull added, and with recOut its
+// whole record (nbx_body: pos, vel, acc, mass, radius, id), for a copy to
+// the host right after this launch.
+template <bool kExact>
+__device__ __forceinline__ void store_acc(const DevState &S, uint32_t i, float x, float y,
+                                          float ax, float ay) {
+  add_attractor<kExact>(S.attr, x, y, ax, ay);
+  S.acc[i] = make_float2(ax, ay);
+  if (S.recOut) {
+    const float4 p = S.pv[i];
+    const float2 m = S.mr[i];
+    uint32_t *r = S.recOut + (size_t)i * 9;
+    r[0] = __float_as_uint(p.x);
+    r[1] = __float_as_uint(p.y);
+    r[2] = __float_as_uint(p.z);
+    r[3] = __float_as_uint(p.w);
+    r[4] = __float_as_uint(ax);
+    r[5] = __float_as_uint(ay);
+    r[6] = __float_as_uint(m.x);
+    r[7] = __float_as_uint(m.y);
+    r[8] = S.id[i];
+  }
+}
+
 // Every target of the launch, one warp per 32.  kPairs selects the paired
 // leaf loop for the default plain walk.
 template <bool kExact, bool kCount, int kCorr, bool kClamp, bool kPairs>
@@ -399,14 +844,14 @@ __device__ __forceinline__ void forces_walk(
     const bool anyWide = !kClamp && __any_sync(0xffffffffu, wide);
     if (anyWide)
       walk_targets<kExact, kCount, kCorr, true>(S, tSq, eSq, bandSq, eps, x, y, cur,
-                                                sBody[w], sW, sStage[kCorr == 1 ? w : 0],
+                                                sBody[w], &sW, sStage[kCorr == 1 ? w : 0],
                                                 ax, ay, nFar, nNear, nVisit, nIter, nChunk);
     else if (kPlainX2) {
       float *sX = reinterpret_cast<float *>(sBody[w]);
       walk_plain_x2(S, tSq, eSq, x, y, cur, sX, sX + 32, sX + 64, ax, ay);
     } else
       walk_targets<kExact, kCount, kCorr, kClamp>(S, tSq, eSq, bandSq, eps, x, y, cur,
-                                                  sBody[w], sW, sStage[kCorr == 1 ? w : 0],
+                                                  sBody[w], &sW, sStage[kCorr == 1 ? w : 0],
                                                   ax, ay, nFar, nNear, nVisit, nIter, nChunk);
     if (kCount) {
       unsigned long long f = nFar, nn = nNear, v = nVisit;
@@ -426,24 +871,7 @@ __device__ __forceinline__ void forces_walk(
       if (query) {
         queryAcc[i] = make_float2(ax, ay);
       } else {
-        add_attractor<kExact>(S.attr, x, y, ax, ay);
-        S.acc[i] = make_float2(ax, ay);
-        if (S.recOut) {
-          // the body's whole record (nbx_body: pos, vel, acc, mass,
-          // radius, id), for a copy to the host right after this launch
-          const float4 p = S.pv[i];
-          const float2 m = S.mr[i];
-          uint32_t *r = S.recOut + (size_t)i * 9;
-          r[0] = __float_as_uint(p.x);
-          r[1] = __float_as_uint(p.y);
-          r[2] = __float_as_uint(p.z);
-          r[3] = __float_as_uint(p.w);
-          r[4] = __float_as_uint(ax);
-          r[5] = __float_as_uint(ay);
-          r[6] = __float_as_uint(m.x);
-          r[7] = __float_as_uint(m.y);
-          r[8] = S.id[i];
-        }
+        store_acc<kExact>(S, i, x, y, ax, ay);
       }
     }
   }
@@ -456,7 +884,7 @@ __device__ __forceinline__ void forces_walk(
 // overflow, takes the clamped walk instead.  Launch bounds: a full SM of
 // kBlock-thread blocks (2048 threads: at most 32 registers) for every walk
 // but the learned correction's, whose MMA fragments keep it at 3 blocks of
-// 256, and the default plain walk's: 1536 threads per SM (40 registers),
+// 256, and the paired plain walk's: 1536 threads per SM (40 registers),
 // 1% faster than 2048 at 32 registers and identical in results.  kBlock
 // and kPairs vary only for the default plain walk (the autotuner's block
 // shape and leaf width).
@@ -484,6 +912,80 @@ __global__ void __launch_bounds__(kBlock, kCorr == 1 ? 3
   }
   forces_walk<kExact, kCount, kCorr, kClamp, kPairs>(S, tSq, eSq, counts, bandSq, eps, query,
                                                      nQuery, queryAcc, sBody, sW, sStage);
+}
+
+// The default force pass (leaf_pairs 1): walk_group for one group of
+// targets per warp, walk_plain_x2 where that does not fit, and the clamped
+// walk for a group of an instance that reaches beyond the coordinate limit,
+// as in k_forces.
+constexpr int kGroupWarpsPerSM = 20;
+template <int kBlock>
+__global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
+                                              ? kGroupWarpsPerSM * 32 / kBlock : 1)
+    k_forces_groups(DevState S, float tSq, float eSq) {
+  extern __shared__ uint4 sDyn[]; // a WalkStage per warp
+  const int lane = threadIdx.x & 31;
+  WalkStage &st = reinterpret_cast<WalkStage *>(sDyn)[threadIdx.x >> 5];
+  const uint32_t warpsTotal = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t gEnd = S.tgEnd ? S.tgEnd : S.nGroups;
+  for (uint32_t g = S.tgBegin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); g < gEnd;
+       g += warpsTotal) {
+    const uint32_t first = S.nseg == 1 ? g * 32u : S.groupFirst[g];
+    const uint32_t sg = S.segOf[first];
+    const SegDev &G = S.seg[sg];
+    const uint32_t count = min(32u, G.start + G.count - first);
+    const bool mine = (uint32_t)lane < count;
+    const uint32_t i = mine ? first + lane : first;
+    const float4 b = S.xym[i];
+    const uint32_t root = mine && G.travCount > 0 ? G.travBase : kDone;
+    float ax = 0.0f, ay = 0.0f;
+    float4 *staged = reinterpret_cast<float4 *>(&st);
+    static_assert(sizeof(WalkStage) >= 32 * sizeof(float4), "holds a leaf's staged bodies");
+    if (G.wide) {
+      uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
+      walk_targets<false, false, 0, true>(S, tSq, eSq, 0.0f, 0.0f, b.x, b.y, root, staged,
+                                          nullptr, nullptr, ax, ay, c0, c1, c2, c3, c4);
+    } else if (G.travCount > 0) {
+      // A group whose walk does not fit goes in two at the widest step along
+      // its bodies, if that is most of the group's extent (neighbours in
+      // Morton order across the gap between two discs, say).
+      const uint32_t lanes = __ballot_sync(0xffffffffu, mine);
+      uint32_t piece = lanes;
+      while (piece) {
+        const bool in = (piece >> lane) & 1u;
+        const int lead = __ffs(piece) - 1;
+        const float lx = __shfl_sync(0xffffffffu, b.x, lead);
+        const float ly = __shfl_sync(0xffffffffu, b.y, lead);
+        const float x = in ? b.x : lx, y = in ? b.y : ly;
+        if (!walk_group(S, tSq, eSq, x, y, sg, piece, st, ax, ay)) {
+          __syncwarp();
+          const float nx = __shfl_down_sync(0xffffffffu, x, 1);
+          const float ny = __shfl_down_sync(0xffffffffu, y, 1);
+          const bool next = in && lane < 31 && ((piece >> (lane + 1)) & 1u);
+          const float step = next ? fabsf(nx - x) + fabsf(ny - y) : 0.0f;
+          const float widest = warp_max(step);
+          const float extent = warp_max(x) - warp_min(x) + warp_max(y) - warp_min(y);
+          const uint32_t at = __ballot_sync(0xffffffffu, step == widest);
+          if (widest > 0.5f * extent) {
+            piece &= (at & (0u - at)) * 2u - 1u; // the lanes up to the step
+            continue;
+          }
+          float *sX = reinterpret_cast<float *>(staged);
+          float px, py;
+          walk_plain_x2(S, tSq, eSq, b.x, b.y, in ? root : kDone, sX, sX + 32, sX + 64, px, py);
+          if (in) {
+            ax = px;
+            ay = py;
+          }
+        }
+        __syncwarp();
+        // the targets after this piece
+        piece = lanes & ~((piece | (piece - 1u)));
+      }
+    }
+    if (mine) store_acc<false>(S, i, b.x, b.y, ax, ay);
+    __syncwarp();
+  }
 }
 
 // FMA throughput probe: 8 independent chains per thread.
@@ -559,16 +1061,39 @@ uint32_t force_targets(const DevState &S) {
   return e > S.forceBegin ? e - S.forceBegin : 0u;
 }
 
+// Whether groups' walks nearly always fit their scratch (one that does not
+// is walked with a cursor per lane in the same kernel, at few warps per SM):
+// a group opens about 3 log4(n / L) / theta^2 records and its leaves hold
+// about 2.3 L (1 + 1 / theta)^2 bodies, n the mean instance (measured at theta
+// 0.25 to 0.5 and leaf capacities 4 to 64).  2^20 bodies, L 16, us with / without: theta 0.5
+// 610 / 717, 0.45 673 / 812, 0.4 (refused) 1113 / 935; L 64 at theta 0.5
+// (refused) 3700 / 874.  30,000 bodies at theta 0.5: 39 / 88.
+bool group_walk_fits(const DevState &S) {
+  const float L = (float)S.leafCapacity, n = (float)S.n / (float)S.nseg, t = sqrtf(S.tSq);
+  if (!(t > 0.0f)) return false;
+  const float near = 1.0f + 1.0f / t;
+  return 0.5f * log2f(fmaxf(n / L, 1.0f)) <= 40.0f * S.tSq && L * near * near <= 330.0f;
+}
+
 // The default plain walk with kBlock threads per block and the paired or
 // single-body leaf loop.
 template <int kBlock>
-void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs) {
+void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, bool groups) {
   if (blocks <= 0) {
-    const uint32_t warps = (force_targets(S) + 31) / 32, per = kBlock / 32;
+    uint32_t warps = (force_targets(S) + 31) / 32;
+    const uint32_t per = kBlock / 32;
+    if (pairs && groups) warps = (S.tgEnd ? S.tgEnd : S.nGroups) - S.tgBegin;
     const uint32_t b = (warps + per - 1) / per;
     blocks = (int)(b ? b : 1);
   }
-  if (pairs)
+  if (pairs && groups) {
+    constexpr int smem = kBlock / 32 * (int)sizeof(WalkStage);
+    if (smem > 48 * 1024) // above what a launch may ask for by default
+      cudaFuncSetAttribute(k_forces_groups<kBlock>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    k_forces_groups<kBlock><<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq);
+  }
+  else if (pairs)
     k_forces<false, false, 0, false, kBlock, true><<<blocks, kBlock, 0, s>>>(S, S.tSq, S.eSq);
   else
     k_forces<false, false, 0, false, kBlock, false><<<blocks, kBlock, 0, s>>>(S, S.tSq, S.eSq);
@@ -578,9 +1103,13 @@ void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
                    const MlpDev *mlp, float band, int corr, bool noClamp, int threads,
                    bool pairs) {
   if (corr == 0 && !exact && noClamp) {
-    if (threads == 128) launch_plain<128>(s, S, blocks, pairs);
-    else if (threads == 512) launch_plain<512>(s, S, blocks, pairs);
-    else launch_plain<256>(s, S, blocks, pairs);
+    // the group walk where its records nearly always fit, with 128 threads a
+    // block by default (see group_walk_fits), else a cursor per lane
+    const bool groups = pairs && group_walk_fits(S);
+    if (threads == 0) threads = groups ? 128 : 256;
+    if (threads == 128) launch_plain<128>(s, S, blocks, pairs, groups);
+    else if (threads == 512) launch_plain<512>(s, S, blocks, pairs, groups);
+    else launch_plain<256>(s, S, blocks, pairs, groups);
     return;
   }
   if (blocks <= 0) {

@@ -25,7 +25,6 @@ struct SegDev {
   uint32_t largeStart, largeCount;
   uint32_t travCount; // nodes in the traversal layout (non-empty nodes)
   uint32_t travBase;  // first record of this segment's traversal layout
-  uint32_t pad2;
 };
 
 // A node of the force traversal, in depth-first preorder: a = {comX, comY,
@@ -40,6 +39,26 @@ struct alignas(32) TravNode {
   int4 b;
 };
 static_assert(sizeof(TravNode) == 32, "32-byte traversal records");
+
+// The (up to four) children of a branching node for the default force walk,
+// in digit order as arrays of four (lane c of four takes child c): centre
+// of mass, half the mass (the law's Newton step carries a factor 2) and
+// squared size; per child a link -- kQuadLeaf | body count for a leaf, the
+// child's own record otherwise -- and its first body.  An absent child has
+// no mass and a link to an empty leaf.
+// A chain of nodes with one non-empty child each is one child here: its
+// nodes hold the same bodies, so they share centre of mass and mass bit for
+// bit, a walk that accepts any of them adds the same term, and it accepts
+// one of them iff it accepts the smallest.  So every record branches, and is
+// stored at the index of the first body of its node's second child, which
+// no other branching node shares: at most one record per body.  An
+// instance's root is the only child of a record of its own, n + instance.
+struct alignas(32) QuadRec {
+  float4 x, y, halfM, w;
+  uint2 child[4]; // {link, first body}
+};
+static_assert(sizeof(QuadRec) == 96, "three 32-byte loads");
+constexpr uint32_t kQuadLeaf = 0x80000000u;
 
 constexpr int kMaxDepth = 32;   // TreeKernels.cuh:29
 constexpr int kLevelSlots = 34; // depths 0..32 plus an end slot
@@ -141,6 +160,16 @@ struct DevState {
   uint32_t *arrive;     // bottom-up arrival counters
   // traversal layout (preorder)
   TravNode *tN; // preorder traversal records (32 bytes, one load each)
+  QuadRec *tQ; // records of the default force walk (n + nseg)
+  float4 *tUp; // per traversal record, upward pass: {weighted sums x, y,
+               // bottom size^2, link bits}; shares the breadth-first arrays'
+               // storage (comX ..)
+  // target groups of the default force walk: runs of up to 32 consecutive
+  // bodies that never cross an instance, so that a body's group, and with it
+  // the order of its sums, is the same in an ensemble and on its own
+  uint32_t *groupFirst; // first body of each group (nseg > 1; else 32 g)
+  uint32_t nGroups;
+  uint32_t tgBegin, tgEnd; // groups of [forceBegin, forceEnd)
   float4 *tM; // {Ixx, Iyy, Ixy, size} for the learned correction
   float2 *tC; // square centre, for the learned correction
 

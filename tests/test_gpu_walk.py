@@ -1,0 +1,69 @@
+"""The default force walk (one walk per group of up to 32 bodies) at the
+sizes where groups, lists and records have edges, against the CPU oracle's
+traversal of the same tree."""
+import numpy as np
+import pytest
+
+from conftest import same_bits
+
+pytestmark = pytest.mark.gpu
+
+
+def system(nbx, name, n):
+    b = nbx.cold_square(n, 7)
+    if name == "coincident":  # half the bodies on one point: a chain of 32 nodes
+        b["px"][: n // 2], b["py"][: n // 2] = b["px"][0], b["py"][0]
+    if name == "clumps":  # tight pairs far apart: long chains above each pair
+        k = n // 2
+        b["px"][k:2 * k] = np.nextafter(b["px"][:k], np.float32(1e9))
+        b["py"][k:2 * k] = b["py"][:k]
+    return b
+
+
+def term_sums(b, eps):
+    """Sum over the other bodies of each body's |term| of the force law."""
+    x, y, m = (b[k].astype(np.float64) for k in ("px", "py", "mass"))
+    d2 = (x[:, None] - x) ** 2 + (y[:, None] - y) ** 2
+    return (m / (d2 + eps * eps)).sum(1)
+
+
+@pytest.mark.parametrize("name", ["square", "coincident", "clumps"])
+@pytest.mark.parametrize("n", [1, 2, 16, 17, 31, 32, 33, 64, 65, 97, 1000])
+@pytest.mark.parametrize("leaf,theta", [(16, 1.0), (1, 0.5), (64, 0.5), (3, 2.5), (16, 0.0)])
+def test_group_walk(nbx, oracle, name, n, leaf, theta):
+    b = system(nbx, name, n)
+    try:
+        _, _, _, sb, tree = oracle.morton_build(b, leaf)
+    except RuntimeError:
+        pytest.skip("deeper than the reference's node capacity of 8 n + 8")
+    ox, oy = oracle.tree_forces(sb["px"], sb["py"], sb["mass"], tree, theta, 1.0)
+    sim = nbx.Simulation(b, theta=theta, leaf_capacity=leaf)
+    sim.phase("attract")
+    g = sim.download()
+    sim.close()
+    # n terms of a few rounded operations each, summed in another order: at
+    # most (n + 16) half-ulps of the sum of the terms' sizes; a cell's term is
+    # at most a few times its bodies' (it lies no nearer than they do, to a
+    # factor that theta bounds), hence the 4
+    tol = 4.0 * (n + 16) * 2.0 ** -24 * term_sums(sb, 1.0)
+    err = np.hypot(g["ax"].astype(np.float64) - ox, g["ay"].astype(np.float64) - oy)
+    assert (err <= tol).all(), (err / tol).max()
+
+
+def test_group_walk_instances(nbx):
+    """Instances whose sizes leave ragged groups: the same bits as on their own."""
+    sizes = [1, 33, 2, 31, 32, 65, 500, 17]
+    bodies = np.concatenate([nbx.cold_square(s, 3 + s) for s in sizes])
+    ens = nbx.Handle(sizes, theta=0.5)
+    ens.upload(bodies)
+    ens.phase("attract")
+    got = ens.download()
+    ens.close()
+    start = 0
+    for s in sizes:
+        one = nbx.Handle([s], theta=0.5)
+        one.upload(bodies[start:start + s])
+        one.phase("attract")
+        assert same_bits(got[start:start + s], one.download()), s
+        one.close()
+        start += s
