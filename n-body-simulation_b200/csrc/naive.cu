@@ -11,18 +11,23 @@
 // identity gather in place of the Morton gather so the state alternates
 // between the two buffers exactly as a tree step does.
 //
-// Layout: blocks of 256 threads, two targets per thread (512 per block);
-// the block's sources stream through shared memory in tiles of 256 bodies,
-// one float4 {x, y, m, 0} per body, so each load from shared memory is a
-// broadcast that serves two interactions.  A block whose targets all
-// belong to one instance (every block of a single simulation) runs the
-// unchecked loop; blocks that straddle instances, exact arithmetic and
-// eps = 0 run a loop that checks each source's instance and skips j == i
-// (the reference skips it explicitly; with eps > 0 it adds exactly zero).
+// Default arithmetic with a normal eps^2 (k_naive_pairs): one target per
+// thread, sources through shared memory as arrays of x, y and mass, the law of
+// two sources at a time in paired FP32 instructions and their accumulation
+// one after the other, so every sum keeps its order and rounding.
+// Bound: the FP32 pipe, 9 instructions' worth of it per 32 interactions
+// (paired instructions save issue slots, not pipe time).  65,537 bodies:
+// 3468 -> 1832 us, 131,072: 9568 -> 6090 (2.8e12 interactions/s, 69% of the
+// pipe), 5000: 279 -> 84; before, two targets per thread left 8 warps per SM, and
+// each of the law's 13 instructions (rsqrtf scales subnormal arguments: a
+// compare and two multiplies) waited for the last.  One thread per target
+// gives 14 warps per SM there, 3.5 per scheduler, so an SM ends with its
+// schedulers of 4: 86% of what an even split would give.
 //
-// Bound: FP32 issue (9 FMA-pipe instructions and one MUFU rsqrt per
-// interaction in the default arithmetic), 20 FLOP per interaction by the
-// same convention as the tree force pass.
+// Exact arithmetic, eps = 0 and a subnormal eps^2 run a loop that checks each
+// source's instance and skips j == i (k_naive; the reference skips it
+// explicitly; with eps > 0 it adds exactly zero), as does a block of
+// k_naive_pairs whose targets straddle instances.
 #include "nbx_state.cuh"
 
 #include <float.h>
@@ -30,9 +35,8 @@
 namespace nbx {
 namespace {
 
-constexpr int kNaiveThreads = 256;
-constexpr int kNaiveTargets = 2; // per thread
-constexpr int kNaiveBlockTargets = kNaiveThreads * kNaiveTargets;
+constexpr int kNaiveThreads = 128; // targets per block
+constexpr int kTile = 256;         // sources staged at a time
 
 // Exact: the reference's IEEE operations, no contraction.
 __device__ __forceinline__ void naive_term_exact(float4 q, float x, float y,
@@ -57,76 +61,121 @@ __device__ __forceinline__ void naive_term_fast(float4 q, float x, float y,
   ay = fmaf(dy, f, ay);
 }
 
+// The instances of a block's targets: [lo, hi) covers their bodies, and
+// j0, j1 are the thread's own instance; mixed if the targets' instances differ.
+struct Sources {
+  uint32_t lo, hi, j0, j1;
+  bool mixed;
+};
+__device__ __forceinline__ Sources block_sources(const DevState &S, uint32_t i) {
+  const uint32_t first = blockIdx.x * kNaiveThreads;
+  const uint32_t last = min(first + kNaiveThreads, S.n) - 1u;
+  const uint32_t s0 = S.segOf[first], s1 = S.segOf[last];
+  const SegDev &G0 = S.seg[s0], &G1 = S.seg[s1], &G = S.seg[S.segOf[min(i, last)]];
+  return {G0.start, G1.start + G1.count, G.start, G.start + G.count, s0 != s1};
+}
+
+// Sum over [lo, hi) with the checks.
 template <bool kExact>
-__global__ void __launch_bounds__(kNaiveThreads)
-    k_naive(DevState S, float eSq, int alwaysCheck) {
-  __shared__ float4 tile[kNaiveThreads];
-  __shared__ uint32_t sLo, sHi;
-  __shared__ int sMixed;
-  const uint32_t base0 = blockIdx.x * kNaiveBlockTargets;
-  uint32_t idx[kNaiveTargets], j0[kNaiveTargets], j1[kNaiveTargets];
-  float x[kNaiveTargets], y[kNaiveTargets], ax[kNaiveTargets], ay[kNaiveTargets];
-  if (threadIdx.x == 0) {
-    sLo = 0xffffffffu;
-    sHi = 0u;
-    sMixed = alwaysCheck;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int t = 0; t < kNaiveTargets; ++t) {
-    idx[t] = base0 + t * kNaiveThreads + threadIdx.x;
-    x[t] = y[t] = ax[t] = ay[t] = 0.0f;
-    j0[t] = j1[t] = 0u;
-    if (idx[t] < S.n) {
-      const float4 b = S.xym[idx[t]];
-      x[t] = b.x;
-      y[t] = b.y;
-      const SegDev &G = S.seg[S.segOf[idx[t]]];
-      j0[t] = G.start;
-      j1[t] = G.start + G.count;
-      atomicMin(&sLo, j0[t]);
-      atomicMax(&sHi, j1[t]);
+__device__ __forceinline__ void naive_checked(const DevState &S, const Sources &src, uint32_t i,
+                                              float x, float y, float eSq, float4 *tile,
+                                              float &ax, float &ay) {
+  for (uint32_t base = src.lo; base < src.hi; base += kTile) {
+    const uint32_t cnt = min((uint32_t)kTile, src.hi - base);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < cnt; k += kNaiveThreads) tile[k] = S.xym[base + k];
+    __syncthreads();
+    for (uint32_t k = 0; k < cnt; ++k) {
+      const float4 q = tile[k];
+      const uint32_t j = base + k;
+      if (j < src.j0 || j >= src.j1 || j == i) continue;
+      if (kExact) naive_term_exact(q, x, y, eSq, ax, ay);
+      else naive_term_fast(q, x, y, eSq, ax, ay);
     }
   }
-  __syncthreads();
-  const uint32_t lo = sLo, hi = sHi;
+}
+
+template <bool kExact>
+__global__ void __launch_bounds__(kNaiveThreads) k_naive(DevState S, float eSq) {
+  __shared__ float4 tile[kTile];
+  const uint32_t i = blockIdx.x * kNaiveThreads + threadIdx.x;
+  const Sources src = block_sources(S, i);
+  const float4 b = S.xym[min(i, S.n - 1u)];
+  float ax = 0.0f, ay = 0.0f;
+  naive_checked<kExact>(S, src, i, b.x, b.y, eSq, tile, ax, ay);
+  if (i >= S.n) return;
+  add_attractor<kExact>(S.attr, b.x, b.y, ax, ay);
+  S.acc[i] = make_float2(ax, ay);
+}
+
+// For eps^2 >= FLT_MIN: every s is normal, so the flushing reciprocal square
+// root gives rsqrtf's bits.
+__device__ __forceinline__ float rsqrt_normal(float s) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(s));
+  return r;
+}
+
+__global__ void __launch_bounds__(kNaiveThreads) k_naive_pairs(DevState S, float eSq) {
+  __shared__ float4 tile[kTile]; // or the same bytes as x, y and mass arrays
+  const uint32_t i = blockIdx.x * kNaiveThreads + threadIdx.x;
+  const Sources src = block_sources(S, i);
+  const float4 b = S.xym[min(i, S.n - 1u)];
+  const float x = b.x, y = b.y;
+  float ax = 0.0f, ay = 0.0f;
+  if (src.mixed) {
+    naive_checked<false>(S, src, i, x, y, eSq, tile, ax, ay);
+  } else {
+    float *sx = reinterpret_cast<float *>(tile), *sy = sx + kTile, *sm = sy + kTile;
+    constexpr int kPer = kTile / kNaiveThreads;
+    float4 next[kPer];
+    auto fetch = [&](uint32_t base) {
 #pragma unroll
-  for (int t = 0; t < kNaiveTargets; ++t)
-    if (idx[t] < S.n && (j0[t] != lo || j1[t] != hi)) sMixed = 1;
-  __syncthreads();
-  const bool checked = kExact || sMixed != 0;
-  for (uint32_t base = lo; base < hi; base += kNaiveThreads) {
-    const uint32_t j = base + threadIdx.x;
-    tile[threadIdx.x] = j < hi ? S.xym[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    __syncthreads();
-    const uint32_t cnt = min((uint32_t)kNaiveThreads, hi - base);
-    if (!checked && cnt == kNaiveThreads) {
-#pragma unroll 8
-      for (int k = 0; k < kNaiveThreads; ++k) {
-        const float4 q = tile[k];
-#pragma unroll
-        for (int t = 0; t < kNaiveTargets; ++t) naive_term_fast(q, x[t], y[t], eSq, ax[t], ay[t]);
+      for (int k = 0; k < kPer; ++k) {
+        const uint32_t j = base + k * kNaiveThreads + threadIdx.x;
+        next[k] = j < src.hi ? S.xym[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
-    } else {
-      for (uint32_t k = 0; k < cnt; ++k) {
-        const float4 q = tile[k];
-        const uint32_t jj = base + k;
+    };
+    const f2x XX = pk2(x, x), YY = pk2(y, y), E2 = pk2(eSq, eSq);
+    fetch(src.lo);
+    for (uint32_t base = src.lo; base < src.hi; base += kTile) {
+      __syncthreads();
 #pragma unroll
-        for (int t = 0; t < kNaiveTargets; ++t) {
-          if (jj < j0[t] || jj >= j1[t] || jj == idx[t]) continue;
-          if (kExact) naive_term_exact(q, x[t], y[t], eSq, ax[t], ay[t]);
-          else naive_term_fast(q, x[t], y[t], eSq, ax[t], ay[t]);
+      for (int k = 0; k < kPer; ++k) {
+        sx[k * kNaiveThreads + threadIdx.x] = next[k].x;
+        sy[k * kNaiveThreads + threadIdx.x] = next[k].y;
+        sm[k * kNaiveThreads + threadIdx.x] = next[k].z;
+      }
+      __syncthreads();
+      fetch(base + kTile);
+      // a last partial tile: massless sources to a multiple of four
+      const uint32_t cnt = min((uint32_t)kTile, src.hi - base);
+#pragma unroll 8
+      for (uint32_t k = 0; k < cnt; k += 4) {
+        const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&sx[k]);
+        const ulonglong2 Y = *reinterpret_cast<const ulonglong2 *>(&sy[k]);
+        const ulonglong2 M = *reinterpret_cast<const ulonglong2 *>(&sm[k]);
+        const f2x X2[2] = {X.x, X.y}, Y2[2] = {Y.x, Y.y}, M2[2] = {M.x, M.y};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const f2x DX = sub2(X2[h], XX), DY = sub2(Y2[h], YY);
+          float s0, s1, dx0, dx1, dy0, dy1, f0, f1;
+          upk2(fma2(DX, DX, fma2(DY, DY, E2)), s0, s1);
+          const f2x R = pk2(rsqrt_normal(s0), rsqrt_normal(s1));
+          upk2(mul2(M2[h], mul2(mul2(R, R), R)), f0, f1);
+          upk2(DX, dx0, dx1);
+          upk2(DY, dy0, dy1);
+          ax = fmaf(dx0, f0, ax);
+          ay = fmaf(dy0, f0, ay);
+          ax = fmaf(dx1, f1, ax);
+          ay = fmaf(dy1, f1, ay);
         }
       }
     }
-    __syncthreads();
   }
-#pragma unroll
-  for (int t = 0; t < kNaiveTargets; ++t) {
-    if (idx[t] >= S.n) continue;
-    add_attractor<kExact>(S.attr, x[t], y[t], ax[t], ay[t]);
-    S.acc[idx[t]] = make_float2(ax[t], ay[t]);
-  }
+  if (i >= S.n) return;
+  add_attractor<false>(S.attr, x, y, ax, ay);
+  S.acc[i] = make_float2(ax, ay);
 }
 
 // The naive step's stand-in for the Morton gather: the same buffer swap,
@@ -163,12 +212,10 @@ DevState launch_naive_gather(cudaStream_t s, const DevState &S) {
 // All-pairs accelerations of the bodies in S.xym into S.acc.
 void launch_naive_forces(cudaStream_t s, const DevState &S, bool exact) {
   if (S.n == 0) return;
-  const uint32_t blocks = (S.n + kNaiveBlockTargets - 1) / kNaiveBlockTargets;
-  const int check = S.eSq > 0.0f ? 0 : 1; // eps = 0: skip j == i explicitly
-  if (exact)
-    k_naive<true><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq, 1);
-  else
-    k_naive<false><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq, check);
+  const uint32_t blocks = (S.n + kNaiveThreads - 1) / kNaiveThreads;
+  if (exact) k_naive<true><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
+  else if (S.eSq >= FLT_MIN) k_naive_pairs<<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
+  else k_naive<false><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
 }
 
 } // namespace nbx

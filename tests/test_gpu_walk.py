@@ -67,3 +67,30 @@ def test_group_walk_instances(nbx):
         assert same_bits(got[start:start + s], one.download()), s
         one.close()
         start += s
+
+
+@pytest.mark.parametrize("n", [1, 2, 127, 128, 129, 255, 256, 257, 259, 600])
+@pytest.mark.parametrize("eps", [1.0, 1e-19, 1e-20, 0.0])
+def test_naive_tiles(nbx, oracle, n, eps):
+    """The all-pairs law around its block and tile sizes, with a normal (the
+    paired kernel), a subnormal and a zero eps^2 (the checked one), alone and
+    as an instance that shares blocks with others."""
+    b = nbx.cold_square(n, 5)
+    x, y, m = (b[k].astype(np.float64) for k in ("px", "py", "mass"))
+    dx, dy = x - x[:, None], y - y[:, None]
+    s = dx * dx + dy * dy + float(np.float32(eps)) ** 2
+    with np.errstate(divide="ignore", invalid="ignore"):
+        f = np.where(dx * dx + dy * dy > 0, m / (s * np.sqrt(s)), 0.0)
+    ex, ey = (dx * f).sum(1), (dy * f).sum(1)
+    # n terms of about ten rounded operations each: (n + 16) half-ulps of the
+    # sum of their sizes
+    tol = (n + 16) * 2.0 ** -24 * (np.hypot(dx, dy) * f).sum(1) + 1e-30
+    others = nbx.cold_square(70, 9)
+    for sizes, bodies, at in (([n], b, 0), ([70, n, 70], np.concatenate([others, b, others]), 70)):
+        sim = nbx.Handle(sizes, force_law=1, epsilon=eps)
+        sim.upload(bodies)
+        sim.phase("attract")
+        g = sim.download()[at:at + n]
+        sim.close()
+        err = np.hypot(g["ax"] - ex, g["ay"] - ey)
+        assert (err <= tol).all(), (sizes, (err / tol).max())
