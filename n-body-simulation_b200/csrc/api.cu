@@ -61,8 +61,9 @@ int mlp_rows_per_block();
 void launch_interaction_count(cudaStream_t s, const DevState &S,
                               unsigned long long *counts);
 double fp32_fma_peak_tflops(cudaStream_t s);
-void launch_query_forces(cudaStream_t s, const DevState &S, bool exact,
-                         const float2 *query, uint32_t nq, float2 *out);
+void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool groups,
+                         SortScratch &sort, const float2 *points, uint32_t nq, const float box[4],
+                         float2 *sorted, float2 *accSorted, float2 *acc);
 void launch_direct_fp64(cudaStream_t s, const float4 *pv, const float2 *mr,
                         uint32_t n, const uint32_t *targets, const uint2 *ranges,
                         uint32_t m, double eps, int plummer, double2 *partial,
@@ -286,6 +287,17 @@ struct nbx_handle {
   float attrHost[8] = {0.0f, 0.0f, 1e6f, 50.0f, 0.0f, 0.0f, 0.0f, 0.0f};
   float maxMass = INFINITY; // largest uploaded mass; +inf if any is negative
   FrameWriter *frames = nullptr; // created by the first nbx_nbs2_record
+  float coordLimit = 0.0f; // the last upload's limit (kCtrCoordLimit)
+  // nbx_accel_at's buffers for more points than the handle has bodies (up to
+  // that many it uses the handle's own staging and sort scratch), grown to
+  // its largest call (at most kQueryChunk points; larger calls go in chunks)
+  static constexpr uint32_t kQueryChunk = 1u << 20;
+  struct {
+    uint32_t cap = 0;
+    float2 *host = nullptr; // pinned: points, then accelerations
+    float2 *dev = nullptr;  // [4][cap]: points, sorted, their sums, sums
+    SortScratch sort;
+  } qs;
   // splat renderer buffers, grown on demand
   struct {
     uint32_t bodies = 0, entries = 0, tiles = 0;
@@ -817,6 +829,7 @@ int nbx_params_default(nbx_params *p) {
 static int frames_flush(nbx_handle *h);
 static void frames_destroy(nbx_handle *h);
 static void render_free(nbx_handle *h);
+static void query_free(nbx_handle *h);
 
 int nbx_create(const nbx_params *p, uint32_t num, const uint32_t *sizes,
                nbx_handle **out) {
@@ -864,6 +877,7 @@ int nbx_destroy(nbx_handle *h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   frames_destroy(h);
   render_free(h);
+  query_free(h);
   destroy_graphs(h);
   for (cudaEvent_t ev : h->forceEv) cudaEventDestroy(ev);
   for (cudaEvent_t ev : h->forceMark)
@@ -970,6 +984,7 @@ int nbx_upload_bodies(nbx_handle *h, const nbx_body *bodies, size_t n) {
     if (mm > 0.0f && std::isfinite(mm))
       lim = std::fmin(lim, 1e36f / (static_cast<float>(h->n) * mm));
     std::memcpy(&coordLimitBits, &lim, sizeof(lim));
+    h->coordLimit = lim;
   }
   // the three cell fields of every SegDev and the limit, ordered before
   // the next step on the stream; the pinned words are free again once the
@@ -1399,6 +1414,7 @@ int nbx_reset(nbx_handle *h, const nbx_body *bodies, size_t n) {
   const int frc = frames_flush(h);
   frames_destroy(h);
   render_free(h);
+  query_free(h);
   if (frc != NBX_OK) return fail(h, frc, "writing a recorded NBS2 frame failed");
   // keep the network parameters across the reallocation (optimizer
   // moments start again)
@@ -2081,27 +2097,96 @@ int nbx_mlp_eval(nbx_handle *h, const float *feat, uint32_t n, float *out,
   return rc;
 }
 
+static void query_free(nbx_handle *h) {
+  auto &q = h->qs;
+  void *ptrs[] = {q.dev, q.sort.keys[0], q.sort.keys[1], q.sort.vals[0], q.sort.vals[1],
+                  q.sort.hist, q.sort.status, q.sort.tileCounter};
+  for (void *p : ptrs)
+    if (p) cudaFree(p);
+  if (q.host) cudaFreeHost(q.host);
+  q = {};
+}
+
+// Room for n points.
+static int query_grow(nbx_handle *h, uint32_t n) {
+  auto &q = h->qs;
+  if (q.cap >= n) return NBX_OK;
+  query_free(h);
+  const uint32_t cap = std::max<uint32_t>(n, 1024);
+  SortScratch &so = q.sort;
+  so.capacity = cap;
+  so.maxTiles = (uint32_t)sort_tiles(cap);
+  NBX_CUDA(h, cudaMallocHost(&q.host, cap * sizeof(float2)));
+  NBX_CUDA(h, cudaMalloc(&q.dev, 4 * (size_t)cap * sizeof(float2)));
+  for (int k = 0; k < 2; ++k) {
+    NBX_CUDA(h, cudaMalloc(&so.keys[k], cap * sizeof(uint32_t)));
+    NBX_CUDA(h, cudaMalloc(&so.vals[k], cap * sizeof(uint32_t)));
+  }
+  NBX_CUDA(h, cudaMalloc(&so.hist, 8 * 256 * sizeof(uint32_t)));
+  NBX_CUDA(h, cudaMalloc(&so.tileCounter, 8 * sizeof(uint32_t)));
+  NBX_CUDA(h, cudaMalloc(&so.status, 3 * sort_pass_words(cap) * sizeof(uint32_t)));
+  q.cap = cap; // only once everything is there
+  return NBX_OK;
+}
+
 int nbx_accel_at(nbx_handle *h, const float *px, const float *py, uint32_t nq,
                  float *ax, float *ay) {
   if (!h || (nq && (!px || !py || !ax || !ay))) return NBX_ERR_ARG;
   cudaSetDevice(h->device);
   if (!h->treeValid) return fail(h, NBX_ERR_STATE, "no tree built");
-  if (nq == 0) return NBX_OK;
-  std::vector<float2> q(nq), r(nq);
-  for (uint32_t i = 0; i < nq; ++i) q[i] = make_float2(px[i], py[i]);
-  void *buf = nullptr;
-  int rc = scratch_alloc(h, &buf, 16ull * nq);
-  if (rc) return rc;
-  float2 *dq = (float2 *)buf, *dr = dq + nq;
-  cudaMemcpyAsync(dq, q.data(), 8ull * nq, cudaMemcpyHostToDevice, h->stream);
-  launch_query_forces(h->stream, h->state(), h->params.exact_math != 0, dq, nq, dr);
-  cudaMemcpyAsync(r.data(), dr, 8ull * nq, cudaMemcpyDeviceToHost, h->stream);
-  cudaError_t e = cudaStreamSynchronize(h->stream);
-  scratch_free(h, buf);
-  if (e != cudaSuccess) return cuda_fail(h, e, "accel_at");
-  for (uint32_t i = 0; i < nq; ++i) {
-    ax[i] = r[i].x;
-    ay[i] = r[i].y;
+  for (uint32_t at = 0; at < nq; at += nbx_handle::kQueryChunk) {
+    const uint32_t n = std::min(nq - at, nbx_handle::kQueryChunk);
+    // 8 bytes a point of the pinned body staging, 32 of the device staging's
+    // 36 a body, and the step's sort scratch: all free between calls (every
+    // user of the pinned staging synchronises; the device's is used in stream
+    // order)
+    float2 *host = reinterpret_cast<float2 *>(h->hPinned);
+    float2 *dev0 = reinterpret_cast<float2 *>(h->dAoS);
+    SortScratch *sort = &h->sort;
+    size_t cap = n;
+    if (n > h->n) {
+      const int rc = query_grow(h, n);
+      if (rc != NBX_OK) {
+        query_free(h);
+        return rc;
+      }
+      host = h->qs.host;
+      dev0 = h->qs.dev;
+      sort = &h->qs.sort;
+      cap = h->qs.cap;
+    }
+    // into pinned memory, with the points' box and whether the clamp-free law
+    // may be used at them
+    const float lim = h->coordLimit;
+    float x0 = FLT_MAX, x1 = -FLT_MAX, y0 = FLT_MAX, y1 = -FLT_MAX;
+    bool inside = true;
+    for (uint32_t i = 0; i < n; ++i) {
+      const float x = px[at + i], y = py[at + i];
+      host[i] = make_float2(x, y);
+      x0 = x < x0 ? x : x0;
+      x1 = x > x1 ? x : x1;
+      y0 = y < y0 ? y : y0;
+      y1 = y > y1 ? y : y1;
+      inside &= std::fabs(x) < lim && std::fabs(y) < lim; // NaN: outside
+    }
+    const float w = x1 - x0, ht = y1 - y0;
+    auto scale = [](float e) { return e > 0.0f && e <= FLT_MAX ? 4096.0f / e : 0.0f; };
+    const float box[4] = {x0, y0, scale(w), scale(ht)};
+    float2 *dev[4];
+    for (int k = 0; k < 4; ++k) dev[k] = dev0 + (size_t)k * cap;
+    NBX_CUDA(h, cudaMemcpyAsync(dev[0], host, n * sizeof(float2), cudaMemcpyHostToDevice,
+                                h->stream));
+    launch_query_forces(h->stream, h->state(), h->params.exact_math != 0,
+                        inside && forces_unclamped(h), *sort, dev[0], n, box, dev[1], dev[2],
+                        dev[3]);
+    NBX_CUDA(h, cudaGetLastError());
+    NBX_CUDA(h, cudaMemcpyAsync(host, dev[3], n * sizeof(float2), cudaMemcpyDeviceToHost,
+                                h->stream));
+    NBX_CUDA(h, cudaStreamSynchronize(h->stream));
+    for (uint32_t i = 0; i < n; ++i) {
+      ax[at + i] = host[i].x;
+      ay[at + i] = host[i].y;
+    }
   }
   return NBX_OK;
 }

@@ -480,8 +480,8 @@ class Handle:
         tree with the handle's theta and epsilon."""
         x = np.ascontiguousarray(px, np.float32)
         y = np.ascontiguousarray(py, np.float32)
-        ax = np.zeros(len(x), np.float32)
-        ay = np.zeros(len(x), np.float32)
+        ax = np.empty(len(x), np.float32)
+        ay = np.empty(len(x), np.float32)
         self._c(lib().nbx_accel_at(self.h, x.ctypes.data, y.ctypes.data, len(x),
                                    ax.ctypes.data, ay.ctypes.data))
         return ax, ay

@@ -94,3 +94,51 @@ def test_naive_tiles(nbx, oracle, n, eps):
         sim.close()
         err = np.hypot(g["ax"] - ex, g["ay"] - ey)
         assert (err <= tol).all(), (sizes, (err / tol).max())
+
+
+@pytest.mark.parametrize("nq", [1, 2, 33, 64, 65, 100, 3000, 20001])
+@pytest.mark.parametrize("spread", [1.0, 1e-3, 30.0])
+@pytest.mark.parametrize("theta", [1.0, 0.5, 0.2])
+def test_points(nbx, nq, spread, theta):
+    """Accelerations at points in any order, few and many, close together and
+    far outside: the default arithmetic against the reference's (exact_math)."""
+    b = nbx.cold_square(3000, 1)
+    rng = np.random.default_rng(nq)
+    half = 3.0 * np.sqrt(3000.0) * spread
+    p = rng.uniform(-half, half, (2, nq)).astype(np.float32)
+    p[:, : nq // 3] = p[:, :1]  # many at one place
+    sim = nbx.Simulation(b, theta=theta)
+    sim.phase("build")
+    ax, ay = sim.accel_at(p[0], p[1])
+    sim.set_params(exact_math=1)
+    ex, ey = sim.accel_at(p[0], p[1])
+    sim.close()
+    x, y = b["px"].astype(np.float64), b["py"].astype(np.float64)
+    terms = np.array([(1.0 / ((x - u) ** 2 + (y - v) ** 2 + 1.0)).sum()
+                      for u, v in p.T[:500].astype(np.float64)])
+    err = np.hypot(ax - ex.astype(np.float64), ay - ey.astype(np.float64))[:500]
+    # as in test_group_walk, 3000 terms at most
+    assert (err <= 4.0 * 3016 * 2.0 ** -24 * terms).all()
+    if nq > 500:  # the rest: the same bits as the same points alone
+        again = nbx.Simulation(b, theta=theta)
+        again.phase("build")
+        k = rng.choice(nq, 300, replace=False)
+        sx, sy = again.accel_at(p[0, k], p[1, k])
+        again.close()
+        assert same_bits(sx, ax[k]) and same_bits(sy, ay[k])
+
+
+def test_points_beyond_the_clamp_limit(nbx):
+    """Points where squared distances overflow take the clamped law, and a
+    NaN point stays NaN without touching its neighbours."""
+    b = nbx.cold_square(200, 1)
+    sim = nbx.Simulation(b)
+    sim.phase("build")
+    p = np.array([[1e19, -2e19, 3.0, np.nan, 5.0], [0.0, 1e19, 4.0, 1.0, 6.0]], np.float32)
+    ax, ay = sim.accel_at(p[0], p[1])
+    sim.set_params(exact_math=1)
+    ex, ey = sim.accel_at(p[0], p[1])
+    sim.close()
+    assert np.isnan(ax[3]) and np.isnan(ex[3])
+    k = [0, 1, 2, 4]
+    assert np.allclose(ax[k], ex[k], rtol=1e-4, atol=0) and np.allclose(ay[k], ey[k], rtol=1e-4, atol=0)
