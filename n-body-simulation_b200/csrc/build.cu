@@ -41,16 +41,6 @@ int grid_for(uint32_t n) {
   return b ? (int)b : 1;
 }
 
-// quantise() in native FP64 (TreeKernels.cuh:48-57): one IEEE subtract and
-// one multiply, each rounded (no contraction), then floor -- the same
-// doubles as the reference's, bit for bit, from the frame's binary64 bits.
-__device__ __forceinline__ uint32_t quantise_fp64(float v, double lo, double scale) {
-  const double q = floor(__dmul_rn(__dsub_rn((double)v, lo), scale));
-  if (!(q > 0.0)) return 0u; // also NaN
-  if (q >= 4294967295.0) return 0xFFFFFFFFu;
-  return (uint32_t)q;
-}
-
 // Morton code of every body; the sort key is its high half (depth-16
 // cells), with the digit histograms of its four radix passes fused.
 __global__ void __launch_bounds__(kBlock)
@@ -61,12 +51,7 @@ __global__ void __launch_bounds__(kBlock)
   const uint32_t n = S.n;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += gridDim.x * blockDim.x) {
-    const float4 p = S.pv[i];
-    const MortonFrame f = S.seg[S.segOf[i]].frame;
-    const double sc = __longlong_as_double((long long)f.scale);
-    const uint64_t c =
-        (spread_bits(quantise_fp64(p.y, __longlong_as_double((long long)f.y0), sc)) << 1) |
-        spread_bits(quantise_fp64(p.x, __longlong_as_double((long long)f.x0), sc));
+    const uint64_t c = body_code(S.pv[i], S.seg[S.segOf[i]].frame);
     const uint32_t k = (uint32_t)(c >> 32);
     keys[i] = k;
     S.codes[i] = c;
@@ -813,15 +798,20 @@ void launch_build(cudaStream_t s, DevState &S, ScanScratch &scan,
   mark(s, "build.bounds");
   // digit rows, tile counters, look-back words and the long-run count were
   // cleared by the step prologue (launch_step_zero)
-  k_morton<<<grid_for(n), kBlock, 0, s>>>(S, keys32(sort, 0), sort.hist);
-  mark(s, "build.morton");
-  // radix passes over the codes' high 32 bits (depth-16 cells), then every
-  // run of equal high bits is ordered by its low bits: the same stable order
-  // as a full 64-bit sort; such runs are rare and short (at most 2 bodies in
-  // the headline states), so this replaces four full passes
-  int buf = radix_sort_u32(s, sort, n, nullptr, 0, 32, true, true, S.status, 0, true);
-  sort_fix_low_bits32(s, sort, buf, n, S.codes, S.longRuns, &S.counters[9], n / 16 + 64,
-                      S.status, true);
+  int buf = 0;
+  if (S.nseg == 1 && n <= kClusterMortonMax) {
+    cluster_sort_morton(s, S, sort); // makes the codes too
+  } else {
+    k_morton<<<grid_for(n), kBlock, 0, s>>>(S, keys32(sort, 0), sort.hist);
+    mark(s, "build.morton");
+    // radix passes over the codes' high 32 bits (depth-16 cells), then every
+    // run of equal high bits is ordered by its low bits: the same stable order
+    // as a full 64-bit sort; such runs are rare and short (at most 2 bodies in
+    // the headline states), so this replaces four full passes
+    buf = radix_sort_u32(s, sort, n, nullptr, 0, 32, true, true, S.status, 0, true);
+    sort_fix_low_bits32(s, sort, buf, n, S.codes, S.longRuns, &S.counters[9], n / 16 + 64,
+                        S.status, true);
+  }
   mark(s, "build.sort");
   if (S.nseg > 1) {
     // stable passes on the instance id keep instances in their ranges

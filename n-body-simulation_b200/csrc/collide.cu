@@ -826,8 +826,9 @@ void launch_collide(cudaStream_t s, DevState &S, ScanScratch &scan,
   // grid buckets and large lists
   exclusive_scan_u32(s, S.bucketCount, S.bucketStart, S.nBuckets + 1, nullptr,
                      nullptr, scan, S.status, nullptr, 0, 0);
-  exclusive_scan_u32(s, S.largeCount, S.largeStartA, S.nseg, nullptr, nullptr,
-                     scan, S.status, nullptr, 0, 1);
+  if (S.nseg > 1) // one instance's large list starts at 0 (set once)
+    exclusive_scan_u32(s, S.largeCount, S.largeStartA, S.nseg, nullptr, nullptr,
+                       scan, S.status, nullptr, 0, 1);
   k_fill_grid<<<grid_for(n), kBlock, 0, s>>>(S);
   mark(s, "collide.grid");
   // partners: count (+ stash), scan, fill + sort
@@ -852,10 +853,14 @@ void launch_collide(cudaStream_t s, DevState &S, ScanScratch &scan,
   // units in before() order: a stable sort of all bodies' coarse keys
   // (value = index), then each run of equal coarse keys in exact minX order;
   // the first counters[1] entries are the units
-  const int buf = radix_sort_u32(s, sort, n, nullptr, 0, 24, true, true, S.status,
-                                 kUnitSortSlot, true);
-  sort_fix_units(s, sort, buf, n, S.box, kNonUnitKey, S.longRuns, &S.counters[10],
-                 n / 16 + 64, S.status, true);
+  int buf = 1;
+  if (n <= kClusterSortMax) {
+    cluster_sort_units(s, S, sort, kNonUnitKey);
+  } else {
+    buf = radix_sort_u32(s, sort, n, nullptr, 0, 24, true, true, S.status, kUnitSortSlot, true);
+    sort_fix_units(s, sort, buf, n, S.box, kNonUnitKey, S.longRuns, &S.counters[10],
+                   n / 16 + 64, S.status, true);
+  }
   mark(s, "collide.units");
   // ordered resolution
   if (side) cudaStreamWaitEvent(s, side->join, 0);

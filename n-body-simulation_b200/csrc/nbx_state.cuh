@@ -212,6 +212,23 @@ __device__ __forceinline__ void add_attractor(const float4 *attr, float px, floa
   }
 }
 
+// quantise() in native FP64 (TreeKernels.cuh:48-57): one IEEE subtract and
+// one multiply, each rounded (no contraction), then floor -- the same
+// doubles as the reference's, bit for bit, from the frame's binary64 bits.
+__device__ __forceinline__ uint32_t quantise_fp64(float v, double lo, double scale) {
+  const double q = floor(__dmul_rn(__dsub_rn((double)v, lo), scale));
+  if (!(q > 0.0)) return 0u; // also NaN
+  if (q >= 4294967295.0) return 0xFFFFFFFFu;
+  return (uint32_t)q;
+}
+
+// Morton code of a body at {x, y} in its instance's frame.
+__device__ __forceinline__ uint64_t body_code(float4 p, const MortonFrame &f) {
+  const double sc = __longlong_as_double((long long)f.scale);
+  return (spread_bits(quantise_fp64(p.y, __longlong_as_double((long long)f.y0), sc)) << 1) |
+         spread_bits(quantise_fp64(p.x, __longlong_as_double((long long)f.x0), sc));
+}
+
 __device__ __forceinline__ float key_to_float(uint32_t k) {
   return u2f((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
@@ -250,5 +267,16 @@ __device__ __forceinline__ void root_frame_seg(const DevState &S, uint32_t sg) {
   b[2] = 0xffffffffu;
   b[3] = 0u;
 }
+
+// The step's two sorts for few bodies, one launch each (scan_sort.cu): the
+// Morton codes of a single instance of at most kClusterMortonMax bodies, made
+// here too (the permutation goes to scratch.vals[0]), and the contact units
+// among at most kClusterSortMax bodies, whose keys are in keys32(scratch, 0),
+// every other body's key being nonUnit (the units go to the first places of
+// scratch.vals[1]).
+constexpr uint32_t kClusterMortonMax = 40000, kClusterSortMax = 65536;
+void cluster_sort_morton(cudaStream_t s, const DevState &S, SortScratch &scratch);
+void cluster_sort_units(cudaStream_t s, const DevState &S, SortScratch &scratch,
+                        uint32_t nonUnit);
 
 } // namespace nbx

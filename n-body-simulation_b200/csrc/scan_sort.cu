@@ -17,7 +17,9 @@
 // input order), so equal keys keep their input order exactly as
 // cub::DeviceRadixSort::SortPairs does (CudaQuadTree.cu:405-407), which the
 // Morton permutation parity needs.
-#include "nbx_internal.cuh"
+#include "nbx_state.cuh"
+
+#include <cooperative_groups.h>
 
 namespace nbx {
 
@@ -492,124 +494,133 @@ struct BoxMinX {
 // Runs of up to kShortRun are insertion-sorted by the thread at their
 // start; longer ones are listed for k_long_runs32.
 template <class LowKey>
+__device__ __forceinline__ void fix_run(const uint32_t *keys, uint32_t *vals, uint32_t n,
+                                        uint32_t i, LowKey lowKey, bool hasSkip, uint32_t skip,
+                                        uint32_t *longRuns, uint32_t *longCount, uint32_t cap,
+                                        uint32_t *err) {
+  const uint32_t hi = keys[i];
+  if (hasSkip && hi == skip) return;
+  if (i > 0 && keys[i - 1] == hi) return;      // not a run start
+  if (i + 1 >= n || keys[i + 1] != hi) return; // single key
+  uint32_t len = 2;
+  while (i + len < n && len <= kShortRun && keys[i + len] == hi) ++len;
+  if (len > kShortRun) {
+    const uint32_t slot = atomicAdd(longCount, 1u);
+    if (slot < cap) longRuns[slot] = i;
+    else atomicOr(err, kStatusSpinLimit);
+    return;
+  }
+  uint32_t lk[kShortRun], v[kShortRun];
+  for (uint32_t a = 0; a < len; ++a) {
+    v[a] = vals[i + a];
+    lk[a] = lowKey(v[a]);
+  }
+  for (uint32_t a = 1; a < len; ++a) { // stable: equal keys keep their order
+    const uint32_t kk = lk[a], vv = v[a];
+    uint32_t b = a;
+    while (b > 0 && lk[b - 1] > kk) {
+      lk[b] = lk[b - 1];
+      v[b] = v[b - 1];
+      --b;
+    }
+    lk[b] = kk;
+    v[b] = vv;
+  }
+  for (uint32_t a = 0; a < len; ++a) vals[i + a] = v[a];
+}
+
+template <class LowKey>
 __global__ void __launch_bounds__(256)
     k_fix_runs32(const uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
                  uint32_t n, LowKey lowKey, bool hasSkip, uint32_t skip,
                  uint32_t *__restrict__ longRuns, uint32_t *longCount, uint32_t cap,
                  uint32_t *err) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += gridDim.x * blockDim.x) {
-    const uint32_t hi = keys[i];
-    if (hasSkip && hi == skip) continue;
-    if (i > 0 && keys[i - 1] == hi) continue;      // not a run start
-    if (i + 1 >= n || keys[i + 1] != hi) continue; // single key
-    uint32_t len = 2;
-    while (i + len < n && len <= kShortRun && keys[i + len] == hi) ++len;
-    if (len > kShortRun) {
-      const uint32_t slot = atomicAdd(longCount, 1u);
-      if (slot < cap) longRuns[slot] = i;
-      else atomicOr(err, kStatusSpinLimit);
-      continue;
-    }
-    uint32_t lk[kShortRun], v[kShortRun];
-    for (uint32_t a = 0; a < len; ++a) {
-      v[a] = vals[i + a];
-      lk[a] = lowKey(v[a]);
-    }
-    for (uint32_t a = 1; a < len; ++a) { // stable: equal keys keep their order
-      const uint32_t kk = lk[a], vv = v[a];
-      uint32_t b = a;
-      while (b > 0 && lk[b - 1] > kk) {
-        lk[b] = lk[b - 1];
-        v[b] = v[b - 1];
-        --b;
-      }
-      lk[b] = kk;
-      v[b] = vv;
-    }
-    for (uint32_t a = 0; a < len; ++a) vals[i + a] = v[a];
-  }
+       i += gridDim.x * blockDim.x)
+    fix_run(keys, vals, n, i, lowKey, hasSkip, skip, longRuns, longCount, cap, err);
 }
 
-// One block per long run: its keys are replaced by the in-run keys, a
-// stable LSD radix sort (4 passes, through the other buffer over the same
-// index range) orders the run, and the keys are restored.
-template <class LowKey>
-__global__ void __launch_bounds__(256)
-    k_long_runs32(uint32_t *__restrict__ keys, uint32_t *__restrict__ vals,
-                  uint32_t *__restrict__ tmpK, uint32_t *__restrict__ tmpV, uint32_t n,
-                  LowKey lowKey, const uint32_t *__restrict__ longRuns,
-                  const uint32_t *longCount, uint32_t cap) {
-  __shared__ uint32_t sHist[256], sOff[256], sWarp[8][256];
-  __shared__ uint32_t sEnd;
+// 256 threads order the long runs first, first + step, ..: a run's keys are
+// replaced by the in-run keys, a stable LSD radix sort (4 passes, through the
+// other buffer over the same index range) orders the run, and the keys are
+// restored.  sync() is a barrier of the 256 threads.
+struct LongRunShared {
+  uint32_t hist[256], off[256], warp[8][256];
+  uint32_t end;
+};
+template <class LowKey, class Sync>
+__device__ void order_long_runs(uint32_t *keys, uint32_t *vals, uint32_t *tmpK, uint32_t *tmpV,
+                                uint32_t n, LowKey lowKey, const uint32_t *longRuns,
+                                uint32_t runs, uint32_t first, uint32_t step, LongRunShared &sh,
+                                Sync sync) {
   const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t runs = min(*longCount, cap);
   const uint32_t ltmask = lanemask_lt();
-  for (uint32_t r = blockIdx.x; r < runs; r += gridDim.x) {
+  for (uint32_t r = first; r < runs; r += step) {
     const uint32_t s0 = longRuns[r];
     const uint32_t hi = keys[s0];
-    if (tid == 0) sEnd = n;
-    __syncthreads();
+    if (tid == 0) sh.end = n;
+    sync();
     for (uint32_t base = s0; base < n; base += 256) {
       const uint32_t i = base + tid;
-      if (i < n && keys[i] != hi) atomicMin(&sEnd, i);
-      __syncthreads();
-      const bool found = sEnd != n;
-      __syncthreads(); // every thread has read sEnd before the next tile
+      if (i < n && keys[i] != hi) atomicMin(&sh.end, i);
+      sync();
+      const bool found = sh.end != n;
+      sync(); // every thread has read the end before the next tile
       if (found) break;
     }
-    const uint32_t e0 = sEnd;
+    const uint32_t e0 = sh.end;
     for (uint32_t i = s0 + tid; i < e0; i += 256) keys[i] = lowKey(vals[i]);
-    __syncthreads();
+    sync();
     uint32_t *srcK = keys, *dstK = tmpK, *srcV = vals, *dstV = tmpV;
     for (int p = 0; p < 4; ++p) {
-      const int sh = 8 * p;
-      sHist[tid] = 0;
-      __syncthreads();
-      for (uint32_t i = s0 + tid; i < e0; i += 256) atomicAdd(&sHist[(srcK[i] >> sh) & 255u], 1u);
-      __syncthreads();
+      const int shift = 8 * p;
+      sh.hist[tid] = 0;
+      sync();
+      for (uint32_t i = s0 + tid; i < e0; i += 256)
+        atomicAdd(&sh.hist[(srcK[i] >> shift) & 255u], 1u);
+      sync();
       if (tid == 0) {
         uint32_t run = s0;
         for (int d = 0; d < 256; ++d) {
-          sOff[d] = run;
-          run += sHist[d];
+          sh.off[d] = run;
+          run += sh.hist[d];
         }
       }
-      __syncthreads();
+      sync();
       for (uint32_t base = s0; base < e0; base += 256) {
         const uint32_t i = base + tid;
         const bool ok = i < e0;
         const uint32_t k = ok ? srcK[i] : 0u;
         const uint32_t v = ok ? srcV[i] : 0u;
-        const uint32_t d = ok ? ((k >> sh) & 255u) : 256u;
+        const uint32_t d = ok ? ((k >> shift) & 255u) : 256u;
         uint32_t peers = __ballot_sync(0xffffffffu, ok);
 #pragma unroll
         for (int bit = 0; bit < 8; ++bit) {
           const uint32_t bb = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
           peers &= ((d >> bit) & 1u) ? bb : ~bb;
         }
-        for (int w = 0; w < 8; ++w) sWarp[w][tid] = 0;
-        __syncthreads();
-        if (ok && __popc(peers & ltmask) == 0) sWarp[warp][d] = __popc(peers);
-        __syncthreads();
+        for (int w = 0; w < 8; ++w) sh.warp[w][tid] = 0;
+        sync();
+        if (ok && __popc(peers & ltmask) == 0) sh.warp[warp][d] = __popc(peers);
+        sync();
         {
           uint32_t acc = 0;
           for (int w = 0; w < 8; ++w) {
-            const uint32_t c = sWarp[w][tid];
-            sWarp[w][tid] = acc;
+            const uint32_t c = sh.warp[w][tid];
+            sh.warp[w][tid] = acc;
             acc += c;
           }
-          sHist[tid] = acc; // this tile's count of digit tid
+          sh.hist[tid] = acc; // this tile's count of digit tid
         }
-        __syncthreads();
+        sync();
         if (ok) {
-          const uint32_t dst = sOff[d] + sWarp[warp][d] + __popc(peers & ltmask);
+          const uint32_t dst = sh.off[d] + sh.warp[warp][d] + __popc(peers & ltmask);
           dstK[dst] = k;
           dstV[dst] = v;
         }
-        __syncthreads();
-        sOff[tid] += sHist[tid];
-        __syncthreads();
+        sync();
+        sh.off[tid] += sh.hist[tid];
+        sync();
       }
       uint32_t *tk = srcK;
       srcK = dstK;
@@ -620,8 +631,18 @@ __global__ void __launch_bounds__(256)
     }
     // four passes: the result is back in keys/vals; restore the run's keys
     for (uint32_t i = s0 + tid; i < e0; i += 256) keys[i] = hi;
-    __syncthreads();
+    sync();
   }
+}
+
+template <class LowKey>
+__global__ void __launch_bounds__(256)
+    k_long_runs32(uint32_t *keys, uint32_t *vals, uint32_t *tmpK, uint32_t *tmpV, uint32_t n,
+                  LowKey lowKey, const uint32_t *longRuns, const uint32_t *longCount,
+                  uint32_t cap) {
+  __shared__ LongRunShared sh;
+  order_long_runs(keys, vals, tmpK, tmpV, n, lowKey, longRuns, min(*longCount, cap), blockIdx.x,
+                  gridDim.x, sh, [] { __syncthreads(); });
 }
 
 } // namespace
@@ -715,6 +736,298 @@ int radix_sort_u32(cudaStream_t s, SortScratch &sc, uint32_t n_max,
   uint32_t *const keys[2] = {keys32(sc, 0), keys32(sc, 1)};
   return radix_sort<uint32_t>(s, sc, keys, n_max, d_n, bit_lo, bit_hi, vals_identity,
                               have_hist, err, slot, zeroed);
+}
+
+// ------------------------------------------------- sorts of few elements
+//
+// Up to kClusterSortMax elements are sorted by one launch: a cluster of eight
+// blocks (one block up to 1024) holds keys and values in its shared memory,
+// split evenly, and each pass scatters them to their places in the blocks'
+// shared memory.  The passes are those of the radix sort above
+// (warp-striped ranks from ballots, stable), the blocks exchange their digit
+// counts in place of the look-back, and the runs of equal keys are ordered in
+// the same launch, so the permutation is the same.
+// Latency bound: a pass is two cluster barriers, ranks and a scatter, 3 us at
+// 8000 elements, where one launch per pass took 7, and its clears, histogram
+// and two run passes 2 to 5 each.  us with the Morton codes / the units, before
+// -> now, at 1000 bodies: 47 -> 14 / 33 -> 12, at 8000: 57 -> 20 / 37 -> 16, at
+// 32,000: 61 -> 43 / 40 -> 18, at 65,000: 63 -> 70 / 42 -> 22.  The eight SMs
+// take 0.8 us per 1000 elements, so the codes keep a launch per pass beyond
+// kClusterMortonMax; the units are few of the bodies.
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr uint32_t kOneBlockMax = 1024;
+
+template <int T, int K> struct alignas(16) ClusterShared {
+  uint2 kv[2][T * K]; // {key, value}: one store to a neighbour
+  uint16_t warpHist[T / 32][258]; // 2 over: rows 8 apart start 8 banks apart
+  uint32_t count[256]; // read by the other blocks
+  uint32_t off[256];
+  uint32_t sums[32];
+  LongRunShared runs;
+};
+
+__device__ __forceinline__ uint32_t round32(uint32_t v) { return (v + 31u) & ~31u; }
+
+// The Morton codes of all bodies of a single instance, made here (k_morton's
+// arithmetic), sorted by their high halves with the low halves' order inside
+// runs.
+struct MortonSource {
+  DevState S;
+  static constexpr bool kAll = true;
+  static constexpr int kPasses = 4;
+  __device__ uint32_t key(uint32_t i) const {
+    const uint64_t c = body_code(S.pv[i], S.seg[0].frame);
+    S.codes[i] = c;
+    return (uint32_t)(c >> 32);
+  }
+  __device__ bool chosen(uint32_t) const { return true; }
+  __device__ uint32_t operator()(uint32_t v) const { return (uint32_t)__ldcg(&S.codes[v]); }
+};
+// The units among the bodies: their coarse keys, the exact minX inside runs.
+struct UnitSource {
+  const uint32_t *keys;
+  const float4 *box;
+  uint32_t nonUnit;
+  static constexpr bool kAll = false;
+  static constexpr int kPasses = 3;
+  __device__ uint32_t key(uint32_t i) const { return keys[i]; }
+  __device__ bool chosen(uint32_t key) const { return key != nonUnit; }
+  __device__ uint32_t operator()(uint32_t v) const { return float_order_key(box[v].x); }
+};
+
+// B blocks of T threads with up to K elements each.
+template <int B, int T, int K, class Source>
+__global__ void __cluster_dims__(B, 1, 1) __launch_bounds__(T, 1)
+    k_cluster_sort(Source src, uint32_t n, uint32_t *keysOut, uint32_t *valsOut, uint32_t *tmpK,
+                   uint32_t *tmpV, uint32_t *longRuns, uint32_t *longCount, uint32_t cap,
+                   uint32_t *err) {
+  extern __shared__ uint4 sDyn[];
+  ClusterShared<T, K> &sh = *reinterpret_cast<ClusterShared<T, K> *>(sDyn);
+  constexpr uint32_t kWarps = T / 32;
+  cg::cluster_group cluster = cg::this_cluster();
+  const uint32_t me = B > 1 ? cluster.block_rank() : 0u;
+  auto sync_all = [&] {
+    if (B > 1) cluster.sync();
+    else __syncthreads();
+  };
+  auto of_block = [&](auto *p, uint32_t b) { return B > 1 ? cluster.map_shared_rank(p, b) : p; };
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t ltmask = lanemask_lt();
+  // element k of a lane: warp * 32 per + 32 k + lane of the block's chunk
+  uint32_t total = n, chunk = round32((n + B - 1) / B);
+  uint32_t per = (chunk + T - 1) / T; // <= K
+  uint32_t key[K], val[K];
+  auto element = [&](int k) { return warp * 32u * per + 32u * k + lane; };
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const uint32_t l = element(k), i = me * chunk + l;
+    val[k] = (uint32_t)k < per && l < chunk && i < n ? i : 0xffffffffu;
+    key[k] = val[k] != 0xffffffffu ? src.key(i) : 0u;
+  }
+  // place dest's block: dest / chunk, exact for dest < 2^16, chunk <= 2^13
+  uint32_t magic = 0xffffffffu / chunk + 1u;
+  auto put = [&](int buf, uint32_t dest, uint32_t k, uint32_t v) {
+    const uint32_t b = __umulhi(dest, magic);
+    *of_block(&sh.kv[buf][dest - b * chunk], b) = make_uint2(k, v);
+  };
+  int cur = 0;
+  if (!Source::kAll) {
+    // the chosen elements, in order, to the first chunks
+    uint32_t mine = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (val[k] != 0xffffffffu && !src.chosen(key[k])) val[k] = 0xffffffffu;
+      mine += __popc(__ballot_sync(0xffffffffu, val[k] != 0xffffffffu));
+    }
+    if (lane == 0) sh.sums[warp] = mine;
+    __syncthreads();
+    if (warp == 0) {
+      const uint32_t v = lane < kWarps ? sh.sums[lane] : 0u;
+      uint32_t inc = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+      }
+      sh.sums[lane] = inc - v;
+      if (lane == 31) sh.count[0] = inc;
+    }
+    sync_all();
+    uint32_t before = 0;
+    total = 0;
+    for (int b = 0; b < B; ++b) {
+      const uint32_t c = *of_block(&sh.count[0], (uint32_t)b);
+      before += b < (int)me ? c : 0u;
+      total += c;
+    }
+    chunk = round32((total + B - 1) / B);
+    if (total == 0) chunk = 32;
+    per = (chunk + T - 1) / T;
+    magic = 0xffffffffu / chunk + 1u;
+    uint32_t dest = before + sh.sums[warp];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const uint32_t have = __ballot_sync(0xffffffffu, val[k] != 0xffffffffu);
+      if (val[k] != 0xffffffffu) put(0, dest + __popc(have & ltmask), key[k], val[k]);
+      dest += __popc(have);
+    }
+    sync_all();
+    if (total == 0) return;
+  }
+  for (int p = 0; p < Source::kPasses; ++p) {
+    const int shift = 8 * p;
+    if (p > 0 || !Source::kAll) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        key[k] = 0u;
+        val[k] = 0xffffffffu;
+        if ((uint32_t)k >= per) continue;
+        const uint32_t l = element(k);
+        const bool ok = l < chunk && me * chunk + l < total;
+        const uint2 e = ok ? sh.kv[cur][l] : make_uint2(0u, 0xffffffffu);
+        key[k] = e.x;
+        val[k] = e.y;
+      }
+    }
+    uint32_t *hist32 = reinterpret_cast<uint32_t *>(sh.warpHist[warp]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) hist32[lane + 32 * q] = 0u;
+    __syncwarp();
+    uint32_t rank[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      rank[k] = 0;
+      if ((uint32_t)k >= per) continue;
+      const uint32_t d = (key[k] >> shift) & 255u;
+      const bool ok = val[k] != 0xffffffffu;
+      uint32_t peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+      for (int bit = 0; bit < 8; ++bit) {
+        const uint32_t bb = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
+        peers &= ((d >> bit) & 1u) ? bb : ~bb;
+      }
+      const uint32_t before = __popc(peers & ltmask);
+      uint32_t b = 0;
+      if (ok) b = sh.warpHist[warp][d];
+      __syncwarp();
+      if (ok && before == 0) sh.warpHist[warp][d] = (uint16_t)(b + __popc(peers));
+      __syncwarp();
+      rank[k] = b + before;
+    }
+    __syncthreads();
+    { // exclusive over the warps: T / 256 lanes to a digit, eight warps to a lane
+      constexpr uint32_t kLanes = T / 256;
+      static_assert(kLanes * 256 == T && kLanes <= 4, "whole digits, at most four lanes");
+      const uint32_t part = tid % kLanes, d = tid / kLanes, w0 = part * 8u;
+      uint32_t h[8], sum = 0;
+#pragma unroll
+      for (uint32_t w = 0; w < 8; ++w) {
+        h[w] = sh.warpHist[w0 + w][d];
+        sum += h[w];
+      }
+      uint32_t inc = sum;
+#pragma unroll
+      for (uint32_t o = 1; o < kLanes; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (part >= o) inc += t;
+      }
+      uint32_t c = inc - sum;
+#pragma unroll
+      for (uint32_t w = 0; w < 8; ++w) {
+        sh.warpHist[w0 + w][d] = (uint16_t)c;
+        c += h[w];
+      }
+      if (part == kLanes - 1) sh.count[d] = inc;
+    }
+    sync_all();
+    if (tid < 256) {
+      uint32_t before = 0, all = 0;
+#pragma unroll
+      for (int b = 0; b < B; ++b) {
+        const uint32_t c = *of_block(&sh.count[tid], (uint32_t)b);
+        before += b < (int)me ? c : 0u;
+        all += c;
+      }
+      uint32_t inc = all;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+      }
+      if (lane == 31) sh.sums[warp] = inc;
+      sh.off[tid] = inc - all + before;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t o = 0;
+#pragma unroll
+      for (uint32_t w = 0; w < 8; ++w) o += w < warp ? sh.sums[w] : 0u;
+      sh.off[tid] += o;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if ((uint32_t)k >= per || val[k] == 0xffffffffu) continue;
+      const uint32_t d = (key[k] >> shift) & 255u;
+      put(cur ^ 1, sh.off[d] + sh.warpHist[warp][d] + rank[k], key[k], val[k]);
+    }
+    cur ^= 1;
+    sync_all();
+  }
+  // to global memory; then the runs of equal keys there
+  const uint32_t base = me * chunk;
+  const uint32_t count = base < total ? min(chunk, total - base) : 0u;
+  for (uint32_t l = tid; l < count; l += T) {
+    const uint2 e = sh.kv[cur][l];
+    keysOut[base + l] = e.x;
+    valsOut[base + l] = e.y;
+  }
+  sync_all();
+  for (uint32_t l = tid; l < count; l += T)
+    fix_run(keysOut, valsOut, total, base + l, src, false, 0u, longRuns, longCount, cap, err);
+  sync_all();
+  const uint32_t runs = min(__ldcg(longCount), cap);
+  if (runs != 0 && tid < 256)
+    order_long_runs(keysOut, valsOut, tmpK, tmpV, total, src, longRuns, runs, me, B,
+                    sh.runs, [] { asm volatile("bar.sync 1, 256;" ::: "memory"); });
+}
+
+template <int B, int T, int K, class Source>
+void cluster_sort(cudaStream_t s, const Source &src, uint32_t n, SortScratch &sc, int out,
+                  uint32_t *longRuns, uint32_t *longCount, uint32_t cap, uint32_t *err) {
+  constexpr int smem = (int)sizeof(ClusterShared<T, K>);
+  static_assert(B * T * K <= 65536 && smem <= 227 * 1024, "16-bit places, one block per SM");
+  cudaFuncSetAttribute(k_cluster_sort<B, T, K, Source>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  k_cluster_sort<B, T, K, Source><<<B, T, smem, s>>>(src, n, keys32(sc, out), sc.vals[out],
+                                                     keys32(sc, out ^ 1), sc.vals[out ^ 1],
+                                                     longRuns, longCount, cap, err);
+}
+
+template <class Source>
+void cluster_sort(cudaStream_t s, const Source &src, uint32_t n, SortScratch &sc, int out,
+                  uint32_t *longRuns, uint32_t *longCount, uint32_t cap, uint32_t *err) {
+  if (n <= kOneBlockMax)
+    cluster_sort<1, 1024, 1>(s, src, n, sc, out, longRuns, longCount, cap, err);
+  else if (n <= 16384)
+    cluster_sort<8, 512, 4>(s, src, n, sc, out, longRuns, longCount, cap, err);
+  else
+    cluster_sort<8, 512, 16>(s, src, n, sc, out, longRuns, longCount, cap, err);
+}
+
+} // namespace
+
+void cluster_sort_morton(cudaStream_t s, const DevState &S, SortScratch &sc) {
+  cluster_sort(s, MortonSource{S}, S.n, sc, 0, S.longRuns, &S.counters[9], S.n / 16 + 64,
+               S.status);
+}
+
+void cluster_sort_units(cudaStream_t s, const DevState &S, SortScratch &sc, uint32_t nonUnit) {
+  cluster_sort(s, UnitSource{keys32(sc, 0), S.box, nonUnit}, S.n, sc, 1, S.longRuns,
+               &S.counters[10], S.n / 16 + 64, S.status);
 }
 
 } // namespace nbx
