@@ -33,7 +33,7 @@ void launch_step_zero(cudaStream_t s, const DevState &S, ScanScratch &scan, Sort
                       bool grid);
 void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
                    const MlpDev *mlp, float band, int corr, bool noClamp, int threads,
-                   bool pairs);
+                   bool pairs, bool chained);
 void render_vertices(cudaStream_t s, const float4 *pv, const float2 *mr, uint32_t n,
                      const RenderParams &P, float4 *v0, float4 *v1, uint32_t *tiles,
                      double4 *partial, unsigned long long *total, float *stats);
@@ -574,7 +574,7 @@ void enqueue_forces_io(nbx_handle *h, cudaStream_t s, const DevState &S) {
     R.recOut = reinterpret_cast<uint32_t *>(h->dAoS);
     launch_forces(cs, R, h->params.exact_math != 0, h->params.force_blocks,
                   h->mlpLoaded ? h->mlpW : nullptr, h->params.mlp_band, h->params.use_mlp,
-                  forces_unclamped(h), h->params.force_block, h->params.leaf_pairs != 0);
+                  forces_unclamped(h), h->params.force_block, h->params.leaf_pairs != 0, false);
     cudaMemcpyAsync(h->ioOut + b, h->dAoS + b, (size_t)(e - b) * sizeof(nbx_body),
                     cudaMemcpyDeviceToHost, cs);
     cudaEventRecord(h->ioDone[c], cs);
@@ -608,7 +608,7 @@ DevState enqueue_step(nbx_handle *h, cudaStream_t s, DevState S) {
   launch_forces(s, S, h->params.exact_math != 0, h->params.force_blocks,
                 h->mlpLoaded ? h->mlpW : nullptr, h->params.mlp_band,
                 h->params.use_mlp, forces_unclamped(h), h->params.force_block,
-                h->params.leaf_pairs != 0);
+                h->params.leaf_pairs != 0, !h->timedCapture);
   if (h->timedCapture) cudaEventRecordWithFlags(h->forceMark[1], s, cudaEventRecordExternal);
   mark(s, "forces");
   return S;
@@ -1515,7 +1515,7 @@ int nbx_phase(nbx_handle *h, int phase) {
     launch_forces(s, S, h->params.exact_math != 0, h->params.force_blocks,
                   h->mlpLoaded ? h->mlpW : nullptr, h->params.mlp_band,
                   h->params.use_mlp, forces_unclamped(h), h->params.force_block,
-                h->params.leaf_pairs != 0);
+                  h->params.leaf_pairs != 0, false);
     break;
   case NBX_PHASE_ATTRACT:
     if (h->params.force_law == 1) {
@@ -1536,7 +1536,7 @@ int nbx_phase(nbx_handle *h, int phase) {
     launch_forces(s, S, h->params.exact_math != 0, h->params.force_blocks,
                   h->mlpLoaded ? h->mlpW : nullptr, h->params.mlp_band,
                   h->params.use_mlp, forces_unclamped(h), h->params.force_block,
-                h->params.leaf_pairs != 0);
+                  h->params.leaf_pairs != 0, false);
     break;
   case NBX_PHASE_STEP:
     enqueue_step(h, s, S);

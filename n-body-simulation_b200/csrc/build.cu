@@ -45,6 +45,7 @@ int grid_for(uint32_t n) {
 // cells), with the digit histograms of its four radix passes fused.
 __global__ void __launch_bounds__(kBlock)
     k_morton(DevState S, uint32_t *__restrict__ keys, uint32_t *hist) {
+  chain_begin();
   __shared__ uint32_t sh[4][256];
   for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) sh[i >> 8][i & 255] = 0;
   __syncthreads();
@@ -453,6 +454,7 @@ __global__ void __launch_bounds__(kBlock) k_upward(DevState S) {
 constexpr int kMaxLeafCap = 64; // nbx_params leaf_capacity bound
 __global__ void __launch_bounds__(kBlock)
     k_gather_counts(DevState S, const uint32_t *__restrict__ perm) {
+  chain_begin();
   __shared__ uint64_t sC[kBlock + 2 * kMaxLeafCap];
   __shared__ int8_t sHi[kBlock + kMaxLeafCap];
   const uint32_t n = S.n;
@@ -563,6 +565,7 @@ __device__ __forceinline__ uint32_t record_of(const DevState &S, uint32_t b, int
 template <bool kFull>
 __global__ void __launch_bounds__(kBlock)
     k_trav_nodes(DevState S, const uint32_t *__restrict__ owner, uint4 *__restrict__ kids) {
+  chain_begin();
   const uint64_t *c = S.sortedCodes;
   const uint32_t total = S.counters[6];
   const bool overflow = total > S.nodeCapacity;
@@ -687,6 +690,7 @@ __device__ __forceinline__ void quad_root(const DevState &S, uint32_t b, float4 
 template <bool kMoments>
 __global__ void __launch_bounds__(kBlock)
     k_trav_upward(DevState S, const uint4 *__restrict__ kids) {
+  chain_begin();
   const uint32_t total = S.counters[6];
   if (total > S.nodeCapacity) return;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total;
@@ -802,7 +806,7 @@ void launch_build(cudaStream_t s, DevState &S, ScanScratch &scan,
   if (S.nseg == 1 && n <= kClusterMortonMax) {
     cluster_sort_morton(s, S, sort); // makes the codes too
   } else {
-    k_morton<<<grid_for(n), kBlock, 0, s>>>(S, keys32(sort, 0), sort.hist);
+    launch_after(s, k_morton, grid_for(n), kBlock, 0, S, keys32(sort, 0), sort.hist);
     mark(s, "build.morton");
     // radix passes over the codes' high 32 bits (depth-16 cells), then every
     // run of equal high bits is ordered by its low bits: the same stable order
@@ -825,7 +829,7 @@ void launch_build(cudaStream_t s, DevState &S, ScanScratch &scan,
     const int segBits = S.nseg <= 256 ? 8 : 16;
     buf = radix_sort_u32(s, sort, n, nullptr, 0, segBits, false, false, S.status);
   }
-  k_gather_counts<<<grid_for(n), kBlock, 0, s>>>(S, sort.vals[buf]);
+  launch_after(s, k_gather_counts, grid_for(n), kBlock, 0, S, sort.vals[buf]);
   mark(s, "build.gather");
   // swap the double-buffered state: the host mirrors this swap
   DevState T = S;
@@ -853,14 +857,14 @@ void launch_trav_tree(cudaStream_t s, const DevState &S, ScanScratch &scan, bool
                      scan, S.status, owner, S.nodeCapacity, 3);
   mark(s, "tree.counts");
   if (moments)
-    k_trav_nodes<true><<<grid_for(n / 2 + 64), kBlock, 0, s>>>(S, owner, kids);
+    launch_after(s, k_trav_nodes<true>, grid_for(n / 2 + 64), kBlock, 0, S, owner, kids);
   else
-    k_trav_nodes<false><<<grid_for(n / 2 + 64), kBlock, 0, s>>>(S, owner, kids);
+    launch_after(s, k_trav_nodes<false>, grid_for(n / 2 + 64), kBlock, 0, S, owner, kids);
   mark(s, "tree.nodes");
   if (moments)
-    k_trav_upward<true><<<grid_for(n / 4 + 64), kBlock, 0, s>>>(S, kids);
+    launch_after(s, k_trav_upward<true>, grid_for(n / 4 + 64), kBlock, 0, S, kids);
   else
-    k_trav_upward<false><<<grid_for(n / 4 + 64), kBlock, 0, s>>>(S, kids);
+    launch_after(s, k_trav_upward<false>, grid_for(n / 4 + 64), kBlock, 0, S, kids);
   mark(s, "tree.upward");
 }
 

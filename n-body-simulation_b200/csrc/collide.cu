@@ -125,6 +125,7 @@ __device__ __forceinline__ bool is_small(const float4 &bx, float smallW) {
 // grid cell and a slot in its bucket (or in its instance's large list).
 __global__ void __launch_bounds__(kBlock)
     k_integrate_boxes(DevState S, int integrate, int collide) {
+  chain_begin();
   const uint32_t n = S.n;
   const float dt = S.dt;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -173,6 +174,7 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 __global__ void __launch_bounds__(kBlock) k_fill_grid(DevState S) {
+  chain_begin();
   const uint32_t n = S.n;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += gridDim.x * blockDim.x) {
@@ -230,6 +232,7 @@ __device__ __forceinline__ void for_each_cell_neighbour(const DevState &S, uint3
 // first kStash partners are stashed so that the fill pass need not search
 // again; small-large pairs are appended for the large body's list.
 __global__ void __launch_bounds__(kBlock) k_partners_count(DevState S) {
+  chain_begin();
   const uint32_t n = S.n;
   const uint32_t mask = S.nBuckets - 1;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -316,6 +319,7 @@ __device__ __forceinline__ void flush_unit_hist(uint32_t (*sh)[256], uint32_t un
 // key and its digit counts come out too.
 __global__ void __launch_bounds__(kBlock)
     k_partners_fill(DevState S, uint32_t *__restrict__ keys, uint32_t *hist) {
+  chain_begin();
   __shared__ uint32_t sh[3][256];
   __shared__ uint32_t sUnits;
   for (int q = threadIdx.x; q < 3 * 256; q += blockDim.x) sh[q >> 8][q & 255] = 0;
@@ -402,6 +406,7 @@ __global__ void __launch_bounds__(kBlock)
 // by before() order: one warp per large body, rank by counting.
 __global__ void __launch_bounds__(kBlock)
     k_sort_large(DevState S, uint32_t *__restrict__ keys, uint32_t *hist) {
+  chain_begin();
   const int lane = threadIdx.x & 31;
   const uint32_t warpId = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const uint32_t nWarps = (gridDim.x * blockDim.x) >> 5;
@@ -548,6 +553,7 @@ __device__ __forceinline__ bool published(const float4 &v) {
 // first or last entry; computed in bulk so the resolution does not search.
 // Also presets every chain record of the body to the sentinel.
 __global__ void __launch_bounds__(kBlock) k_twins(DevState S) {
+  chain_begin();
   if (S.counters[0] > S.pairCapacity) return;
   const float4 unset = make_float4(__uint_as_float(kUnpublished), __uint_as_float(kUnpublished),
                                    __uint_as_float(kUnpublished), __uint_as_float(kUnpublished));
@@ -576,6 +582,7 @@ __global__ void __launch_bounds__(kBlock) k_twins(DevState S) {
 // advances.  The next pair's partner is fetched while the current one waits.
 __global__ void __launch_bounds__(kBlock)
     k_resolve(DevState S, const uint32_t *__restrict__ units) {
+  chain_begin();
   const uint32_t numUnits = S.counters[1];
   const int lane = threadIdx.x & 31;
   if (S.counters[0] > S.pairCapacity) return;
@@ -668,6 +675,7 @@ __global__ void __launch_bounds__(kBlock)
 // instance, flushed with atomics otherwise.  The last block to finish sets
 // every instance's root square and Morton frame (root_frame_seg).
 __global__ void __launch_bounds__(kBlock) k_bounds(DevState S) {
+  chain_begin();
   const uint32_t n = S.n;
   const uint32_t chunk = (n + gridDim.x - 1) / gridDim.x;
   const uint32_t c0 = blockIdx.x * chunk;
@@ -765,6 +773,7 @@ struct ZeroRanges {
 
 // Clears every range (16-byte aligned ranges with 16-byte stores).
 __global__ void __launch_bounds__(kBlock) k_zero_ranges(ZeroRanges z) {
+  chain_begin();
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   for (int r = 0; r < z.count; ++r) {
     uint32_t *p = z.p[r];
@@ -816,8 +825,8 @@ void launch_step_zero(cudaStream_t s, const DevState &S, ScanScratch &scan, Sort
 // Host-side sequencing of the collision phase (no host synchronisation).
 void launch_integrate(cudaStream_t s, const DevState &S, bool integrate,
                       bool collide) {
-  k_integrate_boxes<<<grid_for(S.n), kBlock, 0, s>>>(S, integrate ? 1 : 0,
-                                                     collide ? 1 : 0);
+  launch_after(s, k_integrate_boxes, grid_for(S.n), kBlock, 0, S, integrate ? 1 : 0,
+               collide ? 1 : 0);
 }
 
 void launch_collide(cudaStream_t s, DevState &S, ScanScratch &scan,
@@ -829,18 +838,18 @@ void launch_collide(cudaStream_t s, DevState &S, ScanScratch &scan,
   if (S.nseg > 1) // one instance's large list starts at 0 (set once)
     exclusive_scan_u32(s, S.largeCount, S.largeStartA, S.nseg, nullptr, nullptr,
                        scan, S.status, nullptr, 0, 1);
-  k_fill_grid<<<grid_for(n), kBlock, 0, s>>>(S);
+  launch_after(s, k_fill_grid, grid_for(n), kBlock, 0, S);
   mark(s, "collide.grid");
   // partners: count (+ stash), scan, fill + sort
-  k_partners_count<<<grid_for(n), kBlock, 0, s>>>(S);
+  launch_after(s, k_partners_count, grid_for(n), kBlock, 0, S);
   exclusive_scan_u32(s, S.deg, S.pstart, n, nullptr, &S.counters[0], scan,
                      S.status, nullptr, 0, 2);
   mark(s, "collide.count");
   // the fill kernels also write every body's key for the units' sort
   // (units first, in before() order) and its digit histograms
   uint32_t *unitHist = sort.hist + kUnitSortSlot * 256;
-  k_partners_fill<<<grid_for(n), kBlock, 0, s>>>(S, keys32(sort, 0), unitHist);
-  k_sort_large<<<64, kBlock, 0, s>>>(S, keys32(sort, 0), unitHist);
+  launch_after(s, k_partners_fill, grid_for(n), kBlock, 0, S, keys32(sort, 0), unitHist);
+  launch_after(s, k_sort_large, 64, kBlock, 0, S, keys32(sort, 0), unitHist);
   mark(s, "collide.fill");
   // the pairs' chain entries (k_twins) need only the sorted lists: they
   // run beside the units' sort, on the side stream when there is one
@@ -865,6 +874,7 @@ void launch_collide(cudaStream_t s, DevState &S, ScanScratch &scan,
   // ordered resolution
   if (side) cudaStreamWaitEvent(s, side->join, 0);
   else k_twins<<<grid_for(n), kBlock, 0, s>>>(S);
+  // after two branches (or none): an ordinary launch
   k_resolve<<<148 * 8, kBlock, 0, s>>>(S, sort.vals[buf]);
   mark(s, "collide.resolve");
 }
@@ -873,7 +883,7 @@ void launch_bounds(cudaStream_t s, const DevState &S) {
   uint32_t blocks = (S.n + 1023) / 1024; // 4 bodies per thread
   if (blocks > 148u * 8u) blocks = 148u * 8u;
   if (blocks < 1) blocks = 1;
-  k_bounds<<<blocks, kBlock, 0, s>>>(S);
+  launch_after(s, k_bounds, blocks, kBlock, 0, S);
 }
 
 } // namespace nbx

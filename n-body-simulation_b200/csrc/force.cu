@@ -868,6 +868,7 @@ __global__ void __launch_bounds__(kBlock, kCorr == 1 ? 3
              const MlpDev *__restrict__ mlp = nullptr, float bandSq = 0.0f,
              float eps = 0.0f, const float2 *__restrict__ query = nullptr,
              uint32_t nQuery = 0, float2 *__restrict__ queryAcc = nullptr) {
+  chain_begin();
   constexpr int kBlockWarps = kBlock / 32;
   constexpr int kStage = kCorr == 1 ? kBlockWarps : 1;
   __shared__ float4 sBody[kBlockWarps][32];
@@ -943,6 +944,7 @@ template <int kBlock>
 __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
                                               ? kGroupWarpsPerSM * 32 / kBlock : 1)
     k_forces_groups(DevState S, float tSq, float eSq) {
+  chain_begin();
   extern __shared__ uint4 sDyn[]; // a WalkStage per warp
   const int lane = threadIdx.x & 31;
   WalkStage &st = reinterpret_cast<WalkStage *>(sDyn)[threadIdx.x >> 5];
@@ -1099,7 +1101,8 @@ bool group_walk_fits(const DevState &S) {
 // The default plain walk with kBlock threads per block and the paired or
 // single-body leaf loop.
 template <int kBlock>
-void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, bool groups) {
+void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, bool groups,
+                  bool chained) {
   if (blocks <= 0) {
     uint32_t warps = (force_targets(S) + 31) / 32;
     const uint32_t per = kBlock / 32;
@@ -1112,7 +1115,10 @@ void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, boo
     if (smem > 48 * 1024) // above what a launch may ask for by default
       cudaFuncSetAttribute(k_forces_groups<kBlock>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k_forces_groups<kBlock><<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq);
+    if (chained)
+      launch_after(s, k_forces_groups<kBlock>, blocks, kBlock, smem, S, S.tSq, S.eSq);
+    else
+      k_forces_groups<kBlock><<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq);
   }
   else if (pairs)
     k_forces<false, false, 0, false, kBlock, true><<<blocks, kBlock, 0, s>>>(S, S.tSq, S.eSq);
@@ -1172,17 +1178,18 @@ void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool gro
   if (order) k_query_scatter<<<blocks, 256, 0, s>>>(accSorted, vals, nq, acc);
 }
 
+// chained: the launch follows a kernel of the step's chain on s (chain_begin).
 void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
                    const MlpDev *mlp, float band, int corr, bool noClamp, int threads,
-                   bool pairs) {
+                   bool pairs, bool chained) {
   if (corr == 0 && !exact && noClamp) {
     // the group walk where its records nearly always fit, with 128 threads a
     // block by default (see group_walk_fits), else a cursor per lane
     const bool groups = pairs && group_walk_fits(S);
     if (threads == 0) threads = groups ? 128 : 256;
-    if (threads == 128) launch_plain<128>(s, S, blocks, pairs, groups);
-    else if (threads == 512) launch_plain<512>(s, S, blocks, pairs, groups);
-    else launch_plain<256>(s, S, blocks, pairs, groups);
+    if (threads == 128) launch_plain<128>(s, S, blocks, pairs, groups, chained);
+    else if (threads == 512) launch_plain<512>(s, S, blocks, pairs, groups, chained);
+    else launch_plain<256>(s, S, blocks, pairs, groups, chained);
     return;
   }
   if (blocks <= 0) {

@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(kScanThreads)
                    uint32_t n_max, const uint32_t *d_n, uint32_t *total, uint64_t *status,
                    uint32_t *tileCounter, uint32_t *__restrict__ owner, uint32_t ownerCap,
                    uint32_t *err) {
+  chain_begin();
   __shared__ uint32_t s_items[kScanPadded];
   __shared__ uint32_t s_warp[kScanThreads / 32];
   __shared__ uint32_t s_tile, s_excl;
@@ -256,9 +257,9 @@ void exclusive_scan_u32(cudaStream_t s, const uint32_t *in, uint32_t *out,
                         uint32_t owner_cap, int slot) {
   const uint32_t tiles = (n_max + kScanTile - 1) / kScanTile;
   if (slot >= 0) {
-    k_scan_onepass<<<tiles > 0 ? tiles : 1, kScanThreads, 0, s>>>(
-        in, out, n_max, d_n, total, sc.slotStatus + (size_t)slot * sc.maxTiles,
-        sc.tileCounter + slot, owner, owner_cap, err);
+    launch_after(s, k_scan_onepass, tiles > 0 ? tiles : 1, kScanThreads, 0, in, out, n_max, d_n,
+                 total, sc.slotStatus + (size_t)slot * sc.maxTiles, sc.tileCounter + slot, owner,
+                 owner_cap, err);
     return;
   }
   uint32_t *tileSum = reinterpret_cast<uint32_t *>(sc.status);
@@ -307,6 +308,7 @@ __global__ void __launch_bounds__(kSortThreads, 3)
                const uint32_t *__restrict__ digitCount, uint32_t *status,
                uint32_t *tileCounter, uint32_t n_max, const uint32_t *d_n,
                int shift, uint32_t *err) {
+  chain_begin();
   __shared__ K s_keys[kSortTile];
   __shared__ uint32_t s_vals[kSortTile];
   __shared__ uint32_t s_whist[kSortWarps][256];
@@ -535,6 +537,7 @@ __global__ void __launch_bounds__(256)
                  uint32_t n, LowKey lowKey, bool hasSkip, uint32_t skip,
                  uint32_t *__restrict__ longRuns, uint32_t *longCount, uint32_t cap,
                  uint32_t *err) {
+  chain_begin();
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += gridDim.x * blockDim.x)
     fix_run(keys, vals, n, i, lowKey, hasSkip, skip, longRuns, longCount, cap, err);
@@ -640,6 +643,7 @@ __global__ void __launch_bounds__(256)
     k_long_runs32(uint32_t *keys, uint32_t *vals, uint32_t *tmpK, uint32_t *tmpV, uint32_t n,
                   LowKey lowKey, const uint32_t *longRuns, const uint32_t *longCount,
                   uint32_t cap) {
+  chain_begin();
   __shared__ LongRunShared sh;
   order_long_runs(keys, vals, tmpK, tmpV, n, lowKey, longRuns, min(*longCount, cap), blockIdx.x,
                   gridDim.x, sh, [] { __syncthreads(); });
@@ -654,10 +658,10 @@ void sort_fix_low_bits32(cudaStream_t s, SortScratch &sc, int buf, uint32_t n,
   if (!zeroed) cudaMemsetAsync(runCount, 0, sizeof(uint32_t), s);
   uint32_t b = (n + 255) / 256;
   if (b > 148u * 16u) b = 148u * 16u;
-  const CodeLow lk{codes};
-  k_fix_runs32<<<b, 256, 0, s>>>(keys32(sc, buf), sc.vals[buf], n, lk, false, 0u, longRuns,
+  CodeLow lk{codes};
+  launch_after(s, k_fix_runs32<decltype(lk)>, b, 256, 0, keys32(sc, buf), sc.vals[buf], n, lk, false, 0u, longRuns,
                                  runCount, cap, err);
-  k_long_runs32<<<148, 256, 0, s>>>(keys32(sc, buf), sc.vals[buf], keys32(sc, buf ^ 1),
+  launch_after(s, k_long_runs32<decltype(lk)>, 148, 256, 0, keys32(sc, buf), sc.vals[buf], keys32(sc, buf ^ 1),
                                      sc.vals[buf ^ 1], n, lk, longRuns, runCount, cap);
 }
 
@@ -668,10 +672,10 @@ void sort_fix_units(cudaStream_t s, SortScratch &sc, int buf, uint32_t n, const 
   if (!zeroed) cudaMemsetAsync(runCount, 0, sizeof(uint32_t), s);
   uint32_t b = (n + 255) / 256;
   if (b > 148u * 16u) b = 148u * 16u;
-  const BoxMinX lk{box};
-  k_fix_runs32<<<b, 256, 0, s>>>(keys32(sc, buf), sc.vals[buf], n, lk, true, skip, longRuns,
+  BoxMinX lk{box};
+  launch_after(s, k_fix_runs32<decltype(lk)>, b, 256, 0, keys32(sc, buf), sc.vals[buf], n, lk, true, skip, longRuns,
                                  runCount, cap, err);
-  k_long_runs32<<<148, 256, 0, s>>>(keys32(sc, buf), sc.vals[buf], keys32(sc, buf ^ 1),
+  launch_after(s, k_long_runs32<decltype(lk)>, 148, 256, 0, keys32(sc, buf), sc.vals[buf], keys32(sc, buf ^ 1),
                                      sc.vals[buf ^ 1], n, lk, longRuns, runCount, cap);
 }
 
@@ -708,15 +712,17 @@ int radix_sort(cudaStream_t s, SortScratch &sc, K *const keys[2], uint32_t n_max
   for (int p = 0; p < np; ++p) {
     uint32_t *status = sc.status + passWords * (slot + p);
     const int shift = 8 * (p0 + p);
-    if (p == 0 && vals_identity) {
-      k_onesweep<K, true><<<tiles > 0 ? tiles : 1, kSortThreads, 0, s>>>(
+    void (*kernel)(const K *, const uint32_t *, K *, uint32_t *, const uint32_t *, uint32_t *,
+                   uint32_t *, uint32_t, const uint32_t *, int, uint32_t *) =
+        p == 0 && vals_identity ? k_onesweep<K, true> : k_onesweep<K, false>;
+    if (zeroed || p > 0)
+      launch_after(s, kernel, tiles > 0 ? tiles : 1, kSortThreads, 0, keys[cur], sc.vals[cur],
+                   keys[cur ^ 1], sc.vals[cur ^ 1], hist + p * 256, status,
+                   sc.tileCounter + slot + p, n_max, d_n, shift, err);
+    else // after the clears
+      kernel<<<tiles > 0 ? tiles : 1, kSortThreads, 0, s>>>(
           keys[cur], sc.vals[cur], keys[cur ^ 1], sc.vals[cur ^ 1], hist + p * 256, status,
           sc.tileCounter + slot + p, n_max, d_n, shift, err);
-    } else {
-      k_onesweep<K, false><<<tiles > 0 ? tiles : 1, kSortThreads, 0, s>>>(
-          keys[cur], sc.vals[cur], keys[cur ^ 1], sc.vals[cur ^ 1], hist + p * 256, status,
-          sc.tileCounter + slot + p, n_max, d_n, shift, err);
-    }
     cur ^= 1;
   }
   return cur;
@@ -804,6 +810,7 @@ __global__ void __cluster_dims__(B, 1, 1) __launch_bounds__(T, 1)
     k_cluster_sort(Source src, uint32_t n, uint32_t *keysOut, uint32_t *valsOut, uint32_t *tmpK,
                    uint32_t *tmpV, uint32_t *longRuns, uint32_t *longCount, uint32_t cap,
                    uint32_t *err) {
+  chain_begin();
   extern __shared__ uint4 sDyn[];
   ClusterShared<T, K> &sh = *reinterpret_cast<ClusterShared<T, K> *>(sDyn);
   constexpr uint32_t kWarps = T / 32;
@@ -1002,9 +1009,9 @@ void cluster_sort(cudaStream_t s, const Source &src, uint32_t n, SortScratch &sc
   static_assert(B * T * K <= 65536 && smem <= 227 * 1024, "16-bit places, one block per SM");
   cudaFuncSetAttribute(k_cluster_sort<B, T, K, Source>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  k_cluster_sort<B, T, K, Source><<<B, T, smem, s>>>(src, n, keys32(sc, out), sc.vals[out],
-                                                     keys32(sc, out ^ 1), sc.vals[out ^ 1],
-                                                     longRuns, longCount, cap, err);
+  launch_after(s, k_cluster_sort<B, T, K, Source>, B, T, smem, src, n, keys32(sc, out),
+               sc.vals[out], keys32(sc, out ^ 1), sc.vals[out ^ 1], longRuns, longCount, cap,
+               err);
 }
 
 template <class Source>
