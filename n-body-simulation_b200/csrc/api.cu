@@ -435,6 +435,11 @@ int allocate(nbx_handle *h) {
   A(S.moments, nodes);
   A(S.subtree, nodes);
   A(S.arrive, nodes);
+  const size_t spans = ((size_t)nodes / 256 + 1) * (kMaxDepth + 1);
+  A(S.spanParent, spans);
+  A(S.spanArrive, spans);
+  A(S.spanKids, spans);
+  NBX_CUDA(h, cudaMemset(S.spanKids, 0xff, spans * sizeof(uint4)));
   A(S.tN, nodes); // cudaMalloc: 256-byte aligned, so every record is 32
   A(S.tM, nodes);
   { // written by every build before it is read: not cleared

@@ -502,70 +502,108 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
-// First index in (i, e] whose depth-d prefix differs from code[i]'s (pre),
-// given that the codes from e on all differ (a gallop, then a binary
-// search).  d >= 1.
-__device__ __forceinline__ uint32_t prefix_end(const uint64_t *c, uint32_t i, uint32_t e,
-                                               int d, uint64_t pre) {
-  const int sh = 64 - 2 * d;
-  uint32_t lo = i + 1, hi = e, step = 1;
-  while (lo < hi) {
-    const uint32_t probe = lo + step - 1;
-    if (probe >= hi) break;
-    if ((c[probe] >> sh) != pre) {
-      hi = probe;
-      break;
-    }
-    lo = probe + 1;
-    step <<= 1;
-  }
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if ((c[mid] >> sh) == pre) lo = mid + 1;
-    else hi = mid;
-  }
-  return lo;
-}
-
-// First index in [s0, i] with the depth-d prefix of code[i] (a gallop
-// backwards, then a binary search).  d >= 1.
-__device__ __forceinline__ uint32_t prefix_start(const uint64_t *c, uint32_t s0,
-                                                 uint32_t i, int d) {
-  const int sh = 64 - 2 * d;
-  const uint64_t pre = c[i] >> sh;
-  uint32_t lo = s0, hi = i, step = 1; // answer in [lo, hi]
-  while (hi > lo) {
-    const uint32_t probe = hi - lo >= step ? hi - step : lo;
-    if ((c[probe] >> sh) != pre) {
-      lo = probe + 1;
-      break;
-    }
-    hi = probe;
-    if (probe == lo) break;
-    step <<= 1;
-  }
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if ((c[mid] >> sh) == pre) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
-}
-
 // Record of the node at depth d starting at body b.
 __device__ __forceinline__ uint32_t record_of(const DevState &S, uint32_t b, int d) {
   return S.splitStart[b] + (uint32_t)(d - (int)S.splitLo[b]);
 }
 
-// One thread per record: body range, next and open slots, size and centre
-// (splitNode's arithmetic along the path), parent, the records of the
-// non-empty children in digit order (all ones past the last); arrival
-// counters cleared.  kFull: also the cell centres and sizes of tC/tM (read
-// only by the corrected forms and the network's harvest).
+// Writes record `at` of the default force walk (QuadRec) from the sums, cell
+// and first body of the children in `have` (by digit); returns the link to it.
+// (px, py): a finite place for absent children.
+__device__ __forceinline__ uint32_t quad_record(const DevState &S, uint32_t at, float px,
+                                                float py, uint32_t have, const float4 (&up)[4],
+                                                const float4 (&ca)[4], const uint32_t (&first)[4]) {
+  float x[4], y[4], h[4], w[4];
+  uint2 c[4];
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) {
+    const bool in = (have >> q) & 1u;
+    x[q] = in ? ca[q].x : px;
+    y[q] = in ? ca[q].y : py;
+    h[q] = in ? 0.5f * ca[q].z : 0.0f;
+    w[q] = in ? up[q].z : 0.0f;
+    c[q] = in ? make_uint2(__float_as_uint(up[q].w), first[q]) : make_uint2(kQuadLeaf, 0u);
+  }
+  QuadRec &Q = S.tQ[at];
+  Q.x = make_float4(x[0], x[1], x[2], x[3]);
+  Q.y = make_float4(y[0], y[1], y[2], y[3]);
+  Q.halfM = make_float4(h[0], h[1], h[2], h[3]);
+  Q.w = make_float4(w[0], w[1], w[2], w[3]);
+  *reinterpret_cast<uint4 *>(&Q.child[0]) = make_uint4(c[0].x, c[0].y, c[1].x, c[1].y);
+  *reinterpret_cast<uint4 *>(&Q.child[2]) = make_uint4(c[2].x, c[2].y, c[3].x, c[3].y);
+  return at;
+}
+
+// The record that holds only the root (up, a) of instance sg.
+__device__ __forceinline__ void quad_root(const DevState &S, uint32_t sg, float4 up, float4 a) {
+  const float4 ups[4] = {up}, as[4] = {a};
+  const uint32_t first[4] = {S.seg[sg].start};
+  quad_record(S, S.n + sg, a.x, a.y, 1u, ups, as, first);
+}
+
+// Eight lanes narrow [lo, hi] down to the first index of [lo, hi) where
+// before(index) is false (hi if none), before being true up to it: eight
+// probes a round.  All groups of the warp call it together.
+template <class Before>
+__device__ __forceinline__ uint32_t search8(uint32_t lo, uint32_t hi, Before before) {
+  const uint32_t g = threadIdx.x & 7u, shift = threadIdx.x & 24u;
+  while (__any_sync(0xffffffffu, lo < hi)) {
+    const uint64_t len = hi - lo;
+    auto probe = [&](uint32_t k) { return lo + (uint32_t)(len * (k + 1u) / 9u); };
+    const bool t = lo < hi && before(probe(g));
+    const uint32_t yes = __popc((__ballot_sync(0xffffffffu, t) >> shift) & 255u);
+    if (lo < hi) {
+      const uint32_t l = yes > 0 ? probe(yes - 1u) + 1u : lo;
+      hi = yes < 8 ? probe(yes) : hi;
+      lo = l;
+    }
+  }
+  return lo;
+}
+
+// The traversal records and their sums in one pass, a thread to a record, 256
+// consecutive records (preorder) to a block.
+//
+// A record's parent is the last record before it that is less deep, its
+// subtree ends at the first one after it that is no deeper: both come from the
+// block's depths in shared memory.  Only the ancestors of the block's first
+// record that start before the block (a child's parent) and the ends of the
+// last record's ancestors are searched for in the codes, one per depth, eight
+// probes a round.
+//
+// Then upwards: a leaf sums its bodies (sumNode's order) and climbs, and the
+// last child to arrive at a node sums its children in digit order, then
+// finishNode's divide, and climbs on.  A child leaves its record at its digit
+// of the node and adds its bodies to the node's arrival counter, which is
+// complete at the node's body count.
+//  * A node whose whole subtree lies in the block (most but the top few) has
+//    its counter and its children's sums in shared memory.
+//  * A node that reaches beyond the block has them in global memory, at
+//    (block, depth), which no other such node of the block shares; its own
+//    thread, once it has published the node, subtracts the body count.  Who
+//    brings the counter to 0 is the last and finds everything published; the
+//    counter is 0 and the children's slots are empty again for the next build.
+// kFull: also the cell centres and sizes of tC/tM and the second moments
+// about each centre of mass (read only by the corrected forms and the
+// network's harvest).
+// Bound by the latency of dependent loads.  us between events around the
+// stage, as two kernels with child bounds, parents and ends all searched by
+// bisection and every arrival through global memory -> now: 10,000 bodies
+// 43 -> 29, 99,991 53 -> 34, 2^20 86 -> 71.  At 128 registers (2 blocks per SM)
+// 2 us less below 10^5 bodies and 20 more for 2^22.
 template <bool kFull>
-__global__ void __launch_bounds__(kBlock)
-    k_trav_nodes(DevState S, const uint32_t *__restrict__ owner, uint4 *__restrict__ kids) {
+__global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
+    k_trav_tree(DevState S, const uint32_t *__restrict__ owner) {
   chain_begin();
+  __shared__ float4 sUp[kBlock], sA[kBlock], sM[kFull ? kBlock : 1];
+  __shared__ uint32_t sKids[kBlock]; // bytes: a node's children by digit, how far
+                                     // after it (less one)
+  __shared__ uint32_t sNoDeeper[kMaxDepth + 1][kBlock / 32]; // bit t: depth[t] <= row
+  __shared__ uint8_t sDepthEnds[2]; // of the block's first and last record
+  __shared__ uint32_t sStart[kBlock], sBodies[kBlock], sArrive[kBlock];
+  __shared__ uint32_t sParent[kBlock]; // record
+  __shared__ uint8_t sSpans[kBlock];
+  __shared__ uint32_t sLeft[kMaxDepth + 1], sRight[kMaxDepth + 1];
   const uint64_t *c = S.sortedCodes;
   const uint32_t total = S.counters[6];
   const bool overflow = total > S.nodeCapacity;
@@ -582,211 +620,315 @@ __global__ void __launch_bounds__(kBlock)
     if (overflow && threadIdx.x == 0) atomicOr(S.status, kStatusTreeCapacity);
   }
   if (overflow) return;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total;
-       p += gridDim.x * blockDim.x) {
-    const uint32_t i = owner[p];
-    const SegDev &G = S.seg[S.segOf[i]];
-    const uint32_t s0 = G.start, s1 = G.start + G.count;
-    const uint32_t P = S.splitStart[i];
-    const uint32_t k = p - P;
-    const int lo = S.splitLo[i];
-    const int d = lo + (int)k;
-    const bool leaf = k + 1 == S.splitCount[i];
-    const uint64_t ci = c[i];
-    float cx = G.cx, cy = G.cy, size = G.size;
-    if (kFull || !(fabsf(G.size) >= 0x1p-90f && fabsf(G.size) <= 0x1p+120f)) {
-      for (int t = 0; t < d; ++t) {
-        size = __fmul_rn(size, 0.5f);
-        const int q = digit_at(ci, t);
-        cx = __fadd_rn(cx, __fmul_rn((float)(q & 1) - 0.5f, size));
-        cy = __fadd_rn(cy, __fmul_rn((float)(q >> 1) - 0.5f, size));
-      }
-    } else {
-      // d <= 32 halvings of a normal size stay normal: each is exact, so
-      // the repeated halving is one exponent step
-      size = ldexpf(size, -d);
-    }
-    const uint32_t e = d > 0 ? prefix_end(c, i, s1, d, ci >> (64 - 2 * d)) : s1;
-    // the record after the subtree; all ones past the instance's last
-    const uint32_t next = e < s1 ? S.splitStart[e] : 0xffffffffu;
-    int32_t parent = -1;
-    if (d > 0) {
-      if (k > 0) {
-        parent = (int32_t)(p - 1);
+  const uint32_t t = threadIdx.x;
+  const uint32_t lane = t & 31u, warp = t >> 5;
+  for (uint32_t base = blockIdx.x * kBlock; base < total; base += gridDim.x * kBlock) {
+    const uint32_t p = base + t, held = min((uint32_t)kBlock, total - base);
+    bool leaf = false, spans = false;
+    uint32_t i = 0, sg = 0, s0 = 0, s1 = 0;
+    int d = 0;
+    uint64_t ci = 0;
+    float w = 0.0f, size = 0.0f;
+    if (t < held) {
+      i = owner[p];
+      sg = S.segOf[i];
+      const SegDev &G = S.seg[sg];
+      s0 = G.start;
+      s1 = G.start + G.count;
+      const uint32_t k = p - S.splitStart[i];
+      d = S.splitLo[i] + (int)k;
+      leaf = k + 1 == S.splitCount[i];
+      ci = c[i];
+      float cx = G.cx, cy = G.cy;
+      size = G.size;
+      if (kFull || !(fabsf(G.size) >= 0x1p-90f && fabsf(G.size) <= 0x1p+120f)) {
+        for (int q = 0; q < d; ++q) {
+          size = __fmul_rn(size, 0.5f);
+          const int g = digit_at(ci, q);
+          cx = __fadd_rn(cx, __fmul_rn((float)(g & 1) - 0.5f, size));
+          cy = __fadd_rn(cy, __fmul_rn((float)(g >> 1) - 0.5f, size));
+        }
       } else {
-        // the depth-(d-1) node around i starts before it (the root at s0)
-        const uint32_t j = d == 1 ? s0 : prefix_start(c, s0, i, d - 1);
-        parent = (int32_t)record_of(S, j, d - 1);
+        // d <= 32 halvings of a normal size stay normal: each is exact, so
+        // the repeated halving is one exponent step
+        size = ldexpf(size, -d);
       }
+      w = __fmul_rn(size, size);
+      if (kFull) S.tC[p] = make_float2(cx, cy);
+      sA[t] = make_float4(0.0f, 0.0f, 0.0f, w);
+      if (kFull) sM[t] = make_float4(0.0f, 0.0f, 0.0f, size);
     }
-    uint4 ch = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-    uint32_t children = 0;
-    if (!leaf) {
-      uint32_t bound[5];
-      bound[0] = i;
-      bound[4] = e;
-      for (int q = 1; q < 4; ++q) bound[q] = first_with_digit(c, bound[q - 1], e, d, q);
-      uint32_t r[4];
-      for (int q = 0; q < 4; ++q)
-        if (bound[q + 1] > bound[q]) r[children++] = record_of(S, bound[q], d + 1);
-      for (uint32_t q = children; q < 4; ++q) r[q] = 0xffffffffu;
-      ch = make_uint4(r[0], r[1], r[2], r[3]);
-    }
-    TravNode &T = S.tN[p];
-    T.a = make_float4(0.0f, 0.0f, 0.0f, __fmul_rn(size, size));
-    T.b = make_int4((int)next, (int)(leaf ? next : p + 1), (int)i, (int)e);
-    if (kFull) {
-      S.tM[p] = make_float4(0.0f, 0.0f, 0.0f, size);
-      S.tC[p] = make_float2(cx, cy);
-    }
-    S.parent[p] = parent;
-    S.subtree[p] = children;
-    S.arrive[p] = 0u;
-    kids[p] = ch;
-  }
-}
-
-// Writes record `at` of the default force walk (QuadRec) from the sums, cell
-// and first body of up to four children; returns the link to it.  (px, py):
-// a finite place for absent children.
-__device__ __forceinline__ uint32_t quad_record(const DevState &S, uint32_t at, float px,
-                                                float py, uint32_t children,
-                                                const float4 (&up)[4], const float4 (&ca)[4],
-                                                const int (&first)[4]) {
-  float x[4], y[4], h[4], w[4];
-  uint2 c[4];
+    if (t == 0) sDepthEnds[0] = (uint8_t)d;
+    if (t == held - 1u) sDepthEnds[1] = (uint8_t)d;
+    {
+      uint32_t row = 0, last = 0; // lane's row, and row 32 for lane 0
 #pragma unroll
-  for (uint32_t q = 0; q < 4; ++q) {
-    const bool have = q < children;
-    x[q] = have ? ca[q].x : px;
-    y[q] = have ? ca[q].y : py;
-    h[q] = have ? 0.5f * ca[q].z : 0.0f;
-    w[q] = have ? up[q].z : 0.0f;
-    c[q] = have ? make_uint2(__float_as_uint(up[q].w), (uint32_t)first[q])
-                : make_uint2(kQuadLeaf, 0u);
-  }
-  QuadRec &Q = S.tQ[at];
-  Q.x = make_float4(x[0], x[1], x[2], x[3]);
-  Q.y = make_float4(y[0], y[1], y[2], y[3]);
-  Q.halfM = make_float4(h[0], h[1], h[2], h[3]);
-  Q.w = make_float4(w[0], w[1], w[2], w[3]);
-  *reinterpret_cast<uint4 *>(&Q.child[0]) = make_uint4(c[0].x, c[0].y, c[1].x, c[1].y);
-  *reinterpret_cast<uint4 *>(&Q.child[2]) = make_uint4(c[2].x, c[2].y, c[3].x, c[3].y);
-  return at;
-}
-
-// The record that holds only the root (up, a) of the instance with body b.
-__device__ __forceinline__ void quad_root(const DevState &S, uint32_t b, float4 up, float4 a) {
-  const uint32_t sg = S.segOf[b];
-  const float4 ups[4] = {up}, as[4] = {a};
-  const int first[4] = {(int)S.seg[sg].start};
-  quad_record(S, S.n + sg, a.x, a.y, 1, ups, as, first);
-}
-
-// Bottom-up sums over the traversal records: each leaf sums its bodies
-// (sumNode's order) and climbs; the last non-empty child to arrive sums its
-// parent's children in digit order, then finishNode's divide; second
-// moments about each centre of mass for the corrected forms.
-template <bool kMoments>
-__global__ void __launch_bounds__(kBlock)
-    k_trav_upward(DevState S, const uint4 *__restrict__ kids) {
-  chain_begin();
-  const uint32_t total = S.counters[6];
-  if (total > S.nodeCapacity) return;
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < total;
-       p += gridDim.x * blockDim.x) {
-    if (S.subtree[p] != 0) continue; // interior: summed by its last child
-    const int4 B = S.tN[p].b;
-    const uint32_t b0 = (uint32_t)B.z, b1 = min((uint32_t)B.w, S.n);
-    float px = 0.0f, py = 0.0f, mm = 0.0f;
-    for (uint32_t b = b0; b < b1; ++b) {
-      const float4 q = S.xym[b];
-      px = __fadd_rn(px, __fmul_rn(q.x, q.z));
-      py = __fadd_rn(py, __fmul_rn(q.y, q.z));
-      mm = __fadd_rn(mm, q.z);
-    }
-    const float div = fmaxf(mm, FLT_MIN);
-    const float X = __fdiv_rn(px, div), Y = __fdiv_rn(py, div);
-    if (kMoments) {
-      float ixx = 0.0f, iyy = 0.0f, ixy = 0.0f;
-      for (uint32_t b = b0; b < b1; ++b) {
-        const float4 q = S.xym[b];
-        const float dx = q.x - X, dy = q.y - Y;
-        ixx += q.z * dx * dx;
-        iyy += q.z * dy * dy;
-        ixy += q.z * dx * dy;
+      for (int depth = 0; depth <= kMaxDepth; ++depth) {
+        const uint32_t m = __ballot_sync(0xffffffffu, t < held && d <= depth);
+        if (depth == kMaxDepth) last = m;
+        else if (lane == (uint32_t)depth) row = m;
       }
-      __stcg(&S.tM[p], make_float4(ixx, iyy, ixy, S.tM[p].w));
+      sNoDeeper[lane][warp] = row;
+      if (lane == 0) sNoDeeper[kMaxDepth][warp] = last;
     }
-    const float4 own = S.tN[p].a;
-    const uint32_t leafLink = kQuadLeaf | (uint32_t)(B.w - B.z);
-    __stcg(&S.tUp[p], make_float4(px, py, own.w, __uint_as_float(leafLink)));
-    __stcg(&S.tN[p].a, make_float4(X, Y, mm, own.w));
-    int32_t node = S.parent[p];
-    if (node < 0)
-      quad_root(S, b0, make_float4(px, py, own.w, __uint_as_float(leafLink)),
-                make_float4(X, Y, mm, own.w));
-    for (int guard = 0; node >= 0 && guard <= kMaxDepth; ++guard) {
-      const uint32_t g = (uint32_t)node;
-      if (g >= total) {
-        atomicOr(S.status, kStatusTreeCapacity);
-        break;
+    sStart[t] = i;
+    sKids[t] = 0xffffffffu;
+    sArrive[t] = 0u;
+    __syncthreads();
+    {
+      // by eight lanes a depth: four warps the record at it that holds the
+      // block's first record, four the end of the one that holds the last
+      const bool leftHalf = t < kBlock / 2;
+      const uint32_t b = sStart[leftHalf ? 0 : held - 1];
+      const int dEnd = leftHalf ? (int)sDepthEnds[0] : (int)sDepthEnds[1] + 1;
+      const SegDev &G = S.seg[S.segOf[b]];
+      const uint32_t g0 = G.start, g1 = G.start + G.count;
+      const uint64_t code = c[b];
+      for (int depth = (int)((t & (kBlock / 2 - 1)) >> 3); __any_sync(0xffffffffu, depth < dEnd);
+           depth += kBlock / 16) {
+        // depth 0 is the whole instance
+        const bool search = depth > 0 && depth < dEnd;
+        const int sh = search ? 64 - 2 * depth : 0;
+        uint32_t lo = leftHalf ? g0 : g1, hi = lo;
+        if (search && leftHalf) hi = b;
+        if (search && !leftHalf) lo = b + 1u;
+        const uint32_t j = search8(lo, hi, [&](uint32_t m) {
+          return ((c[m] >> sh) != (code >> sh)) == leftHalf;
+        });
+        if ((t & 7u) == 0 && depth < dEnd) {
+          if (leftHalf) sLeft[depth] = record_of(S, j, depth);
+          else sRight[depth] = j;
+        }
       }
-      const uint32_t children = S.subtree[g];
-      // release: this child's sums are visible to the last arriver;
-      // acquire: the last arriver sees every child's sums
-      uint32_t old;
-      asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
-                   : "=r"(old)
-                   : "l"(&S.arrive[g])
-                   : "memory");
-      if (old + 1 != children) break;
-      const uint4 kv = kids[g];
-      const uint32_t r[4] = {kv.x, kv.y, kv.z, kv.w};
-      float4 up[4], ca[4], mo[4];
-      int first[4]; // the children's first bodies
+    }
+    __syncthreads();
+    uint32_t e = 0, after = 0;
+    if (t < held) {
+      // the first record after this one that is no deeper ends its subtree
+      uint32_t q = kBlock;
+      {
+        uint32_t m = lane < 31 ? sNoDeeper[d][warp] & (0xfffffffeu << lane) : 0u;
+        uint32_t word = warp;
+        while (m == 0 && ++word < kBlock / 32) m = sNoDeeper[d][word];
+        if (m != 0) q = 32u * word + __ffs(m) - 1u;
+      }
+      if (q < held) {
+        after = base + q;
+        e = sStart[q];
+      } else {
+        e = sRight[d];
+        after = e < S.n ? S.splitStart[e] : total;
+        spans = !leaf && after > base + kBlock;
+      }
+      // the last record before this one that is less deep is its parent
+      uint32_t parent = 0xffffffffu;
+      if (d > 0) {
+        uint32_t m = sNoDeeper[d - 1][warp] & ((1u << lane) - 1u);
+        int word = (int)warp;
+        while (m == 0 && --word >= 0) m = sNoDeeper[d - 1][word];
+        parent = m != 0 ? base + 32u * word + 31u - __clz(m) : sLeft[d - 1];
+      }
+      const uint32_t next = e < s1 ? after : 0xffffffffu;
+      S.tN[p].b = make_int4((int)next, (int)(leaf ? next : p + 1), (int)i, (int)e);
+      sParent[t] = parent;
+      sBodies[t] = e - i;
+      sSpans[t] = spans ? 1u : 0u;
+      if (spans) { // published by its arrival below
+        __stcg(&S.tN[p].a, make_float4(0.0f, 0.0f, 0.0f, w));
+        if (kFull) __stcg(&S.tM[p], make_float4(0.0f, 0.0f, 0.0f, size));
+        __stcg(&S.spanParent[p / kBlock * (kMaxDepth + 1) + d], parent);
+      }
+    }
+    __syncthreads();
+    // the node this thread holds the sums of: its record, depth and bodies
+    uint32_t node = p, bodies = e - i;
+    float4 up = make_float4(0.0f, 0.0f, 0.0f, 0.0f), own = up, mom = up;
+    if (leaf) {
+      const uint32_t b1 = min(e, S.n);
+      float px = 0.0f, py = 0.0f, mm = 0.0f;
+      for (uint32_t b = i; b < b1; b += 4) { // four loads in flight
+        float4 q[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) q[k] = S.xym[min(b + k, b1 - 1u)];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+          if (b + k >= b1) continue;
+          px = __fadd_rn(px, __fmul_rn(q[k].x, q[k].z));
+          py = __fadd_rn(py, __fmul_rn(q[k].y, q[k].z));
+          mm = __fadd_rn(mm, q[k].z);
+        }
+      }
+      const float div = fmaxf(mm, FLT_MIN);
+      const float X = __fdiv_rn(px, div), Y = __fdiv_rn(py, div);
+      if (kFull) {
+        float ixx = 0.0f, iyy = 0.0f, ixy = 0.0f;
+        for (uint32_t b = i; b < b1; ++b) {
+          const float4 q = S.xym[b];
+          const float dx = q.x - X, dy = q.y - Y;
+          ixx += q.z * dx * dx;
+          iyy += q.z * dy * dy;
+          ixy += q.z * dx * dy;
+        }
+        mom = make_float4(ixx, iyy, ixy, size);
+      }
+      up = make_float4(px, py, w, __uint_as_float(kQuadLeaf | (e - i)));
+      own = make_float4(X, Y, mm, w);
+    }
+    // at most kMaxDepth + 1 nodes; record indices are range-checked
+    bool publish = spans; // first the arrival of the node's own thread
+    for (int guard = 0; (leaf || spans) && guard <= kMaxDepth + 1; ++guard) {
+      uint32_t l = kBlock; // the next node's place in the block, if summed there
+      uint32_t slot = 0;   // else its place among the nodes beyond a block
+      if (publish) {
+        slot = p / kBlock * (kMaxDepth + 1) + d;
+      } else { // `node` is summed: keep it and arrive at its parent
+        const uint32_t in = node - base;
+        if (in < kBlock) { // its thread stores it at the end, unless it spans
+          sUp[in] = up;
+          sA[in] = own;
+          if (kFull) sM[in] = mom;
+        }
+        if (in >= kBlock || sSpans[in] != 0) {
+          __stcg(&S.tN[node].a, own);
+          if (kFull) __stcg(&S.tM[node], mom);
+        }
+        if (d == 0) {
+          quad_root(S, sg, up, own);
+          break;
+        }
+        const uint32_t parent = in < kBlock ? sParent[in]
+                                            : __ldcg(&S.spanParent[node / kBlock * (kMaxDepth + 1) + d]);
+        if (parent >= total) {
+          atomicOr(S.status, kStatusTreeCapacity);
+          break;
+        }
+        --d;
+        const uint32_t digit = (uint32_t)digit_at(ci, d); // ci lies in the node
+        l = parent - base;
+        if (l < kBlock && sSpans[l] == 0) {
+          reinterpret_cast<uint8_t *>(&sKids[l])[digit] = (uint8_t)(in - l - 1u);
+          __threadfence_block();
+          if (atomicAdd(&sArrive[l], bodies) + bodies != sBodies[l]) break;
+          __threadfence_block();
+        } else {
+          l = kBlock;
+          slot = parent / kBlock * (kMaxDepth + 1) + d;
+          __stcg(&S.tN[node].a, own);
+          if (kFull) __stcg(&S.tM[node], mom);
+          __stcg(&S.tUp[node], up);
+          __stcg(reinterpret_cast<uint32_t *>(&S.spanKids[slot]) + digit, node);
+        }
+        node = parent;
+      }
+      const bool local = l < kBlock;
+      if (!local) {
+        // release: what this thread published is visible to the last arriver;
+        // acquire: the last arriver sees all
+        const uint32_t add = publish ? 0u - bodies : bodies;
+        uint32_t old;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
+                     : "=r"(old)
+                     : "l"(&S.spanArrive[slot]), "r"(add)
+                     : "memory");
+        if (old + add != 0u) break;
+        publish = false;
+      }
+      uint32_t have = 0, first[4];
+      float4 cu[4], ca[4], cm[4];
+      float nw, nsize = 0.0f;
+      if (local) {
+        const uint32_t kv = sKids[l];
+        nw = sA[l].w;
+        if (kFull) nsize = sM[l].w;
+        bodies = sBodies[l];
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          const uint32_t k = l + 1u + ((kv >> (8 * q)) & 255u);
+          if (k >= l + 256u) continue; // 255: empty (a child is at most 255 on)
+          have |= 1u << q;
+          cu[q] = sUp[k];
+          ca[q] = sA[k];
+          if (kFull) cm[q] = sM[k];
+          first[q] = sStart[k];
+        }
+      } else {
+        const uint4 kv = __ldcg(&S.spanKids[slot]);
+        __stcg(&S.spanKids[slot], make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu));
+        nw = __ldcg(&S.tN[node].a).w;
+        if (kFull) nsize = __ldcg(&S.tM[node]).w;
+        const int4 B = __ldcg(&S.tN[node].b);
+        bodies = (uint32_t)(B.w - B.z);
+        const uint32_t r[4] = {kv.x, kv.y, kv.z, kv.w};
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          if (r[q] >= total) continue; // all ones: no such child
+          have |= 1u << q;
+          cu[q] = __ldcg(&S.tUp[r[q]]);
+          ca[q] = __ldcg(&S.tN[r[q]].a);
+          if (kFull) cm[q] = __ldcg(&S.tM[r[q]]);
+          first[q] = (uint32_t)__ldcg(&S.tN[r[q]].b).z;
+        }
+      }
+      // sums in digit order (sumNode), then finishNode's divide
+      float sx = 0.0f, sy = 0.0f, sm = 0.0f, wBot = 0.0f;
+      uint32_t count = 0, link = 0, second = 0;
+#pragma unroll
       for (uint32_t q = 0; q < 4; ++q) {
-        if (q >= children || r[q] >= total) continue;
-        up[q] = __ldcg(&S.tUp[r[q]]);
-        ca[q] = __ldcg(&S.tN[r[q]].a);
-        first[q] = S.tN[r[q]].b.z;
-        if (kMoments) mo[q] = __ldcg(&S.tM[r[q]]);
-      }
-      float sx = 0.0f, sy = 0.0f, sm = 0.0f;
-      for (uint32_t q = 0; q < children && q < 4; ++q) {
-        if (r[q] >= total) break;
-        sx = q == 0 ? up[q].x : __fadd_rn(sx, up[q].x);
-        sy = q == 0 ? up[q].y : __fadd_rn(sy, up[q].y);
-        sm = q == 0 ? ca[q].z : __fadd_rn(sm, ca[q].z);
+        if (!((have >> q) & 1u)) continue;
+        sx = count == 0 ? cu[q].x : __fadd_rn(sx, cu[q].x);
+        sy = count == 0 ? cu[q].y : __fadd_rn(sy, cu[q].y);
+        sm = count == 0 ? ca[q].z : __fadd_rn(sm, ca[q].z);
+        // one child: the same bodies under a smaller square, its record goes up
+        if (count == 0) {
+          wBot = cu[q].z;
+          link = __float_as_uint(cu[q].w);
+        }
+        if (count == 1) second = first[q];
+        ++count;
       }
       const float dv = fmaxf(sm, FLT_MIN);
-      const float PX = __fdiv_rn(sx, dv), PY = __fdiv_rn(sy, dv);
-      if (kMoments) {
+      const float X = __fdiv_rn(sx, dv), Y = __fdiv_rn(sy, dv);
+      if (kFull) {
         float jxx = 0.0f, jyy = 0.0f, jxy = 0.0f;
-        for (uint32_t q = 0; q < children && q < 4; ++q) {
-          if (r[q] >= total) break;
-          const float dx = ca[q].x - PX, dy = ca[q].y - PY;
-          jxx += mo[q].x + ca[q].z * dx * dx;
-          jyy += mo[q].y + ca[q].z * dy * dy;
-          jxy += mo[q].z + ca[q].z * dx * dy;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+          if (!((have >> q) & 1u)) continue;
+          const float dx = ca[q].x - X, dy = ca[q].y - Y;
+          jxx += cm[q].x + ca[q].z * dx * dx;
+          jyy += cm[q].y + ca[q].z * dy * dy;
+          jxy += cm[q].z + ca[q].z * dx * dy;
         }
-        __stcg(&S.tM[g], make_float4(jxx, jyy, jxy, S.tM[g].w));
+        mom = make_float4(jxx, jyy, jxy, nsize);
       }
-      const float ownW = S.tN[g].a.w;
-      // one child: the same bodies under a smaller square, its record goes up
-      float wBot = up[0].z;
-      uint32_t link = __float_as_uint(up[0].w);
-      if (children > 1) {
-        wBot = ownW;
-        link = quad_record(S, (uint32_t)first[1], PX, PY, children, up, ca, first);
+      if (count > 1) { // a node summed in the block: its thread writes the record
+        wBot = nw;
+        link = local ? second : quad_record(S, second, X, Y, have, cu, ca, first);
       }
-      const float4 ownUp = make_float4(sx, sy, wBot, __uint_as_float(link));
-      const float4 ownA = make_float4(PX, PY, sm, ownW);
-      __stcg(&S.tUp[g], ownUp);
-      __stcg(&S.tN[g].a, ownA);
-      node = S.parent[g];
-      if (node < 0) quad_root(S, b0, ownUp, ownA);
+      up = make_float4(sx, sy, wBot, __uint_as_float(link));
+      own = make_float4(X, Y, sm, nw);
     }
+    __syncthreads();
+    if (t < held && !spans) { // the nodes summed in the block, a thread to each
+      const float4 a = sA[t];
+      S.tN[p].a = a;
+      if (kFull) S.tM[p] = sM[t];
+      const uint32_t kv = sKids[t];
+      float4 cu[4], ca[4];
+      uint32_t have = 0, count = 0, second = 0, first[4];
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        const uint32_t k = t + 1u + ((kv >> (8 * q)) & 255u);
+        if (k >= t + 256u) continue;
+        have |= 1u << q;
+        cu[q] = sUp[k];
+        ca[q] = sA[k];
+        first[q] = sStart[k];
+        if (count == 1) second = first[q];
+        ++count;
+      }
+      if (count > 1) quad_record(S, second, a.x, a.y, have, cu, ca, first);
+    }
+    __syncthreads();
   }
 }
 
@@ -850,22 +992,16 @@ void launch_trav_tree(cudaStream_t s, const DevState &S, ScanScratch &scan, bool
   const uint32_t n = S.n;
   // per-record scratch in arrays only the breadth-first build uses
   uint32_t *owner = reinterpret_cast<uint32_t *>(S.start);
-  uint4 *kids = reinterpret_cast<uint4 *>(S.moments);
   // the records per body (splitCount, splitLo) came with the gather
   // the scan also writes each record's first body (owner)
   exclusive_scan_u32(s, S.splitCount, S.splitStart, n, nullptr, &S.counters[6],
                      scan, S.status, owner, S.nodeCapacity, 3);
   mark(s, "tree.counts");
   if (moments)
-    launch_after(s, k_trav_nodes<true>, grid_for(n / 2 + 64), kBlock, 0, S, owner, kids);
+    launch_after(s, k_trav_tree<true>, grid_for(n / 4 + 64), kBlock, 0, S, owner);
   else
-    launch_after(s, k_trav_nodes<false>, grid_for(n / 2 + 64), kBlock, 0, S, owner, kids);
-  mark(s, "tree.nodes");
-  if (moments)
-    launch_after(s, k_trav_upward<true>, grid_for(n / 4 + 64), kBlock, 0, S, kids);
-  else
-    launch_after(s, k_trav_upward<false>, grid_for(n / 4 + 64), kBlock, 0, S, kids);
-  mark(s, "tree.upward");
+    launch_after(s, k_trav_tree<false>, grid_for(n / 4 + 64), kBlock, 0, S, owner);
+  mark(s, "tree.records");
 }
 
 // The reference's breadth-first node arrays (TreeKernels.cuh:88-95) of the

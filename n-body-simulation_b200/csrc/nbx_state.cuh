@@ -158,6 +158,11 @@ struct DevState {
   float4 *moments;      // {Ixx, Iyy, Ixy, spare}
   uint32_t *subtree;    // nodes in subtree
   uint32_t *arrive;     // bottom-up arrival counters
+  // nodes of the traversal layout that reach beyond their block of the build
+  // (k_trav_tree), by (block, depth): parent record, and between builds
+  // empty: the children's records by digit, the arrival counter
+  uint32_t *spanParent, *spanArrive;
+  uint4 *spanKids;
   // traversal layout (preorder)
   TravNode *tN; // preorder traversal records (32 bytes, one load each)
   QuadRec *tQ; // records of the default force walk (n + nseg)

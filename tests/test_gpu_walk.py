@@ -142,3 +142,24 @@ def test_points_beyond_the_clamp_limit(nbx):
     assert np.isnan(ax[3]) and np.isnan(ex[3])
     k = [0, 1, 2, 4]
     assert np.allclose(ax[k], ex[k], rtol=1e-4, atol=0) and np.allclose(ay[k], ey[k], rtol=1e-4, atol=0)
+
+
+@pytest.mark.parametrize("sizes", [[1], [16], [17], [300], [4000, 1, 70, 3, 2600], [9000] * 3])
+@pytest.mark.parametrize("leaf", [1, 16])
+def test_tree_sums(nbx, oracle, sizes, leaf):
+    """The tree's sums where nodes stay in a block of 256 records, reach beyond
+    it, and share blocks with other instances' (also after an earlier build, whose
+    counters must have been left empty): the exact traversal's bits."""
+    parts = [nbx.cold_square(s, 2 + k) for k, s in enumerate(sizes)]
+    h = nbx.Handle(sizes, theta=0.5, exact_math=1, leaf_capacity=leaf)
+    h.upload(np.concatenate(parts))
+    for _ in range(2):
+        h.phase("attract")
+    g = h.download()
+    h.close()
+    at = 0
+    for p in parts:
+        _, _, _, sb, tree = oracle.morton_build(p, leaf)
+        ox, oy = oracle.tree_forces(sb["px"], sb["py"], sb["mass"], tree, 0.5, 1.0)
+        assert same_bits(g["ax"][at:at + len(p)], ox) and same_bits(g["ay"][at:at + len(p)], oy)
+        at += len(p)
