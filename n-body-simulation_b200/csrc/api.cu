@@ -448,6 +448,10 @@ int allocate(nbx_handle *h) {
       return cuda_fail(h, e, "cudaMalloc S.tQ");
     h->allocs.push_back(v);
     S.tQ = static_cast<QuadRec *>(v);
+    if (cudaError_t e = cudaMalloc(&v, ((size_t)n + ns) * sizeof(QuadMom)))
+      return cuda_fail(h, e, "cudaMalloc S.tQM");
+    h->allocs.push_back(v);
+    S.tQM = static_cast<QuadMom *>(v);
   }
   h->groupFirst.clear();
   S.nGroups = (n + 31) / 32; // one instance: group g starts at 32 g

@@ -509,36 +509,45 @@ __device__ __forceinline__ uint32_t record_of(const DevState &S, uint32_t b, int
 
 // Writes record `at` of the default force walk (QuadRec) from the sums, cell
 // and first body of the children in `have` (by digit); returns the link to it.
-// (px, py): a finite place for absent children.
+// (px, py): a finite place for absent children.  kFull: their moments too.
+template <bool kFull>
 __device__ __forceinline__ uint32_t quad_record(const DevState &S, uint32_t at, float px,
                                                 float py, uint32_t have, const float4 (&up)[4],
-                                                const float4 (&ca)[4], const uint32_t (&first)[4]) {
-  float x[4], y[4], h[4], w[4];
+                                                const float4 (&ca)[4], const float4 (&cm)[4],
+                                                const uint32_t (&first)[4]) {
+  float x[4], y[4], m[4], w[4];
   uint2 c[4];
 #pragma unroll
   for (uint32_t q = 0; q < 4; ++q) {
     const bool in = (have >> q) & 1u;
     x[q] = in ? ca[q].x : px;
     y[q] = in ? ca[q].y : py;
-    h[q] = in ? 0.5f * ca[q].z : 0.0f;
+    m[q] = in ? ca[q].z : 0.0f;
     w[q] = in ? up[q].z : 0.0f;
     c[q] = in ? make_uint2(__float_as_uint(up[q].w), first[q]) : make_uint2(kQuadLeaf, 0u);
   }
   QuadRec &Q = S.tQ[at];
   Q.x = make_float4(x[0], x[1], x[2], x[3]);
   Q.y = make_float4(y[0], y[1], y[2], y[3]);
-  Q.halfM = make_float4(h[0], h[1], h[2], h[3]);
+  Q.m = make_float4(m[0], m[1], m[2], m[3]);
   Q.w = make_float4(w[0], w[1], w[2], w[3]);
   *reinterpret_cast<uint4 *>(&Q.child[0]) = make_uint4(c[0].x, c[0].y, c[1].x, c[1].y);
   *reinterpret_cast<uint4 *>(&Q.child[2]) = make_uint4(c[2].x, c[2].y, c[3].x, c[3].y);
+  if (kFull) {
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q)
+      if ((have >> q) & 1u) S.tQM[at].m[q] = make_float4(cm[q].x, cm[q].y, cm[q].z, ca[q].w);
+  }
   return at;
 }
 
-// The record that holds only the root (up, a) of instance sg.
-__device__ __forceinline__ void quad_root(const DevState &S, uint32_t sg, float4 up, float4 a) {
-  const float4 ups[4] = {up}, as[4] = {a};
+// The record that holds only the root (up, a, moments) of instance sg.
+template <bool kFull>
+__device__ __forceinline__ void quad_root(const DevState &S, uint32_t sg, float4 up, float4 a,
+                                          float4 mom) {
+  const float4 ups[4] = {up}, as[4] = {a}, ms[4] = {mom};
   const uint32_t first[4] = {S.seg[sg].start};
-  quad_record(S, S.n + sg, a.x, a.y, 1u, ups, as, first);
+  quad_record<kFull>(S, S.n + sg, a.x, a.y, 1u, ups, as, ms, first);
 }
 
 // Eight lanes narrow [lo, hi] down to the first index of [lo, hi) where
@@ -793,7 +802,7 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
           if (kFull) __stcg(&S.tM[node], mom);
         }
         if (d == 0) {
-          quad_root(S, sg, up, own);
+          quad_root<kFull>(S, sg, up, own, mom);
           break;
         }
         const uint32_t parent = in < kBlock ? sParent[in]
@@ -902,7 +911,7 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
       }
       if (count > 1) { // a node summed in the block: its thread writes the record
         wBot = nw;
-        link = local ? second : quad_record(S, second, X, Y, have, cu, ca, first);
+        link = local ? second : quad_record<kFull>(S, second, X, Y, have, cu, ca, cm, first);
       }
       up = make_float4(sx, sy, wBot, __uint_as_float(link));
       own = make_float4(X, Y, sm, nw);
@@ -913,7 +922,7 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
       S.tN[p].a = a;
       if (kFull) S.tM[p] = sM[t];
       const uint32_t kv = sKids[t];
-      float4 cu[4], ca[4];
+      float4 cu[4], ca[4], cm[4];
       uint32_t have = 0, count = 0, second = 0, first[4];
 #pragma unroll
       for (uint32_t q = 0; q < 4; ++q) {
@@ -922,11 +931,12 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
         have |= 1u << q;
         cu[q] = sUp[k];
         ca[q] = sA[k];
+        if (kFull) cm[q] = sM[k];
         first[q] = sStart[k];
         if (count == 1) second = first[q];
         ++count;
       }
-      if (count > 1) quad_record(S, second, a.x, a.y, have, cu, ca, first);
+      if (count > 1) quad_record<kFull>(S, second, a.x, a.y, have, cu, ca, cm, first);
     }
     __syncthreads();
   }

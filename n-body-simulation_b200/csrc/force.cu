@@ -26,6 +26,7 @@
 #include "mlp.cuh"
 #include "nbx_state.cuh"
 
+#include <algorithm>
 #include <float.h>
 
 namespace nbx {
@@ -370,7 +371,9 @@ constexpr int kSlots = 192;   // opened records (slots are bytes)
 constexpr int kParts = 400;   // children that some lanes accept
 constexpr int kCells = 704;   // cell terms
 constexpr int kLeaves = 128;  // opened leaves
-constexpr int kPairs = 448;   // pairs of their bodies
+constexpr int kPairs = 448;   // pairs of their bodies (the plain walk)
+constexpr int kTerms = 1408;  // cells and bodies (the walks that keep one order)
+constexpr int kChunk = 32;    // terms summed at a time by those
 struct alignas(16) WalkStage {
   union {
     struct { // children the lanes disagree on, their lanes, those that accept
@@ -378,22 +381,40 @@ struct alignas(16) WalkStage {
       uint32_t cm[64], ca[64];
     };
     uint32_t count[kSlots]; // terms of a record's subtree, later its first
-                            // place: cells | leaves << 10 | leaf pairs << 20
+                            // place: cells | leaves << 10 | leaf pairs << 20,
+                            // or items | terms << 10
     struct { // terms being summed: place, half mass, lanes (of each / a pair)
       float x[64], y[64], h[64];
       uint32_t m[64];
     };
+    struct { // the same of the walks that keep one order: place, mass, lanes,
+             // squared size; moments and the chain's largest squared size
+      float4 q[kChunk], mom[kChunk];
+      uint32_t lanes[kChunk];
+    };
   };
   uint32_t rec[kSlots], who[kSlots]; // an opened record and its lanes
   uint32_t part[kParts];             // lanes that accept a child
-  uint32_t starts[kPairs / 32];      // bit p: pair p is the first of a leaf
+  uint32_t starts[kTerms / 32];      // bit p: pair (or term) p starts a leaf (an item)
   uint16_t info[kSlots * 4];         // per child: kInfo bits | slot or pairs
   uint16_t partOf[kSlots * 4];       // per child with kInfoPart: index in part
-  uint16_t cell[kCells];             // cells in order: slot << 2 | child
-  uint16_t leaf[kLeaves];            // leaves in order
+  // in order, as slot << 2 | child: cells, leaves, or both: an item is a cell
+  // or (| kItemLeaf) a leaf
+  union {
+    struct {
+      uint16_t cell[kCells], leaf[kLeaves];
+    };
+    uint16_t item[kCells + kLeaves];
+  };
   uint8_t batch[kSlots];             // first slot of each batch
 };
-static_assert(kSlots <= 256 && kSlots * 4 < 1024 && kPairs < 4096, "packed fields");
+static_assert(kSlots <= 256 && kSlots * 4 < 1024 && kPairs < 4096 && kPairs <= kTerms,
+              "packed fields");
+constexpr uint32_t kItemLeaf = 1024u;
+// What a group walk sums: the default law; the reference's operations; the
+// default law with the quadrupole term.  The last two add a target's cells and
+// bodies to one sum in the order of its walk (as walk_targets does).
+enum GroupWalk { kPlainWalk, kExactWalk, kQuadWalk };
 // a child's low byte: the slot of its opened record, or an opened leaf's pairs
 constexpr uint32_t kInfoLeaf = 1u << 8, kInfoInner = 1u << 9;
 constexpr uint32_t kInfoTerm = 1u << 10, kInfoPart = 1u << 11; // accepted, by some only
@@ -416,6 +437,9 @@ constexpr uint32_t kInfoTerm = 1u << 10, kInfoPart = 1u << 11; // accepted, by s
 //    forwards to place them, which lists the terms in preorder;
 //  * all lanes sum the lists, each term with the mask of the lanes it belongs
 //    to: the law in pairs, the cells' accumulation one by one in order.
+// kExactWalk and kQuadWalk are walk_targets' results bit for bit: cells and
+// leaves are listed together, a term a place, and summed in one order, with
+// the arithmetic written there.
 // Returns false, with nothing summed, if the group's records do not fit.
 //
 // Two discs of 2^20 bodies, theta 0.5, per group: 95 records in 12 batches, 229
@@ -429,9 +453,25 @@ constexpr uint32_t kInfoTerm = 1u << 10, kInfoPart = 1u << 11; // accepted, by s
 // counting or placing, but another order of the sums); eight records at a
 // time (630); 24 or 28 warps per SM at fewer registers (620, 640); both
 // loops over terms unrolled twice more (645); the guess as one mad.hi (+13%).
-__device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float eSq, float x,
-                                           float y, uint32_t sg, uint32_t valid,
+template <GroupWalk kWalk>
+__device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float eSq, float bandSq,
+                                           float x, float y, uint32_t sg, uint32_t valid,
                                            WalkStage &st, float &axOut, float &ayOut) {
+  constexpr bool kExact = kWalk == kExactWalk, kOneOrder = kWalk != kPlainWalk;
+  // (dx^2 + dy^2) theta^2 of two nodes with the roundings of a target's own
+  // test.  (Exact: scalar, since a paired multiply and add came out fused and
+  // decided one test in 10^7 otherwise.)
+  auto far_of = [&](f2x dx, f2x dy, float &f0, float &f1) {
+    if (kExact) {
+      float x0, x1, y0, y1;
+      upk2(dx, x0, x1);
+      upk2(dy, y0, y1);
+      f0 = __fmul_rn(sq_dist<true>(x0, y0), tSq);
+      f1 = __fmul_rn(sq_dist<true>(x1, y1), tSq);
+    } else {
+      upk2(mul2(fma2(dx, dx, mul2(dy, dy)), pk2(tSq, tSq)), f0, f1);
+    }
+  };
   const int lane = threadIdx.x & 31;
   const uint32_t laneBit = 1u << lane, below = laneBit - 1u;
   const f2x XX = pk2(x, x), YY = pk2(y, y), E2 = pk2(eSq, eSq), N3 = pk2(-3.0f, -3.0f);
@@ -440,7 +480,6 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
   uint32_t tail = 1, batches = 0;
   const int half = lane & 1;
   {
-    const f2x T2 = pk2(tSq, tSq);
     f2x LOX, HIX, LOY, HIY;
     {
       const float loX = warp_min(x), hiX = warp_max(x), loY = warp_min(y), hiY = warp_max(y);
@@ -453,9 +492,9 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
       st.rec[0] = S.n + sg;
       st.who[0] = valid;
     }
-    if (lane < kPairs / 32) st.starts[lane] = 0u;
+    for (int k = lane; k < (kOneOrder ? kTerms : kPairs) / 32; k += 32) st.starts[k] = 0u;
     __syncwarp();
-    uint32_t parts = 0, lanePairs = 0;
+    uint32_t parts = 0, lanePairs = 0, laneItems = 0;
     for (uint32_t head = 0; head < tail;) {
       const uint32_t take = min((uint32_t)kTake, tail - head);
       const uint32_t slot = head + (lane >> 1);
@@ -486,8 +525,8 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
         const f2x NY = pk2(fmaxf(fmaxf(ay0[0], ay1[0]), 0.0f), fmaxf(fmaxf(ay0[1], ay1[1]), 0.0f));
         const f2x FX = pk2(fminf(ax0[0], ax1[0]), fminf(ax0[1], ax1[1]));
         const f2x FY = pk2(fminf(ay0[0], ay1[0]), fminf(ay0[1], ay1[1]));
-        upk2(mul2(fma2(NX, NX, mul2(NY, NY)), T2), near2[0], near2[1]);
-        upk2(mul2(fma2(FX, FX, mul2(FY, FY)), T2), far2[0], far2[1]);
+        far_of(NX, NY, near2[0], near2[1]);
+        far_of(FX, FY, far2[0], far2[1]);
       }
       uint32_t accept[2], info[2], lanes[2];
       bool split[2];
@@ -523,7 +562,7 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
           const float2 cw2 = *reinterpret_cast<const float2 *>(&st.cw[k]);
           const uint2 m = *reinterpret_cast<const uint2 *>(&st.cm[k]);
           float r0, r1;
-          upk2(mul2(fma2(DX, DX, mul2(DY, DY)), T2), r0, r1);
+          far_of(DX, DY, r0, r1);
           const uint32_t a0 = m.x & __ballot_sync(0xffffffffu, cw2.x < r0);
           const uint32_t a1 = m.y & __ballot_sync(0xffffffffu, cw2.y < r1);
           if (lane == 0) *reinterpret_cast<uint2 *>(&st.ca[k]) = make_uint2(a0, a1);
@@ -546,10 +585,16 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
       for (int j = 0; j < 2; ++j) {
         open[j] = lanes[j] & ~accept[j];
         inner[j] = open[j] != 0 && !(link[j] & kQuadLeaf);
-        if (accept[j]) info[j] |= kInfoTerm;
+        if (accept[j]) {
+          info[j] |= kInfoTerm;
+          ++laneItems;
+        }
         if (open[j] != 0 && !inner[j]) {
-          const uint32_t pairs = ((link[j] & ~kQuadLeaf) + 1u) >> 1;
+          // an odd leaf's last body has a pair of its own
+          const uint32_t bodies = link[j] & ~kQuadLeaf;
+          const uint32_t pairs = kOneOrder ? bodies : (bodies + 1u) >> 1;
           lanePairs += min(pairs, 65536u);
+          ++laneItems;
           info[j] |= (pairs & 255u) | kInfoLeaf;
           if (pairs > 255u) lanePairs = 65536u; // does not fit the byte
         }
@@ -575,12 +620,14 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
       if (tail > kSlots || parts > kParts) return false;
       __syncwarp();
     }
-    if (__reduce_add_sync(0xffffffffu, lanePairs) > kPairs) return false;
+    if (__reduce_add_sync(0xffffffffu, lanePairs) > (kOneOrder ? kTerms : kPairs)) return false;
+    if (kOneOrder && __reduce_add_sync(0xffffffffu, laneItems) > kCells + kLeaves) return false;
   }
   // subtree counts, from the last batch to the first
   auto child_terms = [&](uint32_t info) {
-    uint32_t v = info & kInfoTerm ? 1u : 0u;
-    if (info & kInfoLeaf) v += (info & 255u) << 20 | 1u << 10;
+    uint32_t v = info & kInfoTerm ? (kOneOrder ? 1u | 1u << 10 : 1u) : 0u;
+    if (info & kInfoLeaf)
+      v += kOneOrder ? (info & 255u) << 10 | 1u : (info & 255u) << 20 | 1u << 10;
     if (info & kInfoInner) v += st.count[info & 255u];
     return v;
   };
@@ -595,8 +642,8 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
     __syncwarp();
   }
   const uint32_t total = st.count[0], nCells = total & 1023u, nLeaves = total >> 10 & 1023u;
-  const uint32_t nPairs = total >> 20;
-  if (nCells > kCells || nLeaves > kLeaves) return false;
+  const uint32_t nPairs = total >> 20, nTerms = total >> 10;
+  if (kOneOrder ? nTerms > kTerms : nCells > kCells || nLeaves > kLeaves) return false;
   __syncwarp();
   if (lane == 0) st.count[0] = 0;
   __syncwarp();
@@ -614,11 +661,26 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const uint16_t code = (uint16_t)(slot << 2 | (2 * half + j));
-        if (info[j] & kInfoTerm) st.cell[at & 1023u] = code;
-        if (info[j] & kInfoInner) st.count[info[j] & 255u] = at + (info[j] & kInfoTerm ? 1u : 0u);
-        if (info[j] & kInfoLeaf) {
-          st.leaf[at >> 10 & 1023u] = code;
-          atomicOr(&st.starts[at >> 25], 1u << (at >> 20 & 31u));
+        if (kOneOrder) {
+          uint32_t own = at;
+          if (info[j] & kInfoTerm) {
+            st.item[own & 1023u] = code;
+            atomicOr(&st.starts[own >> 15], 1u << (own >> 10 & 31u));
+            own += 1u | 1u << 10;
+          }
+          if (info[j] & kInfoInner) st.count[info[j] & 255u] = own;
+          if (info[j] & kInfoLeaf) {
+            st.item[own & 1023u] = (uint16_t)(code | kItemLeaf);
+            atomicOr(&st.starts[own >> 15], 1u << (own >> 10 & 31u));
+          }
+        } else {
+          if (info[j] & kInfoTerm) st.cell[at & 1023u] = code;
+          if (info[j] & kInfoInner)
+            st.count[info[j] & 255u] = at + (info[j] & kInfoTerm ? 1u : 0u);
+          if (info[j] & kInfoLeaf) {
+            st.leaf[at >> 10 & 1023u] = code;
+            atomicOr(&st.starts[at >> 25], 1u << (at >> 20 & 31u));
+          }
         }
         at += v[j];
       }
@@ -630,8 +692,94 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
     const uint32_t info = st.info[code];
     return info & kInfoTerm ? (info & kInfoPart ? st.part[st.partOf[code]] : lanes) : 0u;
   };
-  // the cells, 64 at a time, two to a lane (the next ones' loads under way)
   float ax = 0.0f, ay = 0.0f;
+  if (kOneOrder) {
+    // the terms in order, 32 at a time (the next ones' loads under way)
+    float4 q, mom;
+    uint32_t qm;
+    uint32_t before = 0, last = 0; // items that start before the terms fetched
+                                   // next, and the last one's first term
+    auto fetch = [&](uint32_t base) {
+      q = mom = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+      qm = 0;
+      if (base >= nTerms) return;
+      const uint32_t word = st.starts[base >> 5], mine = word & (laneBit | below);
+      if (base + lane < nTerms) {
+        const uint32_t item = st.item[before + __popc(mine) - 1u], code = item & 1023u;
+        const uint32_t slot = code >> 2, c = code & 3u;
+        const QuadRec *r = tQ + st.rec[slot];
+        const uint32_t lanes = st.who[slot], in = accepts(code, lanes);
+        if (item & kItemLeaf) {
+          const uint32_t j = base + lane - (mine ? base + 31u - __clz(mine) : last);
+          const uint32_t b = __ldg(&r->child[c].y) + j;
+          if (b < S.n) { // defensive bound
+            const float4 v = S.xym[b];
+            q = make_float4(v.x, v.y, v.z, -1.0f);
+          }
+          qm = lanes & ~in;
+        } else {
+          q.x = __ldg(reinterpret_cast<const float *>(&r->x) + c);
+          q.y = __ldg(reinterpret_cast<const float *>(&r->y) + c);
+          q.z = __ldg(reinterpret_cast<const float *>(&r->m) + c);
+          qm = q.z > 0.0f ? in : 0u; // the reference adds a cell only with mass
+          if (kWalk == kQuadWalk) mom = __ldg(&S.tQM[st.rec[slot]].m[c]);
+        }
+      }
+      before += __popc(word);
+      if (word) last = base + 31u - __clz(word);
+    };
+    fetch(0);
+    for (uint32_t base = 0; base < nTerms; base += kChunk) {
+      st.q[lane] = q;
+      if (kWalk == kQuadWalk) st.mom[lane] = mom;
+      st.lanes[lane] = qm;
+      __syncwarp();
+      fetch(base + kChunk);
+      const uint32_t n = min((uint32_t)kChunk, nTerms - base);
+#pragma unroll 4
+      for (uint32_t k = 0; k < n; ++k) {
+        const float4 v = st.q[k];
+        const bool on = (st.lanes[k] & laneBit) != 0;
+        const float dx = kExact ? __fsub_rn(v.x, x) : v.x - x;
+        const float dy = kExact ? __fsub_rn(v.y, y) : v.y - y;
+        const float dSq = sq_dist<kExact>(dx, dy);
+        const float fac = law_factor<kExact, kExact>(dSq, v.z, eSq);
+        float tx, ty;
+        if (kExact) {
+          tx = __fadd_rn(ax, __fmul_rn(dx, fac));
+          ty = __fadd_rn(ay, __fmul_rn(dy, fac));
+        } else {
+          tx = fmaf(dx, fac, ax);
+          ty = fmaf(dy, fac, ay);
+        }
+        if (kWalk == kQuadWalk) {
+          const float4 M = st.mom[k]; // a body's size is -1: never in the band
+          // the node of the chain that the target accepts: the largest one that
+          // passes (each is exactly a quarter of the last)
+          float w = M.w;
+          while (w >= dSq * tSq && on) w *= 0.25f;
+          const bool band = on && w >= dSq * bandSq;
+          if (__ballot_sync(0xffffffffu, band)) {
+            float qx, qy;
+            quad_term(dx, dy, dSq, eSq, v.z, M.x, M.y, M.z, qx, qy);
+            if (band) {
+              tx = ax + fac * (dx + qx);
+              ty = ay + fac * (dy + qy);
+            }
+          }
+        }
+        ax = on ? tx : ax;
+        ay = on ? ty : ay;
+      }
+      __syncwarp();
+    }
+    if (valid & laneBit) {
+      axOut = ax;
+      ayOut = ay;
+    }
+    return true;
+  }
+  // the cells, 64 at a time, two to a lane (the next ones' loads under way)
   {
     float qx[2], qy[2], qh[2];
     uint32_t qm[2];
@@ -645,7 +793,7 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
           const QuadRec *q = tQ + st.rec[slot];
           qx[j] = __ldg(reinterpret_cast<const float *>(&q->x) + c);
           qy[j] = __ldg(reinterpret_cast<const float *>(&q->y) + c);
-          qh[j] = __ldg(reinterpret_cast<const float *>(&q->halfM) + c);
+          qh[j] = 0.5f * __ldg(reinterpret_cast<const float *>(&q->m) + c);
           qm[j] = accepts(code, st.who[slot]);
         }
       }
@@ -883,23 +1031,27 @@ __global__ void __launch_bounds__(kBlock, kCorr == 1 ? 3
                                                      nQuery, queryAcc, sBody, sW, sStage);
 }
 
-// Sums of the plain walk for the targets of `lanes` (places (x, y), a valid
-// one on every lane) in instance sg: walk_group, walk_plain_x2 where that
-// does not fit, and the clamped walk for an instance that reaches beyond the
-// coordinate limit, as in k_forces.
-__device__ __forceinline__ void group_forces(const DevState &S, float tSq, float eSq, float x,
-                                             float y, uint32_t sg, uint32_t lanes, WalkStage &st,
+// Sums of a group walk for the targets of `lanes` (places (x, y), a valid
+// one on every lane) in instance sg: walk_group, the cursor walk where that
+// does not fit, and, for an instance that reaches beyond the coordinate limit,
+// the clamped one (exact arithmetic always clamps), as in k_forces.
+template <GroupWalk kWalk>
+__device__ __forceinline__ void group_forces(const DevState &S, float tSq, float eSq,
+                                             float bandSq, float eps, float x, float y,
+                                             uint32_t sg, uint32_t lanes, WalkStage &st,
                                              float &ax, float &ay) {
+  constexpr bool kExact = kWalk == kExactWalk;
+  constexpr int kCorr = kWalk == kQuadWalk ? 2 : 0;
   const int lane = threadIdx.x & 31;
   const SegDev &G = S.seg[sg];
   if (G.travCount == 0) return; // no tree (capacity)
   float4 *staged = reinterpret_cast<float4 *>(&st);
   static_assert(sizeof(WalkStage) >= 32 * sizeof(float4), "holds a leaf's staged bodies");
+  uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
   if (G.wide) {
-    uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
-    walk_targets<false, false, 0, true>(S, tSq, eSq, 0.0f, 0.0f, x, y,
-                                        (lanes >> lane) & 1u ? G.travBase : kDone, staged,
-                                        nullptr, nullptr, ax, ay, c0, c1, c2, c3, c4);
+    walk_targets<kExact, false, kCorr, true>(S, tSq, eSq, bandSq, eps, x, y,
+                                             (lanes >> lane) & 1u ? G.travBase : kDone, staged,
+                                             nullptr, nullptr, ax, ay, c0, c1, c2, c3, c4);
     return;
   }
   // A group whose walk does not fit goes in two at the widest step along its
@@ -912,7 +1064,7 @@ __device__ __forceinline__ void group_forces(const DevState &S, float tSq, float
     const float leadX = __shfl_sync(0xffffffffu, x, lead);
     const float leadY = __shfl_sync(0xffffffffu, y, lead);
     const float px = in ? x : leadX, py = in ? y : leadY;
-    if (!walk_group(S, tSq, eSq, px, py, sg, piece, st, ax, ay)) {
+    if (!walk_group<kWalk>(S, tSq, eSq, bandSq, px, py, sg, piece, st, ax, ay)) {
       __syncwarp();
       const float nx = __shfl_down_sync(0xffffffffu, px, 1);
       const float ny = __shfl_down_sync(0xffffffffu, py, 1);
@@ -925,9 +1077,15 @@ __device__ __forceinline__ void group_forces(const DevState &S, float tSq, float
         piece &= (at & (0u - at)) * 2u - 1u; // the lanes up to the step
         continue;
       }
-      float *sX = reinterpret_cast<float *>(staged);
-      float wx, wy;
-      walk_plain_x2(S, tSq, eSq, x, y, in ? G.travBase : kDone, sX, sX + 32, sX + 64, wx, wy);
+      const uint32_t root = in ? G.travBase : kDone;
+      float wx = 0.0f, wy = 0.0f;
+      if (kWalk == kPlainWalk) {
+        float *sX = reinterpret_cast<float *>(staged);
+        walk_plain_x2(S, tSq, eSq, x, y, root, sX, sX + 32, sX + 64, wx, wy);
+      } else {
+        walk_targets<kExact, false, kCorr, kExact>(S, tSq, eSq, bandSq, eps, x, y, root, staged,
+                                                   nullptr, nullptr, wx, wy, c0, c1, c2, c3, c4);
+      }
       if (in) {
         ax = wx;
         ay = wy;
@@ -938,12 +1096,13 @@ __device__ __forceinline__ void group_forces(const DevState &S, float tSq, float
   }
 }
 
-// The default force pass (leaf_pairs 1), one group of targets per warp.
+// A force pass, one group of targets per warp: the default one (leaf_pairs 1),
+// exact arithmetic, or the quadrupole term.
 constexpr int kGroupWarpsPerSM = 20;
-template <int kBlock>
+template <int kBlock, GroupWalk kWalk>
 __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
                                               ? kGroupWarpsPerSM * 32 / kBlock : 1)
-    k_forces_groups(DevState S, float tSq, float eSq) {
+    k_forces_groups(DevState S, float tSq, float eSq, float bandSq, float eps) {
   chain_begin();
   extern __shared__ uint4 sDyn[]; // a WalkStage per warp
   const int lane = threadIdx.x & 31;
@@ -960,8 +1119,9 @@ __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
     const uint32_t i = mine ? first + lane : first;
     const float4 b = S.xym[i];
     float ax = 0.0f, ay = 0.0f;
-    group_forces(S, tSq, eSq, b.x, b.y, sg, __ballot_sync(0xffffffffu, mine), st, ax, ay);
-    if (mine) store_acc<false>(S, i, b.x, b.y, ax, ay);
+    group_forces<kWalk>(S, tSq, eSq, bandSq, eps, b.x, b.y, sg,
+                        __ballot_sync(0xffffffffu, mine), st, ax, ay);
+    if (mine) store_acc<kWalk == kExactWalk>(S, i, b.x, b.y, ax, ay);
     __syncwarp();
   }
 }
@@ -969,6 +1129,7 @@ __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
 // The same sums at query points (instance 0's tree), `per` consecutive points
 // to a warp.
 constexpr int kQueryBlock = 128;
+template <GroupWalk kWalk>
 __global__ void __launch_bounds__(kQueryBlock, kGroupWarpsPerSM * 32 / kQueryBlock)
     k_query_groups(DevState S, float tSq, float eSq, const float2 *__restrict__ query,
                    uint32_t nQuery, uint32_t per, float2 *__restrict__ queryAcc) {
@@ -983,7 +1144,8 @@ __global__ void __launch_bounds__(kQueryBlock, kGroupWarpsPerSM * 32 / kQueryBlo
   const uint32_t i = (uint32_t)first + (mine ? lane : 0);
   const float2 q = query[i];
   float ax = 0.0f, ay = 0.0f;
-  group_forces(S, tSq, eSq, q.x, q.y, 0u, __ballot_sync(0xffffffffu, mine), st, ax, ay);
+  group_forces<kWalk>(S, tSq, eSq, 0.0f, 0.0f, q.x, q.y, 0u, __ballot_sync(0xffffffffu, mine),
+                      st, ax, ay);
   if (mine) queryAcc[i] = make_float2(ax, ay);
 }
 
@@ -1098,28 +1260,36 @@ bool group_walk_fits(const DevState &S) {
   return 0.5f * log2f(fmaxf(n / L, 1.0f)) <= 40.0f * S.tSq && L * near * near <= 330.0f;
 }
 
+template <int kBlock, GroupWalk kWalk>
+void launch_groups(cudaStream_t s, const DevState &S, int blocks, float band, bool chained) {
+  constexpr int smem = kBlock / 32 * (int)sizeof(WalkStage);
+  if (smem > 48 * 1024) // above what a launch may ask for by default
+    cudaFuncSetAttribute(k_forces_groups<kBlock, kWalk>,
+                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (blocks <= 0) {
+    const uint32_t warps = (S.tgEnd ? S.tgEnd : S.nGroups) - S.tgBegin, per = kBlock / 32;
+    blocks = (int)std::max(1u, (warps + per - 1) / per);
+  }
+  if (chained)
+    launch_after(s, k_forces_groups<kBlock, kWalk>, blocks, kBlock, smem, S, S.tSq, S.eSq,
+                 band * band, sqrtf(S.eSq));
+  else
+    k_forces_groups<kBlock, kWalk>
+        <<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq, band * band, sqrtf(S.eSq));
+}
+
 // The default plain walk with kBlock threads per block and the paired or
 // single-body leaf loop.
 template <int kBlock>
 void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, bool groups,
                   bool chained) {
-  if (blocks <= 0) {
-    uint32_t warps = (force_targets(S) + 31) / 32;
-    const uint32_t per = kBlock / 32;
-    if (pairs && groups) warps = (S.tgEnd ? S.tgEnd : S.nGroups) - S.tgBegin;
+  const bool whole = blocks <= 0;
+  if (whole) {
+    const uint32_t warps = (force_targets(S) + 31) / 32, per = kBlock / 32;
     const uint32_t b = (warps + per - 1) / per;
     blocks = (int)(b ? b : 1);
   }
-  if (pairs && groups) {
-    constexpr int smem = kBlock / 32 * (int)sizeof(WalkStage);
-    if (smem > 48 * 1024) // above what a launch may ask for by default
-      cudaFuncSetAttribute(k_forces_groups<kBlock>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (chained)
-      launch_after(s, k_forces_groups<kBlock>, blocks, kBlock, smem, S, S.tSq, S.eSq);
-    else
-      k_forces_groups<kBlock><<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq);
-  }
+  if (pairs && groups) launch_groups<kBlock, kPlainWalk>(s, S, whole ? 0 : blocks, 0.0f, chained);
   else if (pairs)
     k_forces<false, false, 0, false, kBlock, true><<<blocks, kBlock, 0, s>>>(S, S.tSq, S.eSq);
   else
@@ -1157,15 +1327,15 @@ void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool gro
     query = sorted;
     out = accSorted;
   }
-  if (!exact && groups && group_walk_fits(S)) {
+  if ((exact || groups) && group_walk_fits(S)) {
     uint32_t per = 32;
     while (per > 1 && ((nq + per - 1) / per < 148u * kGroupWarpsPerSM ||
                        (uint64_t)per * S.n > 64ull * nq))
       per >>= 1;
     const uint32_t warps = (nq + per - 1) / per;
-    k_query_groups<<<(warps * 32 + kQueryBlock - 1) / kQueryBlock, kQueryBlock,
-                     kQueryBlock / 32 * sizeof(WalkStage), s>>>(S, S.tSq, S.eSq, query, nq, per,
-                                                                out);
+    auto kernel = exact ? k_query_groups<kExactWalk> : k_query_groups<kPlainWalk>;
+    kernel<<<(warps * 32 + kQueryBlock - 1) / kQueryBlock, kQueryBlock,
+             kQueryBlock / 32 * sizeof(WalkStage), s>>>(S, S.tSq, S.eSq, query, nq, per, out);
   } else {
     const uint32_t b = ((nq + 31) / 32 + kWarps - 1) / kWarps;
     if (exact)
@@ -1191,6 +1361,23 @@ void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
     else if (threads == 512) launch_plain<512>(s, S, blocks, pairs, groups, chained);
     else launch_plain<256>(s, S, blocks, pairs, groups, chained);
     return;
+  }
+  // The walks that keep one order, in groups too where those fit and a
+  // cursor's ~300 dependent loads count: us with a cursor / in groups, exact,
+  // theta 0.5: 10,000 bodies 88 / 61, 30,000 119 / 84, 100,000 175 / 164, 262,147
+  // 311 / 313, 2^20 1072 / 1142 (theta 1: 100,000 75 / 84); the quadrupole
+  // term, theta 0.65, band 0.4: 10,000 66 / 53, 30,000 84 / 66, 100,000 121 / 135,
+  // 2^20 746 / 967: scalar sums and terms of every lane's, unlike the plain
+  // walk's pairs, are all they have to offer once there are warps enough.
+  if (S.n <= 65536u && group_walk_fits(S)) {
+    if (corr == 0 && exact) {
+      launch_groups<128, kExactWalk>(s, S, blocks, 0.0f, chained);
+      return;
+    }
+    if (corr == 2 && noClamp) {
+      launch_groups<128, kQuadWalk>(s, S, blocks, band, chained);
+      return;
+    }
   }
   if (blocks <= 0) {
     uint32_t warps = (force_targets(S) + 31) / 32;

@@ -41,9 +41,8 @@ struct alignas(32) TravNode {
 static_assert(sizeof(TravNode) == 32, "32-byte traversal records");
 
 // The (up to four) children of a branching node for the default force walk,
-// in digit order as arrays of four (lane c of four takes child c): centre
-// of mass, half the mass (the law's Newton step carries a factor 2) and
-// squared size; per child a link -- kQuadLeaf | body count for a leaf, the
+// in digit order as arrays of four: centre of mass, mass and squared size;
+// per child a link -- kQuadLeaf | body count for a leaf, the
 // child's own record otherwise -- and its first body.  An absent child has
 // no mass and a link to an empty leaf.
 // A chain of nodes with one non-empty child each is one child here: its
@@ -54,10 +53,15 @@ static_assert(sizeof(TravNode) == 32, "32-byte traversal records");
 // no other branching node shares: at most one record per body.  An
 // instance's root is the only child of a record of its own, n + instance.
 struct alignas(32) QuadRec {
-  float4 x, y, halfM, w;
+  float4 x, y, m, w;
   uint2 child[4]; // {link, first body}
 };
 static_assert(sizeof(QuadRec) == 96, "three 32-byte loads");
+// The same children for the quadrupole term: {Ixx, Iyy, Ixy, squared size of
+// the largest node of the child's chain}.
+struct alignas(32) QuadMom {
+  float4 m[4];
+};
 constexpr uint32_t kQuadLeaf = 0x80000000u;
 
 constexpr int kMaxDepth = 32;   // TreeKernels.cuh:29
@@ -165,7 +169,8 @@ struct DevState {
   uint4 *spanKids;
   // traversal layout (preorder)
   TravNode *tN; // preorder traversal records (32 bytes, one load each)
-  QuadRec *tQ; // records of the default force walk (n + nseg)
+  QuadRec *tQ;  // records of the group walks (n + nseg)
+  QuadMom *tQM; // their moments, where the build computes them
   float4 *tUp; // per traversal record, upward pass: {weighted sums x, y,
                // bottom size^2, link bits}; shares the breadth-first arrays'
                // storage (comX ..)
