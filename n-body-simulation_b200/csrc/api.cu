@@ -229,7 +229,8 @@ struct nbx_handle {
   uint32_t n = 0, nseg = 0;
   std::vector<uint32_t> segStart, segCount;
   std::vector<uint32_t> groupFirst; // DevState::groupFirst
-  std::vector<void *> allocs;
+  char *arena = nullptr; // every device array of the handle (see carve)
+  size_t arenaUsed = 0;
   DevState base{};       // buffer set A current
   int cur = 0;           // 0: state in set A (pv), 1: in set B (pv2)
   ScanScratch scan;
@@ -341,14 +342,13 @@ int cuda_fail(nbx_handle *h, cudaError_t e, const char *what) {
     if (e_ != cudaSuccess) return cuda_fail((h), e_, #call);                 \
   } while (0)
 
-template <typename T> cudaError_t dalloc(nbx_handle *h, T *&p, size_t count) {
-  void *v = nullptr;
-  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-  cudaError_t e = cudaMalloc(&v, bytes);
-  if (e != cudaSuccess) return e;
-  h->allocs.push_back(v);
-  p = static_cast<T *>(v);
-  return cudaMemset(v, 0, bytes);
+// The next piece of the handle's one device allocation: allocate() lays the
+// pieces out twice, first to add up their sizes (arena null), then to set the
+// pointers.  256-byte aligned, with as much again between pieces.
+template <typename T> void carve(nbx_handle *h, T *&p, size_t count) {
+  const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + 511) & ~(size_t)255;
+  p = h->arena ? reinterpret_cast<T *>(h->arena + h->arenaUsed) : nullptr;
+  h->arenaUsed += bytes;
 }
 
 uint32_t next_pow2(uint64_t v) {
@@ -371,8 +371,18 @@ int allocate(nbx_handle *h) {
   S.nBuckets = next_pow2(2ull * std::max<uint32_t>(n, 1));
   const uint32_t nodes = S.nodeCapacity;
   const uint32_t sortCap = 2 * n + 64;
-#define A(ptr, count) \
-  if (cudaError_t e = dalloc(h, ptr, count)) return cuda_fail(h, e, "cudaMalloc " #ptr)
+  h->groupFirst.clear();
+  S.nGroups = (n + 31) / 32; // one instance: group g starts at 32 g
+  if (ns > 1) {
+    for (uint32_t s = 0; s < ns; ++s)
+      for (uint32_t b = 0; b < h->segCount[s]; b += 32)
+        h->groupFirst.push_back(h->segStart[s] + b);
+    S.nGroups = (uint32_t)h->groupFirst.size();
+  }
+  const size_t spans = ((size_t)nodes / 256 + 1) * (kMaxDepth + 1);
+  size_t cleared = 0; // the pieces after it are written before they are read
+  auto layout = [&] {
+#define A(ptr, count) carve(h, ptr, count)
   A(S.seg, ns);
   A(S.segOf, n);
   A(S.pv, n);
@@ -435,33 +445,12 @@ int allocate(nbx_handle *h) {
   A(S.moments, nodes);
   A(S.subtree, nodes);
   A(S.arrive, nodes);
-  const size_t spans = ((size_t)nodes / 256 + 1) * (kMaxDepth + 1);
   A(S.spanParent, spans);
   A(S.spanArrive, spans);
   A(S.spanKids, spans);
-  NBX_CUDA(h, cudaMemset(S.spanKids, 0xff, spans * sizeof(uint4)));
   A(S.tN, nodes); // cudaMalloc: 256-byte aligned, so every record is 32
   A(S.tM, nodes);
-  { // written by every build before it is read: not cleared
-    void *v = nullptr;
-    if (cudaError_t e = cudaMalloc(&v, ((size_t)n + ns) * sizeof(QuadRec)))
-      return cuda_fail(h, e, "cudaMalloc S.tQ");
-    h->allocs.push_back(v);
-    S.tQ = static_cast<QuadRec *>(v);
-    if (cudaError_t e = cudaMalloc(&v, ((size_t)n + ns) * sizeof(QuadMom)))
-      return cuda_fail(h, e, "cudaMalloc S.tQM");
-    h->allocs.push_back(v);
-    S.tQM = static_cast<QuadMom *>(v);
-  }
-  h->groupFirst.clear();
-  S.nGroups = (n + 31) / 32; // one instance: group g starts at 32 g
-  if (ns > 1) {
-    for (uint32_t s = 0; s < ns; ++s)
-      for (uint32_t b = 0; b < h->segCount[s]; b += 32)
-        h->groupFirst.push_back(h->segStart[s] + b);
-    S.nGroups = (uint32_t)h->groupFirst.size();
-    A(S.groupFirst, S.nGroups);
-  }
+  if (ns > 1) A(S.groupFirst, S.nGroups);
   // scan / sort scratch
   SortScratch &so = h->sort;
   so.capacity = sortCap;
@@ -478,7 +467,6 @@ int allocate(nbx_handle *h) {
   A(sc.status, sc.maxTiles + 1);
   A(sc.slotStatus, (size_t)kScanSlots * sc.maxTiles);
   A(sc.tileCounter, kScanSlots);
-  A(sc.tileCounter, 1);
   A(h->dAoS, n);
   A(h->dF64, 16 * 592);
   A(S.tC, nodes);
@@ -488,7 +476,19 @@ int allocate(nbx_handle *h) {
   A(h->mlpGrad, kMlpParams + 1);
   A(h->mlpW, 1);
   A(S.attr, 2);
+  cleared = h->arenaUsed;
+  A(S.tQ, (size_t)n + ns); // written by every build
+  A(S.tQM, (size_t)n + ns);
 #undef A
+  };
+  h->arena = nullptr;
+  h->arenaUsed = 0;
+  layout();
+  NBX_CUDA(h, cudaMalloc(&h->arena, h->arenaUsed));
+  h->arenaUsed = 0;
+  layout();
+  NBX_CUDA(h, cudaMemset(h->arena, 0, cleared));
+  NBX_CUDA(h, cudaMemset(S.spanKids, 0xff, spans * sizeof(uint4)));
   NBX_CUDA(h, cudaMemcpy(S.attr, h->attrHost, sizeof(h->attrHost), cudaMemcpyHostToDevice));
   if (!h->groupFirst.empty())
     NBX_CUDA(h, cudaMemcpy(S.groupFirst, h->groupFirst.data(), S.nGroups * sizeof(uint32_t),
@@ -896,7 +896,7 @@ int nbx_destroy(nbx_handle *h) {
     if (h->ioDone[c]) cudaEventDestroy(h->ioDone[c]);
     if (h->ioStream[c]) cudaStreamDestroy(h->ioStream[c]);
   }
-  for (void *v : h->allocs) cudaFree(v);
+  if (h->arena) cudaFree(h->arena);
   for (void *v : h->scratch) cudaFree(v);
   if (h->hPinned) cudaFreeHost(h->hPinned);
   if (h->hWord) cudaFreeHost(h->hWord);
@@ -1434,8 +1434,8 @@ int nbx_reset(nbx_handle *h, const nbx_body *bodies, size_t n) {
                            cudaMemcpyDeviceToHost));
   }
   destroy_graphs(h);
-  for (void *v : h->allocs) cudaFree(v);
-  h->allocs.clear();
+  if (h->arena) cudaFree(h->arena);
+  h->arena = nullptr;
   for (void *v : h->scratch) cudaFree(v);
   h->scratch.clear();
   if (h->hPinned) cudaFreeHost(h->hPinned);
