@@ -447,6 +447,8 @@ int allocate(nbx_handle *h) {
   A(S.arrive, nodes);
   A(S.spanParent, spans);
   A(S.spanArrive, spans);
+  A(S.spanArriveTop, spans);
+  A(S.spanList, spans);
   A(S.spanKids, spans);
   A(S.tN, nodes); // cudaMalloc: 256-byte aligned, so every record is 32
   A(S.tM, nodes);

@@ -570,6 +570,61 @@ __device__ __forceinline__ uint32_t search8(uint32_t lo, uint32_t hi, Before bef
   return lo;
 }
 
+// Sums of a node from those of its children in `have`, in digit order
+// (sumNode), then finishNode's divide: up = {weighted sums, bottom size^2,
+// link}, own = {centre of mass, mass, size^2}, mom = {moments, size}.  One
+// child has the same bodies under a smaller square: its link goes up.  With
+// more the link is the node's own record, at its second child's first body;
+// record: write that too.
+template <bool kFull>
+__device__ __forceinline__ void sum_children(const DevState &S, uint32_t have,
+                                             const float4 (&cu)[4], const float4 (&ca)[4],
+                                             const float4 (&cm)[4], const uint32_t (&first)[4],
+                                             float w, float size, bool record, float4 &up,
+                                             float4 &own, float4 &mom) {
+  float sx = 0.0f, sy = 0.0f, sm = 0.0f, wBot = 0.0f;
+  uint32_t count = 0, link = 0, second = 0;
+#pragma unroll
+  for (uint32_t q = 0; q < 4; ++q) {
+    if (!((have >> q) & 1u)) continue;
+    sx = count == 0 ? cu[q].x : __fadd_rn(sx, cu[q].x);
+    sy = count == 0 ? cu[q].y : __fadd_rn(sy, cu[q].y);
+    sm = count == 0 ? ca[q].z : __fadd_rn(sm, ca[q].z);
+    if (count == 0) {
+      wBot = cu[q].z;
+      link = __float_as_uint(cu[q].w);
+    }
+    if (count == 1) second = first[q];
+    ++count;
+  }
+  const float dv = fmaxf(sm, FLT_MIN);
+  const float X = __fdiv_rn(sx, dv), Y = __fdiv_rn(sy, dv);
+  if (kFull) {
+    float jxx = 0.0f, jyy = 0.0f, jxy = 0.0f;
+#pragma unroll
+    for (uint32_t q = 0; q < 4; ++q) {
+      if (!((have >> q) & 1u)) continue;
+      const float dx = ca[q].x - X, dy = ca[q].y - Y;
+      jxx += cm[q].x + ca[q].z * dx * dx;
+      jyy += cm[q].y + ca[q].z * dy * dy;
+      jxy += cm[q].z + ca[q].z * dx * dy;
+    }
+    mom = make_float4(jxx, jyy, jxy, size);
+  }
+  if (count > 1) {
+    wBot = w;
+    link = second;
+    if (record) quad_record<kFull>(S, second, X, Y, have, cu, ca, cm, first);
+  }
+  up = make_float4(sx, sy, wBot, __uint_as_float(link));
+  own = make_float4(X, Y, sm, w);
+}
+
+// Place of a spanning node (k_trav_tree) in the arrays span*.
+__device__ __forceinline__ uint32_t span_slot(uint32_t record, int depth) {
+  return record / kBlock * (kMaxDepth + 1) + (uint32_t)depth;
+}
+
 // The traversal records and their sums in one pass, a thread to a record, 256
 // consecutive records (preorder) to a block.
 //
@@ -580,26 +635,23 @@ __device__ __forceinline__ uint32_t search8(uint32_t lo, uint32_t hi, Before bef
 // last record's ancestors are searched for in the codes, one per depth, eight
 // probes a round.
 //
-// Then upwards: a leaf sums its bodies (sumNode's order) and climbs, and the
-// last child to arrive at a node sums its children in digit order, then
-// finishNode's divide, and climbs on.  A child leaves its record at its digit
-// of the node and adds its bodies to the node's arrival counter, which is
-// complete at the node's body count.
-//  * A node whose whole subtree lies in the block (most but the top few) has
-//    its counter and its children's sums in shared memory.
-//  * A node that reaches beyond the block has them in global memory, at
-//    (block, depth), which no other such node of the block shares; its own
-//    thread, once it has published the node, subtracts the body count.  Who
-//    brings the counter to 0 is the last and finds everything published; the
-//    counter is 0 and the children's slots are empty again for the next build.
+// Then upwards, as far as subtrees lie in the block (all nodes but the top
+// few): a leaf sums its bodies (sumNode's order) and climbs, and the last child
+// to arrive at a node sums its children and climbs on.  A child leaves its
+// place at its digit of the node and adds its bodies to the node's arrival
+// counter, which is complete at the node's body count.  A node that reaches
+// beyond the block ("spans") has its children's records and counter in global
+// memory, at (block, depth), which no other spanning node of the block shares;
+// k_trav_top sums those, from the children found here.
 // kFull: also the cell centres and sizes of tC/tM and the second moments
 // about each centre of mass (read only by the corrected forms and the
 // network's harvest).
 // Bound by the latency of dependent loads.  us between events around the
-// stage, as two kernels with child bounds, parents and ends all searched by
-// bisection and every arrival through global memory -> now: 10,000 bodies
-// 43 -> 29, 99,991 53 -> 34, 2^20 86 -> 71.  At 128 registers (2 blocks per SM)
-// 2 us less below 10^5 bodies and 20 more for 2^22.
+// stage with k_trav_top: as two kernels, with child bounds, parents and ends
+// all bisected and every arrival through global memory, 10,000 bodies 43,
+// 99,991 53, 2^20 86, 2^22 167 without the quad records; with the spanning nodes
+// summed here, whose threads held their blocks, 31, 34, 70, 228; now 28, 34, 65,
+// 159.
 template <bool kFull>
 __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
     k_trav_tree(DevState S, const uint32_t *__restrict__ owner) {
@@ -742,11 +794,19 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
       sParent[t] = parent;
       sBodies[t] = e - i;
       sSpans[t] = spans ? 1u : 0u;
-      if (spans) { // published by its arrival below
-        __stcg(&S.tN[p].a, make_float4(0.0f, 0.0f, 0.0f, w));
-        if (kFull) __stcg(&S.tM[p], make_float4(0.0f, 0.0f, 0.0f, size));
-        __stcg(&S.spanParent[p / kBlock * (kMaxDepth + 1) + d], parent);
+      if (spans) { // for k_trav_top
+        S.tN[p].a = make_float4(0.0f, 0.0f, 0.0f, w);
+        if (kFull) S.tM[p] = make_float4(0.0f, 0.0f, 0.0f, size);
+        S.spanParent[span_slot(p, d)] = parent;
       }
+    }
+    // the spanning nodes' list
+    const uint32_t spanning = __ballot_sync(0xffffffffu, spans);
+    if (spanning) {
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&S.counters[kCtrSpans], (uint32_t)__popc(spanning));
+      at = __shfl_sync(0xffffffffu, at, 0) + __popc(spanning & ((1u << lane) - 1u));
+      if (spans) S.spanList[at] = make_uint2(p, (uint32_t)d);
     }
     __syncthreads();
     // the node this thread holds the sums of: its record, depth and bodies
@@ -783,138 +843,54 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
       up = make_float4(px, py, w, __uint_as_float(kQuadLeaf | (e - i)));
       own = make_float4(X, Y, mm, w);
     }
-    // at most kMaxDepth + 1 nodes; record indices are range-checked
-    bool publish = spans; // first the arrival of the node's own thread
-    for (int guard = 0; (leaf || spans) && guard <= kMaxDepth + 1; ++guard) {
-      uint32_t l = kBlock; // the next node's place in the block, if summed there
-      uint32_t slot = 0;   // else its place among the nodes beyond a block
-      if (publish) {
-        slot = p / kBlock * (kMaxDepth + 1) + d;
-      } else { // `node` is summed: keep it and arrive at its parent
-        const uint32_t in = node - base;
-        if (in < kBlock) { // its thread stores it at the end, unless it spans
-          sUp[in] = up;
-          sA[in] = own;
-          if (kFull) sM[in] = mom;
-        }
-        if (in >= kBlock || sSpans[in] != 0) {
-          __stcg(&S.tN[node].a, own);
-          if (kFull) __stcg(&S.tM[node], mom);
-        }
-        if (d == 0) {
-          quad_root<kFull>(S, sg, up, own, mom);
-          break;
-        }
-        const uint32_t parent = in < kBlock ? sParent[in]
-                                            : __ldcg(&S.spanParent[node / kBlock * (kMaxDepth + 1) + d]);
-        if (parent >= total) {
-          atomicOr(S.status, kStatusTreeCapacity);
-          break;
-        }
-        --d;
-        const uint32_t digit = (uint32_t)digit_at(ci, d); // ci lies in the node
-        l = parent - base;
-        if (l < kBlock && sSpans[l] == 0) {
-          reinterpret_cast<uint8_t *>(&sKids[l])[digit] = (uint8_t)(in - l - 1u);
-          __threadfence_block();
-          if (atomicAdd(&sArrive[l], bodies) + bodies != sBodies[l]) break;
-          __threadfence_block();
-        } else {
-          l = kBlock;
-          slot = parent / kBlock * (kMaxDepth + 1) + d;
-          __stcg(&S.tN[node].a, own);
-          if (kFull) __stcg(&S.tM[node], mom);
-          __stcg(&S.tUp[node], up);
-          __stcg(reinterpret_cast<uint32_t *>(&S.spanKids[slot]) + digit, node);
-        }
-        node = parent;
+    // at most kMaxDepth + 1 nodes, all in the block
+    for (int guard = 0; leaf && guard <= kMaxDepth; ++guard) {
+      // `node` is summed: keep it (its thread stores it below) and arrive at its
+      // parent
+      const uint32_t in = node - base;
+      sUp[in] = up;
+      sA[in] = own;
+      if (kFull) sM[in] = mom;
+      if (d == 0) {
+        quad_root<kFull>(S, sg, up, own, mom);
+        break;
       }
-      const bool local = l < kBlock;
-      if (!local) {
-        // release: what this thread published is visible to the last arriver;
-        // acquire: the last arriver sees all
-        const uint32_t add = publish ? 0u - bodies : bodies;
-        uint32_t old;
-        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
-                     : "=r"(old)
-                     : "l"(&S.spanArrive[slot]), "r"(add)
-                     : "memory");
-        if (old + add != 0u) break;
-        publish = false;
+      const uint32_t parent = sParent[in];
+      if (parent >= total) {
+        atomicOr(S.status, kStatusTreeCapacity);
+        break;
       }
+      --d;
+      const uint32_t digit = (uint32_t)digit_at(ci, d); // ci lies in the node
+      const uint32_t l = parent - base;
+      if (l >= kBlock || sSpans[l] != 0) {
+        const uint32_t slot = span_slot(parent, d);
+        S.tUp[node] = up;
+        reinterpret_cast<uint32_t *>(&S.spanKids[slot])[digit] = node;
+        atomicAdd(&S.spanArrive[slot], bodies);
+        break;
+      }
+      reinterpret_cast<uint8_t *>(&sKids[l])[digit] = (uint8_t)(in - l - 1u);
+      __threadfence_block();
+      if (atomicAdd(&sArrive[l], bodies) + bodies != sBodies[l]) break;
+      __threadfence_block();
+      node = parent;
+      const uint32_t kv = sKids[l];
+      bodies = sBodies[l];
       uint32_t have = 0, first[4];
       float4 cu[4], ca[4], cm[4];
-      float nw, nsize = 0.0f;
-      if (local) {
-        const uint32_t kv = sKids[l];
-        nw = sA[l].w;
-        if (kFull) nsize = sM[l].w;
-        bodies = sBodies[l];
-#pragma unroll
-        for (uint32_t q = 0; q < 4; ++q) {
-          const uint32_t k = l + 1u + ((kv >> (8 * q)) & 255u);
-          if (k >= l + 256u) continue; // 255: empty (a child is at most 255 on)
-          have |= 1u << q;
-          cu[q] = sUp[k];
-          ca[q] = sA[k];
-          if (kFull) cm[q] = sM[k];
-          first[q] = sStart[k];
-        }
-      } else {
-        const uint4 kv = __ldcg(&S.spanKids[slot]);
-        __stcg(&S.spanKids[slot], make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu));
-        nw = __ldcg(&S.tN[node].a).w;
-        if (kFull) nsize = __ldcg(&S.tM[node]).w;
-        const int4 B = __ldcg(&S.tN[node].b);
-        bodies = (uint32_t)(B.w - B.z);
-        const uint32_t r[4] = {kv.x, kv.y, kv.z, kv.w};
-#pragma unroll
-        for (uint32_t q = 0; q < 4; ++q) {
-          if (r[q] >= total) continue; // all ones: no such child
-          have |= 1u << q;
-          cu[q] = __ldcg(&S.tUp[r[q]]);
-          ca[q] = __ldcg(&S.tN[r[q]].a);
-          if (kFull) cm[q] = __ldcg(&S.tM[r[q]]);
-          first[q] = (uint32_t)__ldcg(&S.tN[r[q]].b).z;
-        }
-      }
-      // sums in digit order (sumNode), then finishNode's divide
-      float sx = 0.0f, sy = 0.0f, sm = 0.0f, wBot = 0.0f;
-      uint32_t count = 0, link = 0, second = 0;
 #pragma unroll
       for (uint32_t q = 0; q < 4; ++q) {
-        if (!((have >> q) & 1u)) continue;
-        sx = count == 0 ? cu[q].x : __fadd_rn(sx, cu[q].x);
-        sy = count == 0 ? cu[q].y : __fadd_rn(sy, cu[q].y);
-        sm = count == 0 ? ca[q].z : __fadd_rn(sm, ca[q].z);
-        // one child: the same bodies under a smaller square, its record goes up
-        if (count == 0) {
-          wBot = cu[q].z;
-          link = __float_as_uint(cu[q].w);
-        }
-        if (count == 1) second = first[q];
-        ++count;
+        const uint32_t k = l + 1u + ((kv >> (8 * q)) & 255u);
+        if (k >= l + 256u) continue; // 255: empty (a child is at most 255 on)
+        have |= 1u << q;
+        cu[q] = sUp[k];
+        ca[q] = sA[k];
+        if (kFull) cm[q] = sM[k];
+        first[q] = sStart[k];
       }
-      const float dv = fmaxf(sm, FLT_MIN);
-      const float X = __fdiv_rn(sx, dv), Y = __fdiv_rn(sy, dv);
-      if (kFull) {
-        float jxx = 0.0f, jyy = 0.0f, jxy = 0.0f;
-#pragma unroll
-        for (uint32_t q = 0; q < 4; ++q) {
-          if (!((have >> q) & 1u)) continue;
-          const float dx = ca[q].x - X, dy = ca[q].y - Y;
-          jxx += cm[q].x + ca[q].z * dx * dx;
-          jyy += cm[q].y + ca[q].z * dy * dy;
-          jxy += cm[q].z + ca[q].z * dx * dy;
-        }
-        mom = make_float4(jxx, jyy, jxy, nsize);
-      }
-      if (count > 1) { // a node summed in the block: its thread writes the record
-        wBot = nw;
-        link = local ? second : quad_record<kFull>(S, second, X, Y, have, cu, ca, cm, first);
-      }
-      up = make_float4(sx, sy, wBot, __uint_as_float(link));
-      own = make_float4(X, Y, sm, nw);
+      sum_children<kFull>(S, have, cu, ca, cm, first, sA[l].w, kFull ? sM[l].w : 0.0f, false, up,
+                          own, mom);
     }
     __syncthreads();
     if (t < held && !spans) { // the nodes summed in the block, a thread to each
@@ -939,6 +915,80 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
       if (count > 1) quad_record<kFull>(S, second, a.x, a.y, have, cu, ca, cm, first);
     }
     __syncthreads();
+  }
+}
+
+// Sums the spanning nodes of k_trav_tree, a thread to each whose children all
+// lay in blocks, climbing from there: a child brought to its parent here adds
+// its bodies to a second counter, and the one that completes the count of the
+// first is the last.  Leaves the nodes' slots empty for the next build.
+// ~10 nodes a block of records; bound by the chain of arrivals (release,
+// atomic, two rounds of loads a level).
+template <bool kFull>
+__global__ void __launch_bounds__(kBlock) k_trav_top(DevState S) {
+  chain_begin();
+  const uint32_t total = S.counters[6];
+  if (total > S.nodeCapacity) return;
+  const uint32_t n = S.counters[kCtrSpans];
+  for (uint32_t k = blockIdx.x * kBlock + threadIdx.x; k < n; k += gridDim.x * kBlock) {
+    const uint2 entry = S.spanList[k];
+    uint32_t node = entry.x;
+    int d = (int)entry.y;
+    uint32_t slot = span_slot(node, d);
+    const int4 B = S.tN[node].b;
+    uint32_t bodies = (uint32_t)(B.w - B.z);
+    // a node with spanning children never shows its full count here
+    if (__ldcg(&S.spanArrive[slot]) != bodies) continue;
+    const uint64_t ci = S.sortedCodes[B.z];
+    for (int guard = 0; guard <= kMaxDepth; ++guard) {
+      const uint4 kv = __ldcg(&S.spanKids[slot]);
+      const float w = __ldcg(&S.tN[node].a).w;
+      const float size = kFull ? __ldcg(&S.tM[node]).w : 0.0f;
+      const uint32_t parent = d > 0 ? S.spanParent[slot] : 0u;
+      __stcg(&S.spanKids[slot], make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu));
+      __stcg(&S.spanArrive[slot], 0u);
+      __stcg(&S.spanArriveTop[slot], 0u);
+      const uint32_t r[4] = {kv.x, kv.y, kv.z, kv.w};
+      uint32_t have = 0, first[4];
+      float4 cu[4], ca[4], cm[4], up, own, mom;
+#pragma unroll
+      for (uint32_t q = 0; q < 4; ++q) {
+        if (r[q] >= total) continue; // all ones: no such child
+        have |= 1u << q;
+        cu[q] = __ldcg(&S.tUp[r[q]]);
+        ca[q] = __ldcg(&S.tN[r[q]].a);
+        if (kFull) cm[q] = __ldcg(&S.tM[r[q]]);
+        first[q] = (uint32_t)S.tN[r[q]].b.z;
+      }
+      sum_children<kFull>(S, have, cu, ca, cm, first, w, size, true, up, own, mom);
+      __stcg(&S.tN[node].a, own);
+      if (kFull) __stcg(&S.tM[node], mom);
+      if (d == 0) {
+        quad_root<kFull>(S, S.segOf[B.z], up, own, mom);
+        break;
+      }
+      if (parent >= total) {
+        atomicOr(S.status, kStatusTreeCapacity);
+        break;
+      }
+      --d;
+      slot = span_slot(parent, d);
+      const int4 pb = S.tN[parent].b;
+      __stcg(&S.tUp[node], up);
+      __stcg(reinterpret_cast<uint32_t *>(&S.spanKids[slot]) + digit_at(ci, d), node);
+      // release: the child's sums are visible to the last arriver; acquire: the
+      // last arriver sees every child's
+      uint32_t old;
+      asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
+                   : "=r"(old)
+                   : "l"(&S.spanArriveTop[slot]), "r"(bodies)
+                   : "memory");
+      // (a first count that the last arriver has already emptied reads 0, which
+      // cannot complete it either)
+      if (old + bodies + __ldcg(&S.spanArrive[slot]) != (uint32_t)(pb.w - pb.z)) break;
+      node = parent;
+      bodies = (uint32_t)(pb.w - pb.z);
+    }
   }
 }
 
@@ -1007,10 +1057,13 @@ void launch_trav_tree(cudaStream_t s, const DevState &S, ScanScratch &scan, bool
   exclusive_scan_u32(s, S.splitCount, S.splitStart, n, nullptr, &S.counters[6],
                      scan, S.status, owner, S.nodeCapacity, 3);
   mark(s, "tree.counts");
-  if (moments)
+  if (moments) {
     launch_after(s, k_trav_tree<true>, grid_for(n / 4 + 64), kBlock, 0, S, owner);
-  else
+    launch_after(s, k_trav_top<true>, grid_for(n / 64 + 64), kBlock, 0, S);
+  } else {
     launch_after(s, k_trav_tree<false>, grid_for(n / 4 + 64), kBlock, 0, S, owner);
+    launch_after(s, k_trav_top<false>, grid_for(n / 64 + 64), kBlock, 0, S);
+  }
   mark(s, "tree.records");
 }
 

@@ -791,12 +791,12 @@ __global__ void __launch_bounds__(kBlock) k_zero_ranges(ZeroRanges z) {
 } // namespace
 
 // What a step's phases expect cleared, in one launch: the collision
-// counters (units, unit claims, small-large pairs, long runs of both
-// sorts), both sorts' digit rows, tile counters and look-back words (the
-// Morton sort in slots 0-3, the units' in 4-6) and the four scan slots
-// (grid buckets, large lists, partner lists, traversal records); with
-// grid, also the collision grid's bucket and large counts (a step or phase
-// that collides).
+// counters (units, unit claims, small-large pairs), the counts of long runs
+// of both sorts and of the traversal layout's spanning nodes, both sorts'
+// digit rows, tile counters and look-back words (the Morton sort in slots
+// 0-3, the units' in 4-6) and the four scan slots (grid buckets, large lists,
+// partner lists, traversal records); with grid, also the collision grid's
+// bucket and large counts (a step or phase that collides).
 void launch_step_zero(cudaStream_t s, const DevState &S, ScanScratch &scan, SortScratch &sort,
                       bool grid) {
   ZeroRanges z{};
@@ -811,7 +811,7 @@ void launch_step_zero(cudaStream_t s, const DevState &S, ScanScratch &scan, Sort
   }
   add(S.counters + 1, 2); // units, unit claims
   add(S.counters + 5, 1); // small-large pairs
-  add(S.counters + 9, 2); // long runs of the Morton and the units' sorts
+  add(S.counters + 9, 3); // long runs of the Morton and the units' sorts, spanning nodes
   add(sort.hist, 7 * 256);
   add(sort.tileCounter, 8);
   const uint32_t statusWords = 7 * (uint32_t)sort_pass_words(S.n);

@@ -73,6 +73,7 @@ constexpr int kLevelSlots = 34; // depths 0..32 plus an end slot
 // (float bits), and each build marks the instances whose bodies reach
 // beyond it (SegDev::wide), for the force pass to keep the clamp there.
 constexpr int kCtrCoordLimit = 15;
+constexpr int kCtrSpans = 11; // spanning nodes of the build (DevState::spanList)
 constexpr int kCtrBoundsDone = 7; // blocks of the bounds pass done (self-resetting)
 
 // Everything a step's kernels touch.  All pointers are device pointers.
@@ -139,6 +140,7 @@ struct DevState {
                          // [5]=small-large pairs [6]=traversal records
                          // [8]=id check
                          // [9]=long Morton runs [12]=upload mass bits
+                         // [kCtrSpans] (above)
                          // [7]=bounds blocks done [10]=long unit runs
                          // [13]=expiry test flag [kCtrCoordLimit] (above)
 
@@ -163,9 +165,11 @@ struct DevState {
   uint32_t *subtree;    // nodes in subtree
   uint32_t *arrive;     // bottom-up arrival counters
   // nodes of the traversal layout that reach beyond their block of the build
-  // (k_trav_tree), by (block, depth): parent record, and between builds
-  // empty: the children's records by digit, the arrival counter
-  uint32_t *spanParent, *spanArrive;
+  // (k_trav_tree): their {record, depth}, and by (block, depth) the parent
+  // record and, empty between builds, the bodies of the children summed in
+  // blocks and of those summed at the top, and the children's records by digit
+  uint2 *spanList;
+  uint32_t *spanParent, *spanArrive, *spanArriveTop;
   uint4 *spanKids;
   // traversal layout (preorder)
   TravNode *tN; // preorder traversal records (32 bytes, one load each)
