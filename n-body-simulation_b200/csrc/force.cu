@@ -7,10 +7,11 @@
 // a leaf's bodies one by one, otherwise descend.
 //
 // The default force pass walks the tree once per group of 32 bodies over
-// records of four children (walk_group).  Exact arithmetic, the clamped law,
-// the corrected forms, queries and counting keep a cursor per lane
-// (walk_targets), so that a body's terms are summed in the reference's
-// order: along a lane's walk of the depth-first preorder layout (build.cu)
+// records of four children (walk_group), and so do queries, and exact
+// arithmetic and the quadrupole term of few bodies.  Many of those, the
+// learned correction (walk_learned), the clamped law, counting and whatever
+// does not fit a group's scratch keep a cursor per lane (walk_targets), so that
+// a body's terms are summed in the reference's order: along a lane's walk of the depth-first preorder layout (build.cu)
 // the position only increases (descend = +1, skip = +subtree size), so the
 // warp always serves the smallest position any lane is waiting at.  The
 // node's record is read once per warp (one broadcast load through L1;
@@ -130,14 +131,12 @@ __device__ __forceinline__ void quad_term(float dx, float dy, float dSq,
 
 // One warp's walk: lane targets (x, y) start at node cur (kDone: none) and
 // add their terms to (ax, ay); kCount adds the walk's counts instead.
-// kCorr = 1: accepted cells with size^2 >= d^2 * band^2 get the learned
-// correction (mlp.cuh), evaluated for the warp's rows on tensor cores;
-// kCorr = 2: they get the analytic quadrupole term instead (the control).
+// kCorr = 2: accepted cells with size^2 >= d^2 * band^2 get the analytic
+// quadrupole term (the control of the learned correction, walk_learned).
 template <bool kExact, bool kCount, int kCorr, bool kClamp>
 __device__ __forceinline__ void walk_targets(
-    const DevState &S, float tSq, float eSq, float bandSq, float eps, float x, float y,
-    uint32_t cur, float4 *sBodyW, const MlpDev *sW, __nv_bfloat16 (*sStageW)[16],
-    float &ax, float &ay, uint32_t &nFar, uint32_t &nNear, uint32_t &nVisit,
+    const DevState &S, float tSq, float eSq, float bandSq, float x, float y, uint32_t cur,
+    float4 *sBodyW, float &ax, float &ay, uint32_t &nFar, uint32_t &nNear, uint32_t &nVisit,
     uint32_t &nIter, uint32_t &nChunk) {
   const int lane = threadIdx.x & 31;
   for (;;) {
@@ -185,26 +184,6 @@ __device__ __forceinline__ void walk_targets(
           }
         }
       }
-      if (kCorr == 1) {
-        const bool band = use && A.w >= dSq * bandSq;
-        if (__ballot_sync(0xffffffffu, band)) {
-          const float4 M = S.tM[k];
-          const float2 Q = S.tC[k];
-          float f[9], ux = 0.0f, uy = 0.0f;
-          bool ok = band && mlp_features(dx, dy, dSq, A.z, M.w, Q.x, Q.y, A.x,
-                                         A.y, M.x, M.y, M.z, 1.0f, eps, f, ux, uy);
-          if (!ok)
-            for (int q = 0; q < 9; ++q) f[q] = 0.0f;
-          float o0, o1;
-          mlp_warp(*sW, f, sStageW, o0, o1);
-          if (ok) {
-            // |mono| * ((1 + t0) u + t1 w), w = (-uy, ux)
-            const float r = dSq * rsqrtf(dSq);
-            tx = ax + fac * (dx * (1.0f + o0) - r * o1 * uy);
-            ty = ay + fac * (dy * (1.0f + o0) + r * o1 * ux);
-          }
-        }
-      }
       ax = use ? tx : ax;
       ay = use ? ty : ay;
       if (kCount) nFar += use ? 1u : 0u;
@@ -236,6 +215,125 @@ __device__ __forceinline__ void walk_targets(
       }
       if (kCount && openLeaf) nNear += bEnd > b0 ? bEnd - b0 : 0u;
     }
+  }
+}
+
+// One warp's walk with the learned correction (mlp.cuh) of the accepted
+// cells with size^2 >= d^2 * band^2, in rounds: the warp walks on (a cursor per
+// lane, as walk_targets) and lists the nodes that give some lane a term, and
+// the (node, lane) rows that want the network; then evaluates 32 rows at a
+// time on the tensor cores; then adds the round's terms in the list's order,
+// so every lane's sum is that of evaluating each node's rows on the spot.
+// There a call of the network (~400 instructions) holds only the few
+// lanes that are at the node: 100,000 bodies of a disc, theta 0.7, band 0.5,
+// 412 us; in rounds 221, of which the warps issue for half, with the longest
+// walks (one wave of warps) the rest.
+constexpr uint32_t kLearnedNodes = 96, kLearnedRows = 224;
+struct LearnedStage {
+  uint4 node[kLearnedNodes]; // record, lanes that add it, correct it, open it
+  float2 term[kLearnedRows]; // a row's corrected direction, to be scaled by the law's factor
+  union {
+    __nv_bfloat16 feat[32][16]; // while evaluating
+    float4 body[32];            // while adding: a leaf's bodies
+  };
+  uint16_t row[kLearnedRows]; // node << 5 | lane
+};
+static_assert(kLearnedNodes << 5 <= 65536u, "a row fits 16 bits");
+
+__device__ __forceinline__ void walk_learned(const DevState &S, float tSq, float eSq,
+                                             float bandSq, float eps, float x, float y,
+                                             uint32_t cur, LearnedStage &st, const MlpDev &sW,
+                                             float &ax, float &ay) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t below = (1u << lane) - 1u;
+  for (bool more = true; more;) {
+    uint32_t nodes = 0, rows = 0;
+    while (nodes < kLearnedNodes && rows + 32u <= kLearnedRows) {
+      const uint32_t k = __reduce_min_sync(0xffffffffu, cur);
+      if (k == kDone) {
+        more = false;
+        break;
+      }
+      float4 A;
+      int4 B;
+      ld_node(&S.tN[k], A, B);
+      const bool at = cur == k;
+      const float dx = A.x - x, dy = A.y - y;
+      const float dSq = sq_dist<false>(dx, dy);
+      const bool accept = at && A.w < dSq * tSq;
+      const bool use = accept && A.z > 0.0f;
+      const bool band = use && A.w >= dSq * bandSq;
+      cur = at ? (accept ? (uint32_t)B.x : (uint32_t)B.y) : cur;
+      const uint32_t adds = __ballot_sync(0xffffffffu, use);
+      const uint32_t opens = __ballot_sync(0xffffffffu, at && !accept && B.y == B.x);
+      if ((adds | opens) == 0u) continue;
+      const uint32_t corrects = __ballot_sync(0xffffffffu, band);
+      if (band) st.row[rows + __popc(corrects & below)] = (uint16_t)(nodes << 5 | lane);
+      if (lane == 0) st.node[nodes] = make_uint4(k, adds, corrects, opens);
+      rows += __popc(corrects);
+      ++nodes;
+    }
+    __syncwarp();
+    for (uint32_t r = 0; r < rows; r += 32) {
+      const bool on = r + lane < rows;
+      const uint32_t row = st.row[on ? r + lane : r];
+      const float px = __shfl_sync(0xffffffffu, x, row & 31u);
+      const float py = __shfl_sync(0xffffffffu, y, row & 31u);
+      const uint32_t k = st.node[row >> 5].x;
+      const float4 A = S.tN[k].a, M = S.tM[k];
+      const float2 Q = S.tC[k];
+      const float dx = A.x - px, dy = A.y - py;
+      const float dSq = sq_dist<false>(dx, dy);
+      float f[9], ux = 0.0f, uy = 0.0f;
+      const bool ok = on && mlp_features(dx, dy, dSq, A.z, M.w, Q.x, Q.y, A.x, A.y, M.x, M.y,
+                                         M.z, 1.0f, eps, f, ux, uy);
+      if (!ok)
+        for (int q = 0; q < 9; ++q) f[q] = 0.0f;
+      float o0, o1;
+      mlp_warp(sW, f, st.feat, o0, o1);
+      float2 term = make_float2(dx, dy);
+      if (ok) {
+        // |mono| * ((1 + t0) u + t1 w), w = (-uy, ux)
+        const float d = dSq * rsqrtf(dSq);
+        term = make_float2(dx * (1.0f + o0) - d * o1 * uy, dy * (1.0f + o0) + d * o1 * ux);
+      }
+      if (on) st.term[r + lane] = term;
+    }
+    __syncwarp();
+    rows = 0;
+    for (uint32_t e = 0; e < nodes; ++e) {
+      const uint4 N = st.node[e];
+      float4 A;
+      int4 B;
+      ld_node(&S.tN[N.x], A, B);
+      const float dx = A.x - x, dy = A.y - y;
+      const float fac = law_factor<false, true>(sq_dist<false>(dx, dy), A.z, eSq);
+      float2 term = make_float2(dx, dy);
+      if ((N.z >> lane) & 1u) term = st.term[rows + __popc(N.z & below)];
+      rows += __popc(N.z);
+      const bool use = (N.y >> lane) & 1u, open = (N.w >> lane) & 1u;
+      ax = use ? fmaf(term.x, fac, ax) : ax;
+      ay = use ? fmaf(term.y, fac, ay) : ay;
+      if (N.w == 0u) continue;
+      const uint32_t b0 = (uint32_t)B.z, b1 = (uint32_t)B.w;
+      const uint32_t bEnd = b1 <= S.n ? b1 : S.n; // defensive bound
+      for (uint32_t base = b0; base < bEnd; base += 32) {
+        const uint32_t cnt = min(32u, bEnd - base);
+        __syncwarp();
+        if ((uint32_t)lane < cnt) st.body[lane] = S.xym[base + lane];
+        __syncwarp();
+#pragma unroll 4
+        for (uint32_t j = 0; j < cnt; ++j) {
+          const float4 q = st.body[j];
+          const float ex = q.x - x, ey = q.y - y;
+          float tx = ax, ty = ay;
+          add_term<false, true>(ex, ey, sq_dist<false>(ex, ey), q.z, eSq, tx, ty);
+          ax = open ? tx : ax;
+          ay = open ? ty : ay;
+        }
+      }
+    }
+    __syncwarp();
   }
 }
 
@@ -921,9 +1019,8 @@ __device__ __forceinline__ void store_acc(const DevState &S, uint32_t i, float x
 template <bool kExact, bool kCount, int kCorr, bool kClamp, bool kPairs>
 __device__ __forceinline__ void forces_walk(
     const DevState &S, float tSq, float eSq, unsigned long long *counts,
-    float bandSq, float eps, const float2 *__restrict__ query, uint32_t nQuery,
-    float2 *__restrict__ queryAcc, float4 (*sBody)[32], const MlpDev &sW,
-    __nv_bfloat16 (*sStage)[32][16]) {
+    float bandSq, const float2 *__restrict__ query, uint32_t nQuery,
+    float2 *__restrict__ queryAcc, float4 (*sBody)[32]) {
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   const uint32_t warpsTotal = (gridDim.x * blockDim.x) >> 5;
@@ -959,16 +1056,14 @@ __device__ __forceinline__ void forces_walk(
     constexpr bool kPlainX2 = kPairs && !kExact && !kCount && kCorr == 0 && !kClamp;
     const bool anyWide = !kClamp && __any_sync(0xffffffffu, wide);
     if (anyWide)
-      walk_targets<kExact, kCount, kCorr, true>(S, tSq, eSq, bandSq, eps, x, y, cur,
-                                                sBody[w], &sW, sStage[kCorr == 1 ? w : 0],
-                                                ax, ay, nFar, nNear, nVisit, nIter, nChunk);
+      walk_targets<kExact, kCount, kCorr, true>(S, tSq, eSq, bandSq, x, y, cur, sBody[w], ax,
+                                                ay, nFar, nNear, nVisit, nIter, nChunk);
     else if (kPlainX2) {
       float *sX = reinterpret_cast<float *>(sBody[w]);
       walk_plain_x2(S, tSq, eSq, x, y, cur, sX, sX + 32, sX + 64, ax, ay);
     } else
-      walk_targets<kExact, kCount, kCorr, kClamp>(S, tSq, eSq, bandSq, eps, x, y, cur,
-                                                  sBody[w], &sW, sStage[kCorr == 1 ? w : 0],
-                                                  ax, ay, nFar, nNear, nVisit, nIter, nChunk);
+      walk_targets<kExact, kCount, kCorr, kClamp>(S, tSq, eSq, bandSq, x, y, cur, sBody[w], ax,
+                                                  ay, nFar, nNear, nVisit, nIter, nChunk);
     if (kCount) {
       unsigned long long f = nFar, nn = nNear, v = nVisit;
       for (int o = 16; o > 0; o >>= 1) {
@@ -999,36 +1094,58 @@ __device__ __forceinline__ void forces_walk(
 // stored at upload (the build's SegDev::wide), where distances could
 // overflow, takes the clamped walk instead.  Launch bounds: a full SM of
 // kBlock-thread blocks (2048 threads: at most 32 registers) for every walk
-// but the learned correction's, whose MMA fragments keep it at 3 blocks of
-// 256, and the paired plain walk's: 1536 threads per SM (40 registers),
+// but the paired plain walk's: 1536 threads per SM (40 registers),
 // 1% faster than 2048 at 32 registers and identical in results.  kBlock
 // and kPairs vary only for the default plain walk (the autotuner's block
 // shape and leaf width).
 template <bool kExact, bool kCount = false, int kCorr = 0, bool kClamp = true,
           int kBlock = kForceBlock, bool kPairs = true>
-__global__ void __launch_bounds__(kBlock, kCorr == 1 ? 3
-                                          : (kPairs && !kExact && !kCount && kCorr == 0 &&
-                                                     !kClamp
-                                                 ? 1536 / kBlock
-                                                 : 2048 / kBlock))
+__global__ void __launch_bounds__(kBlock, kPairs && !kExact && !kCount && kCorr == 0 && !kClamp
+                                              ? 1536 / kBlock
+                                              : 2048 / kBlock)
     k_forces(DevState S, float tSq, float eSq,
-             unsigned long long *counts = nullptr,
-             const MlpDev *__restrict__ mlp = nullptr, float bandSq = 0.0f,
-             float eps = 0.0f, const float2 *__restrict__ query = nullptr,
-             uint32_t nQuery = 0, float2 *__restrict__ queryAcc = nullptr) {
+             unsigned long long *counts = nullptr, float bandSq = 0.0f,
+             const float2 *__restrict__ query = nullptr, uint32_t nQuery = 0,
+             float2 *__restrict__ queryAcc = nullptr) {
   chain_begin();
-  constexpr int kBlockWarps = kBlock / 32;
-  constexpr int kStage = kCorr == 1 ? kBlockWarps : 1;
-  __shared__ float4 sBody[kBlockWarps][32];
+  __shared__ float4 sBody[kBlock / 32][32];
+  forces_walk<kExact, kCount, kCorr, kClamp, kPairs>(S, tSq, eSq, counts, bandSq, query, nQuery,
+                                                     queryAcc, sBody);
+}
+
+// The force pass with the learned correction, one warp per 32 bodies.  us by
+// threads a block at 100,000 bodies (fewer repeat the weights in shared memory,
+// more wait for a block's longest walk): 32 264, 64 235, 128 221, 192 226,
+// 256 236.
+constexpr int kLearnedBlock = 128;
+__global__ void __launch_bounds__(kLearnedBlock, 768 / kLearnedBlock)
+    k_forces_learned(DevState S, float tSq, float eSq, const MlpDev *__restrict__ mlp,
+                     float bandSq, float eps) {
+  chain_begin();
+  __shared__ LearnedStage sStage[kLearnedBlock / 32];
   __shared__ MlpDev sW;
-  __shared__ __nv_bfloat16 sStage[kStage][32][16];
-  if (kCorr == 1) {
-    for (int q = threadIdx.x; q < (int)(sizeof(MlpDev) / 4); q += blockDim.x)
-      reinterpret_cast<uint32_t *>(&sW)[q] = reinterpret_cast<const uint32_t *>(mlp)[q];
-    __syncthreads();
+  for (int q = threadIdx.x; q < (int)(sizeof(MlpDev) / 4); q += blockDim.x)
+    reinterpret_cast<uint32_t *>(&sW)[q] = reinterpret_cast<const uint32_t *>(mlp)[q];
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const uint32_t end = S.forceEnd ? min(S.forceEnd, S.n) : S.n;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t wb = S.forceBegin + ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u); wb < end;
+       wb += stride) {
+    const uint32_t i = wb + lane;
+    const bool valid = i < end;
+    float x = 0.0f, y = 0.0f, ax = 0.0f, ay = 0.0f;
+    uint32_t cur = kDone;
+    if (valid) {
+      const float4 b = S.xym[i];
+      x = b.x;
+      y = b.y;
+      const SegDev &G = S.seg[S.segOf[i]];
+      if (G.travCount > 0) cur = G.travBase;
+    }
+    walk_learned(S, tSq, eSq, bandSq, eps, x, y, cur, sStage[threadIdx.x >> 5], sW, ax, ay);
+    if (valid) store_acc<false>(S, i, x, y, ax, ay);
   }
-  forces_walk<kExact, kCount, kCorr, kClamp, kPairs>(S, tSq, eSq, counts, bandSq, eps, query,
-                                                     nQuery, queryAcc, sBody, sW, sStage);
 }
 
 // Sums of a group walk for the targets of `lanes` (places (x, y), a valid
@@ -1037,8 +1154,8 @@ __global__ void __launch_bounds__(kBlock, kCorr == 1 ? 3
 // the clamped one (exact arithmetic always clamps), as in k_forces.
 template <GroupWalk kWalk>
 __device__ __forceinline__ void group_forces(const DevState &S, float tSq, float eSq,
-                                             float bandSq, float eps, float x, float y,
-                                             uint32_t sg, uint32_t lanes, WalkStage &st,
+                                             float bandSq, float x, float y, uint32_t sg,
+                                             uint32_t lanes, WalkStage &st,
                                              float &ax, float &ay) {
   constexpr bool kExact = kWalk == kExactWalk;
   constexpr int kCorr = kWalk == kQuadWalk ? 2 : 0;
@@ -1049,9 +1166,9 @@ __device__ __forceinline__ void group_forces(const DevState &S, float tSq, float
   static_assert(sizeof(WalkStage) >= 32 * sizeof(float4), "holds a leaf's staged bodies");
   uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
   if (G.wide) {
-    walk_targets<kExact, false, kCorr, true>(S, tSq, eSq, bandSq, eps, x, y,
+    walk_targets<kExact, false, kCorr, true>(S, tSq, eSq, bandSq, x, y,
                                              (lanes >> lane) & 1u ? G.travBase : kDone, staged,
-                                             nullptr, nullptr, ax, ay, c0, c1, c2, c3, c4);
+                                             ax, ay, c0, c1, c2, c3, c4);
     return;
   }
   // A group whose walk does not fit goes in two at the widest step along its
@@ -1083,8 +1200,8 @@ __device__ __forceinline__ void group_forces(const DevState &S, float tSq, float
         float *sX = reinterpret_cast<float *>(staged);
         walk_plain_x2(S, tSq, eSq, x, y, root, sX, sX + 32, sX + 64, wx, wy);
       } else {
-        walk_targets<kExact, false, kCorr, kExact>(S, tSq, eSq, bandSq, eps, x, y, root, staged,
-                                                   nullptr, nullptr, wx, wy, c0, c1, c2, c3, c4);
+        walk_targets<kExact, false, kCorr, kExact>(S, tSq, eSq, bandSq, x, y, root, staged, wx,
+                                                   wy, c0, c1, c2, c3, c4);
       }
       if (in) {
         ax = wx;
@@ -1102,7 +1219,7 @@ constexpr int kGroupWarpsPerSM = 20;
 template <int kBlock, GroupWalk kWalk>
 __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
                                               ? kGroupWarpsPerSM * 32 / kBlock : 1)
-    k_forces_groups(DevState S, float tSq, float eSq, float bandSq, float eps) {
+    k_forces_groups(DevState S, float tSq, float eSq, float bandSq) {
   chain_begin();
   extern __shared__ uint4 sDyn[]; // a WalkStage per warp
   const int lane = threadIdx.x & 31;
@@ -1119,7 +1236,7 @@ __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
     const uint32_t i = mine ? first + lane : first;
     const float4 b = S.xym[i];
     float ax = 0.0f, ay = 0.0f;
-    group_forces<kWalk>(S, tSq, eSq, bandSq, eps, b.x, b.y, sg,
+    group_forces<kWalk>(S, tSq, eSq, bandSq, b.x, b.y, sg,
                         __ballot_sync(0xffffffffu, mine), st, ax, ay);
     if (mine) store_acc<kWalk == kExactWalk>(S, i, b.x, b.y, ax, ay);
     __syncwarp();
@@ -1144,7 +1261,7 @@ __global__ void __launch_bounds__(kQueryBlock, kGroupWarpsPerSM * 32 / kQueryBlo
   const uint32_t i = (uint32_t)first + (mine ? lane : 0);
   const float2 q = query[i];
   float ax = 0.0f, ay = 0.0f;
-  group_forces<kWalk>(S, tSq, eSq, 0.0f, 0.0f, q.x, q.y, 0u, __ballot_sync(0xffffffffu, mine),
+  group_forces<kWalk>(S, tSq, eSq, 0.0f, q.x, q.y, 0u, __ballot_sync(0xffffffffu, mine),
                       st, ax, ay);
   if (mine) queryAcc[i] = make_float2(ax, ay);
 }
@@ -1272,10 +1389,9 @@ void launch_groups(cudaStream_t s, const DevState &S, int blocks, float band, bo
   }
   if (chained)
     launch_after(s, k_forces_groups<kBlock, kWalk>, blocks, kBlock, smem, S, S.tSq, S.eSq,
-                 band * band, sqrtf(S.eSq));
+                 band * band);
   else
-    k_forces_groups<kBlock, kWalk>
-        <<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq, band * band, sqrtf(S.eSq));
+    k_forces_groups<kBlock, kWalk><<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq, band * band);
 }
 
 // The default plain walk with kBlock threads per block and the paired or
@@ -1339,11 +1455,9 @@ void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool gro
   } else {
     const uint32_t b = ((nq + 31) / 32 + kWarps - 1) / kWarps;
     if (exact)
-      k_forces<true><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, nullptr, 0.0f, 0.0f,
-                                               query, nq, out);
+      k_forces<true><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, 0.0f, query, nq, out);
     else
-      k_forces<false><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, nullptr, 0.0f, 0.0f,
-                                                query, nq, out);
+      k_forces<false><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, 0.0f, query, nq, out);
   }
   if (order) k_query_scatter<<<blocks, 256, 0, s>>>(accSorted, vals, nq, acc);
 }
@@ -1379,20 +1493,24 @@ void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
       return;
     }
   }
-  if (blocks <= 0) {
-    uint32_t warps = (force_targets(S) + 31) / 32;
-    uint32_t b = (warps + kWarps - 1) / kWarps;
-    blocks = (int)(b ? b : 1);
+  const uint32_t warps = (force_targets(S) + 31) / 32;
+  if (corr == 1 && mlp) {
+    constexpr uint32_t per = kLearnedBlock / 32;
+    const int grid = blocks > 0 ? blocks : (int)std::max(1u, (warps + per - 1) / per);
+    if (chained)
+      launch_after(s, k_forces_learned, grid, kLearnedBlock, 0, S, S.tSq, S.eSq, mlp,
+                   band * band, sqrtf(S.eSq));
+    else
+      k_forces_learned<<<grid, kLearnedBlock, 0, s>>>(S, S.tSq, S.eSq, mlp, band * band,
+                                                      sqrtf(S.eSq));
+    return;
   }
-  if (corr == 1 && mlp)
-    k_forces<false, false, 1><<<blocks, kForceBlock, 0, s>>>(
-        S, S.tSq, S.eSq, nullptr, mlp, band * band, sqrtf(S.eSq));
-  else if (corr == 2 && noClamp)
-    k_forces<false, false, 2, false><<<blocks, kForceBlock, 0, s>>>(
-        S, S.tSq, S.eSq, nullptr, nullptr, band * band, sqrtf(S.eSq));
+  if (blocks <= 0) blocks = (int)std::max(1u, (warps + kWarps - 1) / kWarps);
+  if (corr == 2 && noClamp)
+    k_forces<false, false, 2, false>
+        <<<blocks, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, band * band);
   else if (corr == 2)
-    k_forces<false, false, 2><<<blocks, kForceBlock, 0, s>>>(
-        S, S.tSq, S.eSq, nullptr, nullptr, band * band, sqrtf(S.eSq));
+    k_forces<false, false, 2><<<blocks, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, band * band);
   else if (exact)
     k_forces<true><<<blocks, kForceBlock, 0, s>>>(S, S.tSq, S.eSq);
   else

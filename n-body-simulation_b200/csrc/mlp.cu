@@ -313,7 +313,7 @@ __global__ void k_mlp_eval_simt(const float *__restrict__ feat, uint32_t n,
 __global__ void k_mlp_eval_mma(const float *__restrict__ feat, uint32_t n,
                                const MlpDev *__restrict__ Wg, float *out) {
   __shared__ MlpDev W;
-  __shared__ __nv_bfloat16 stage[kBlock / 32][32][16];
+  __shared__ __align__(16) __nv_bfloat16 stage[kBlock / 32][32][16];
   for (int i = threadIdx.x; i < (int)(sizeof(MlpDev) / 4); i += blockDim.x)
     reinterpret_cast<uint32_t *>(&W)[i] = reinterpret_cast<const uint32_t *>(Wg)[i];
   __syncthreads();

@@ -106,14 +106,12 @@ __device__ __forceinline__ void mlp_warp(const MlpDev &W, const float feat[9],
                                          float &o1) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  // stage the input rows so each lane can read its A fragments
-  uint32_t *row = reinterpret_cast<uint32_t *>(stage[lane]);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const float lo = 2 * k < 9 ? feat[2 * k] : 0.0f;
-    const float hi = 2 * k + 1 < 9 ? feat[2 * k + 1] : 0.0f;
-    row[k] = pack_bf16(lo, hi);
-  }
+  // stage the input rows so each lane can read its A fragments (columns 9 to
+  // 15 are zero)
+  *reinterpret_cast<uint4 *>(stage[lane]) =
+      make_uint4(pack_bf16(feat[0], feat[1]), pack_bf16(feat[2], feat[3]),
+                 pack_bf16(feat[4], feat[5]), pack_bf16(feat[6], feat[7]));
+  *reinterpret_cast<uint32_t *>(&stage[lane][8]) = pack_bf16(feat[8], 0.0f);
   __syncwarp();
   uint32_t a[2][4];
 #pragma unroll
@@ -122,8 +120,8 @@ __device__ __forceinline__ void mlp_warp(const MlpDev &W, const float feat[9],
     const uint32_t *r1 = reinterpret_cast<const uint32_t *>(stage[mt * 16 + g + 8]);
     a[mt][0] = r0[t];
     a[mt][1] = r1[t];
-    a[mt][2] = r0[t + 4];
-    a[mt][3] = r1[t + 4];
+    a[mt][2] = t == 0 ? r0[4] : 0u;
+    a[mt][3] = t == 0 ? r1[4] : 0u;
   }
   __syncwarp();
   // layer 1: [32 x 16] x [16 x 32]
