@@ -196,6 +196,7 @@ size_t scan_scratch_tiles(uint32_t n_max);
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 12;
 constexpr int kSortTile = kSortThreads * kSortItems; // 3072
+constexpr int kSortGroup = 16; // tiles whose counts are also published together
 constexpr int kSortWarps = kSortThreads / 32;
 
 struct SortScratch {

@@ -381,8 +381,7 @@ __global__ void __launch_bounds__(kSortThreads, 3)
       s_whist[w][d] = count;
       count += c;
     }
-    st_relaxed_u32(status + (size_t)tile * 256 + d,
-                   ((tile == 0 ? 2u : 1u) << kRFlagShift) | count);
+    st_relaxed_u32(status + (size_t)tile * 256 + d, (1u << kRFlagShift) | count);
   }
   // exclusive scans over digits (256 entries, one per thread) of the tile's
   // counts and of the pass's whole-array counts (the digit's global start)
@@ -423,21 +422,50 @@ __global__ void __launch_bounds__(kSortThreads, 3)
       s_vals[p] = val[k];
     }
   }
-  // look-back for digit d, with the items already out of registers
+  // look-back for digit d, with the items already out of registers: the tiles
+  // of this one's group of kSortGroup, then the groups before it by their last
+  // tiles' words.  The tiles of a wave publish nearly together, so walking
+  // over the tiles alone took a round trip per 2 x 16 of them before a whole
+  // prefix was met, in 342 tiles (2^20 keys) ten; a pass 19 us, so 17.  Groups of
+  // 8 or 24 tiles are no better.
   {
-    uint32_t excl = 0;
-    if (tile != 0) {
+    const int inGroup = (int)(tile % kSortGroup), group = (int)(tile / kSortGroup);
+    const bool last = inGroup == kSortGroup - 1;
+    uint32_t *groups = status + (size_t)((n_max + kSortTile - 1) / kSortTile) * 256;
+    uint32_t excl = 0, spins = 0;
+    for (;;) {
+      uint32_t sum = 0, all = 1u << kRFlagShift;
+#pragma unroll
+      for (int j = 1; j < kSortGroup; ++j) {
+        const uint32_t w = j <= inGroup ? ld_relaxed_u32(status + (size_t)(tile - j) * 256 + d)
+                                        : 1u << kRFlagShift;
+        all &= w;
+        sum += w & kRValueMask;
+      }
+      excl = sum;
+      if (all != 0) break;
+      if (++spins > kSpinLimit) {
+        atomicOr(err, kStatusSpinLimit);
+        break;
+      }
+      __nanosleep(32);
+    }
+    const uint32_t groupSum = excl + count; // of the last tile
+    if (last)
+      st_relaxed_u32(groups + (size_t)group * 256 + d,
+                     ((group == 0 ? 2u : 1u) << kRFlagShift) | groupSum);
+    if (group != 0) {
       // kLookBack predecessors per round trip (independent loads in
-      // flight); tile 0 is always inclusive, so the walk ends before it
-      // would read below tile 0
+      // flight); group 0 is always inclusive, so the walk ends before it
+      // would read below group 0
       constexpr int kLookBack = 16;
-      int pred = (int)tile - 1;
-      uint32_t spins = 0;
+      int pred = group - 1;
+      spins = 0;
       for (;;) {
         uint32_t w[kLookBack];
 #pragma unroll
         for (int j = 0; j < kLookBack; ++j)
-          w[j] = pred - j >= 0 ? ld_relaxed_u32(status + (size_t)(pred - j) * 256 + d)
+          w[j] = pred - j >= 0 ? ld_relaxed_u32(groups + (size_t)(pred - j) * 256 + d)
                                : (2u << kRFlagShift);
         int take = 0;
         bool done = false;
@@ -460,8 +488,9 @@ __global__ void __launch_bounds__(kSortThreads, 3)
           __nanosleep(32);
         }
       }
-      st_relaxed_u32(status + (size_t)tile * 256 + d,
-                     (2u << kRFlagShift) | ((excl + count) & kRValueMask));
+      if (last)
+        st_relaxed_u32(groups + (size_t)group * 256 + d,
+                       (2u << kRFlagShift) | ((excl + count) & kRValueMask));
     }
     s_global[d] = digitStart + excl;
   }
@@ -684,7 +713,8 @@ size_t sort_tiles(uint32_t n_max) {
 }
 
 size_t sort_pass_words(uint32_t n_max) {
-  return 256 * (size_t)((n_max + kSortTile - 1) / kSortTile + 1);
+  const size_t tiles = (n_max + kSortTile - 1) / kSortTile;
+  return 256 * (tiles + tiles / kSortGroup + 1); // a tile's row, a group's row
 }
 
 namespace {
