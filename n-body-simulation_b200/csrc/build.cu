@@ -574,14 +574,13 @@ __device__ __forceinline__ uint32_t search8(uint32_t lo, uint32_t hi, Before bef
 // (sumNode), then finishNode's divide: up = {weighted sums, bottom size^2,
 // link}, own = {centre of mass, mass, size^2}, mom = {moments, size}.  One
 // child has the same bodies under a smaller square: its link goes up.  With
-// more the link is the node's own record, at its second child's first body;
-// record: write that too.
+// more (true) the link is the node's own record, at its second child's first
+// body.
 template <bool kFull>
-__device__ __forceinline__ void sum_children(const DevState &S, uint32_t have,
-                                             const float4 (&cu)[4], const float4 (&ca)[4],
-                                             const float4 (&cm)[4], const uint32_t (&first)[4],
-                                             float w, float size, bool record, float4 &up,
-                                             float4 &own, float4 &mom) {
+__device__ __forceinline__ bool sum_children(uint32_t have, const float4 (&cu)[4],
+                                             const float4 (&ca)[4], const float4 (&cm)[4],
+                                             const uint32_t (&first)[4], float w, float size,
+                                             float4 &up, float4 &own, float4 &mom) {
   float sx = 0.0f, sy = 0.0f, sm = 0.0f, wBot = 0.0f;
   uint32_t count = 0, link = 0, second = 0;
 #pragma unroll
@@ -614,10 +613,10 @@ __device__ __forceinline__ void sum_children(const DevState &S, uint32_t have,
   if (count > 1) {
     wBot = w;
     link = second;
-    if (record) quad_record<kFull>(S, second, X, Y, have, cu, ca, cm, first);
   }
   up = make_float4(sx, sy, wBot, __uint_as_float(link));
   own = make_float4(X, Y, sm, w);
+  return count > 1;
 }
 
 // Place of a spanning node (k_trav_tree) in the arrays span*.
@@ -651,7 +650,7 @@ __device__ __forceinline__ uint32_t span_slot(uint32_t record, int depth) {
 // all bisected and every arrival through global memory, 10,000 bodies 43,
 // 99,991 53, 2^20 86, 2^22 167 without the quad records; with the spanning nodes
 // summed here, whose threads held their blocks, 31, 34, 70, 228; now 28, 34, 65,
-// 159.
+// 157.
 template <bool kFull>
 __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
     k_trav_tree(DevState S, const uint32_t *__restrict__ owner) {
@@ -806,7 +805,7 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
       uint32_t at = 0;
       if (lane == 0) at = atomicAdd(&S.counters[kCtrSpans], (uint32_t)__popc(spanning));
       at = __shfl_sync(0xffffffffu, at, 0) + __popc(spanning & ((1u << lane) - 1u));
-      if (spans) S.spanList[at] = make_uint2(p, (uint32_t)d);
+      if (spans) S.spanList[at] = make_uint4(p, (uint32_t)d, e - i, i);
     }
     __syncthreads();
     // the node this thread holds the sums of: its record, depth and bodies
@@ -889,8 +888,7 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
         if (kFull) cm[q] = sM[k];
         first[q] = sStart[k];
       }
-      sum_children<kFull>(S, have, cu, ca, cm, first, sA[l].w, kFull ? sM[l].w : 0.0f, false, up,
-                          own, mom);
+      sum_children<kFull>(have, cu, ca, cm, first, sA[l].w, kFull ? sM[l].w : 0.0f, up, own, mom);
     }
     __syncthreads();
     if (t < held && !spans) { // the nodes summed in the block, a thread to each
@@ -922,32 +920,51 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
 // lay in blocks, climbing from there: a child brought to its parent here adds
 // its bodies to a second counter, and the one that completes the count of the
 // first is the last.  Leaves the nodes' slots empty for the next build.
-// ~10 nodes a block of records; bound by the chain of arrivals (release,
-// atomic, two rounds of loads a level).
+// ~10 nodes a block of records; bound by the chain of arrivals, so what a level
+// needs of its parent is loaded beside its children's sums, and the node's
+// own record is written after its arrival (with the moments 48 -> 42 us of the
+// stage at 262,144 bodies; without, at 2^22, 159 -> 157).  Depth by depth with
+// barriers instead, in one block, takes 2 us less at 10,000 to 100,000
+// bodies and 20 more at 2^20.
+constexpr int kTopBlock = 64;
 template <bool kFull>
-__global__ void __launch_bounds__(kBlock) k_trav_top(DevState S) {
+__global__ void __launch_bounds__(kTopBlock) k_trav_top(DevState S) {
   chain_begin();
   const uint32_t total = S.counters[6];
   if (total > S.nodeCapacity) return;
   const uint32_t n = S.counters[kCtrSpans];
-  for (uint32_t k = blockIdx.x * kBlock + threadIdx.x; k < n; k += gridDim.x * kBlock) {
-    const uint2 entry = S.spanList[k];
-    uint32_t node = entry.x;
+  for (uint32_t k = blockIdx.x * kTopBlock + threadIdx.x; k < n; k += gridDim.x * kTopBlock) {
+    const uint4 entry = S.spanList[k];
+    uint32_t node = entry.x, bodies = entry.z;
     int d = (int)entry.y;
     uint32_t slot = span_slot(node, d);
-    const int4 B = S.tN[node].b;
-    uint32_t bodies = (uint32_t)(B.w - B.z);
+    const uint64_t ci = S.sortedCodes[entry.w];
+    uint32_t parent = S.spanParent[slot];
+    float w = __ldcg(&S.tN[node].a).w, size = kFull ? __ldcg(&S.tM[node]).w : 0.0f;
     // a node with spanning children never shows its full count here
     if (__ldcg(&S.spanArrive[slot]) != bodies) continue;
-    const uint64_t ci = S.sortedCodes[B.z];
     for (int guard = 0; guard <= kMaxDepth; ++guard) {
       const uint4 kv = __ldcg(&S.spanKids[slot]);
-      const float w = __ldcg(&S.tN[node].a).w;
-      const float size = kFull ? __ldcg(&S.tM[node]).w : 0.0f;
-      const uint32_t parent = d > 0 ? S.spanParent[slot] : 0u;
       __stcg(&S.spanKids[slot], make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu));
       __stcg(&S.spanArrive[slot], 0u);
       __stcg(&S.spanArriveTop[slot], 0u);
+      const bool top = d == 0;
+      if (!top && parent >= total) {
+        atomicOr(S.status, kStatusTreeCapacity);
+        break;
+      }
+      // of the parent (before this node's arrival nobody empties its count)
+      uint32_t pSlot = 0, pParent = 0, pBlocks = 0, pBodies = 0;
+      float pw = 0.0f, pSize = 0.0f;
+      if (!top) {
+        pSlot = span_slot(parent, d - 1);
+        pParent = S.spanParent[pSlot];
+        pBlocks = __ldcg(&S.spanArrive[pSlot]);
+        pw = __ldcg(&S.tN[parent].a).w;
+        if (kFull) pSize = __ldcg(&S.tM[parent]).w;
+        const int4 b = S.tN[parent].b;
+        pBodies = (uint32_t)(b.w - b.z);
+      }
       const uint32_t r[4] = {kv.x, kv.y, kv.z, kv.w};
       uint32_t have = 0, first[4];
       float4 cu[4], ca[4], cm[4], up, own, mom;
@@ -960,34 +977,34 @@ __global__ void __launch_bounds__(kBlock) k_trav_top(DevState S) {
         if (kFull) cm[q] = __ldcg(&S.tM[r[q]]);
         first[q] = (uint32_t)S.tN[r[q]].b.z;
       }
-      sum_children<kFull>(S, have, cu, ca, cm, first, w, size, true, up, own, mom);
+      const bool record = sum_children<kFull>(have, cu, ca, cm, first, w, size, up, own, mom);
+      const uint32_t link = __float_as_uint(up.w);
       __stcg(&S.tN[node].a, own);
       if (kFull) __stcg(&S.tM[node], mom);
-      if (d == 0) {
-        quad_root<kFull>(S, S.segOf[B.z], up, own, mom);
+      uint32_t old = 0;
+      if (!top) {
+        __stcg(&S.tUp[node], up);
+        __stcg(reinterpret_cast<uint32_t *>(&S.spanKids[pSlot]) + digit_at(ci, d - 1), node);
+        // release: the child's sums are visible to the last arriver; acquire: the
+        // last arriver sees every child's
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
+                     : "=r"(old)
+                     : "l"(&S.spanArriveTop[pSlot]), "r"(bodies)
+                     : "memory");
+      }
+      if (record) quad_record<kFull>(S, link, own.x, own.y, have, cu, ca, cm, first);
+      if (top) {
+        quad_root<kFull>(S, S.segOf[entry.w], up, own, mom);
         break;
       }
-      if (parent >= total) {
-        atomicOr(S.status, kStatusTreeCapacity);
-        break;
-      }
-      --d;
-      slot = span_slot(parent, d);
-      const int4 pb = S.tN[parent].b;
-      __stcg(&S.tUp[node], up);
-      __stcg(reinterpret_cast<uint32_t *>(&S.spanKids[slot]) + digit_at(ci, d), node);
-      // release: the child's sums are visible to the last arriver; acquire: the
-      // last arriver sees every child's
-      uint32_t old;
-      asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
-                   : "=r"(old)
-                   : "l"(&S.spanArriveTop[slot]), "r"(bodies)
-                   : "memory");
-      // (a first count that the last arriver has already emptied reads 0, which
-      // cannot complete it either)
-      if (old + bodies + __ldcg(&S.spanArrive[slot]) != (uint32_t)(pb.w - pb.z)) break;
+      if (old + bodies + pBlocks != pBodies) break;
       node = parent;
-      bodies = (uint32_t)(pb.w - pb.z);
+      slot = pSlot;
+      parent = pParent;
+      bodies = pBodies;
+      w = pw;
+      size = pSize;
+      --d;
     }
   }
 }
@@ -1059,10 +1076,10 @@ void launch_trav_tree(cudaStream_t s, const DevState &S, ScanScratch &scan, bool
   mark(s, "tree.counts");
   if (moments) {
     launch_after(s, k_trav_tree<true>, grid_for(n / 4 + 64), kBlock, 0, S, owner);
-    launch_after(s, k_trav_top<true>, grid_for(n / 64 + 64), kBlock, 0, S);
+    launch_after(s, k_trav_top<true>, n / 4096 + 2, kTopBlock, 0, S);
   } else {
     launch_after(s, k_trav_tree<false>, grid_for(n / 4 + 64), kBlock, 0, S, owner);
-    launch_after(s, k_trav_top<false>, grid_for(n / 64 + 64), kBlock, 0, S);
+    launch_after(s, k_trav_top<false>, n / 4096 + 2, kTopBlock, 0, S);
   }
   mark(s, "tree.records");
 }

@@ -165,10 +165,11 @@ struct DevState {
   uint32_t *subtree;    // nodes in subtree
   uint32_t *arrive;     // bottom-up arrival counters
   // nodes of the traversal layout that reach beyond their block of the build
-  // (k_trav_tree): their {record, depth}, and by (block, depth) the parent
-  // record and, empty between builds, the bodies of the children summed in
-  // blocks and of those summed at the top, and the children's records by digit
-  uint2 *spanList;
+  // (k_trav_tree): their {record, depth, bodies, first body}, and by (block,
+  // depth) the parent record and, empty between builds, the bodies of the
+  // children summed in blocks and of those summed at the top, and the
+  // children's records by digit
+  uint4 *spanList;
   uint32_t *spanParent, *spanArrive, *spanArriveTop;
   uint4 *spanKids;
   // traversal layout (preorder)
