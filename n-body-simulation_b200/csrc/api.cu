@@ -13,6 +13,7 @@
 #include <mutex>
 #include <thread>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <new>
 #include <random>
@@ -62,8 +63,8 @@ void launch_interaction_count(cudaStream_t s, const DevState &S,
                               unsigned long long *counts);
 double fp32_fma_peak_tflops(cudaStream_t s);
 void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool groups,
-                         SortScratch &sort, const float2 *points, uint32_t nq, const float box[4],
-                         float2 *sorted, float2 *accSorted, float2 *acc);
+                         SortScratch &sort, float2 *points, uint32_t nq, const float box[4],
+                         float2 *sorted);
 void launch_direct_fp64(cudaStream_t s, const float4 *pv, const float2 *mr,
                         uint32_t n, const uint32_t *targets, const uint2 *ranges,
                         uint32_t m, double eps, int plummer, double2 *partial,
@@ -289,15 +290,16 @@ struct nbx_handle {
   float maxMass = INFINITY; // largest uploaded mass; +inf if any is negative
   FrameWriter *frames = nullptr; // created by the first nbx_nbs2_record
   float coordLimit = 0.0f; // the last upload's limit (kCtrCoordLimit)
-  // nbx_accel_at's buffers for more points than the handle has bodies (up to
-  // that many it uses the handle's own staging and sort scratch), grown to
-  // its largest call (at most kQueryChunk points; larger calls go in chunks)
+  // nbx_accel_at's buffers for more points than the handle's own staging and
+  // sort scratch take, grown to its largest call (at most kQueryChunk points;
+  // larger calls go in chunks): pageable host memory and one device
+  // allocation, since pinning and each allocation cost a first call 0.3 ms
   static constexpr uint32_t kQueryChunk = 1u << 20;
   struct {
-    uint32_t cap = 0;
-    float2 *host = nullptr; // pinned: points, then accelerations
-    float2 *dev = nullptr;  // [4][cap]: points, sorted, their sums, sums
-    SortScratch sort;
+    uint32_t hostCap = 0, cap = 0;
+    float2 *host = nullptr; // points, then accelerations
+    float2 *dev = nullptr;  // [2][cap]: points, then sums; sorted, then their sums
+    SortScratch sort;       // in dev's allocation
   } qs;
   // splat renderer buffers, grown on demand
   struct {
@@ -450,7 +452,7 @@ int allocate(nbx_handle *h) {
   A(S.spanArriveTop, spans);
   A(S.spanList, spans);
   A(S.spanKids, spans);
-  A(S.tN, nodes); // cudaMalloc: 256-byte aligned, so every record is 32
+  A(S.tN, nodes); // 256-byte aligned (carve), so every record is 32
   A(S.tM, nodes);
   if (ns > 1) A(S.groupFirst, S.nGroups);
   // scan / sort scratch
@@ -2110,33 +2112,55 @@ int nbx_mlp_eval(nbx_handle *h, const float *feat, uint32_t n, float *out,
 
 static void query_free(nbx_handle *h) {
   auto &q = h->qs;
-  void *ptrs[] = {q.dev, q.sort.keys[0], q.sort.keys[1], q.sort.vals[0], q.sort.vals[1],
-                  q.sort.hist, q.sort.status, q.sort.tileCounter};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
-  if (q.host) cudaFreeHost(q.host);
+  free(q.host);
+  if (q.dev) cudaFree(q.dev);
   q = {};
 }
 
-// Room for n points.
+// Host room for n points.
+static int query_grow_host(nbx_handle *h, uint32_t n) {
+  auto &q = h->qs;
+  if (q.hostCap >= n) return NBX_OK;
+  free(q.host);
+  q.hostCap = 0;
+  q.host = static_cast<float2 *>(malloc(n * sizeof(float2)));
+  if (!q.host) return fail(h, NBX_ERR_NOMEM, "no host memory for the points");
+  q.hostCap = n;
+  return NBX_OK;
+}
+
+// Device room for n points and their sort, in 256-byte aligned parts.
 static int query_grow(nbx_handle *h, uint32_t n) {
   auto &q = h->qs;
   if (q.cap >= n) return NBX_OK;
-  query_free(h);
-  const uint32_t cap = std::max<uint32_t>(n, 1024);
+  if (q.dev) cudaFree(q.dev);
+  q.dev = nullptr;
+  q.cap = 0;
+  size_t used = 0;
+  auto next = [&](size_t bytes) {
+    const size_t at = used;
+    used += (bytes + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t words = n * sizeof(uint32_t);
+  const size_t points = next(2 * (size_t)n * sizeof(float2));
+  const size_t keys[2] = {next(words), next(words)}, vals[2] = {next(words), next(words)};
+  const size_t hist = next(8 * 256 * sizeof(uint32_t)), tiles = next(8 * sizeof(uint32_t));
+  const size_t status = next(3 * sort_pass_words(n) * sizeof(uint32_t));
+  char *base = nullptr;
+  NBX_CUDA(h, cudaMalloc(&base, used));
+  q.dev = reinterpret_cast<float2 *>(base + points);
   SortScratch &so = q.sort;
-  so.capacity = cap;
-  so.maxTiles = (uint32_t)sort_tiles(cap);
-  NBX_CUDA(h, cudaMallocHost(&q.host, cap * sizeof(float2)));
-  NBX_CUDA(h, cudaMalloc(&q.dev, 4 * (size_t)cap * sizeof(float2)));
+  so.capacity = n;
+  so.maxTiles = (uint32_t)sort_tiles(n);
   for (int k = 0; k < 2; ++k) {
-    NBX_CUDA(h, cudaMalloc(&so.keys[k], cap * sizeof(uint32_t)));
-    NBX_CUDA(h, cudaMalloc(&so.vals[k], cap * sizeof(uint32_t)));
+    so.keys[k] = reinterpret_cast<uint64_t *>(base + keys[k]);
+    so.vals[k] = reinterpret_cast<uint32_t *>(base + vals[k]);
   }
-  NBX_CUDA(h, cudaMalloc(&so.hist, 8 * 256 * sizeof(uint32_t)));
-  NBX_CUDA(h, cudaMalloc(&so.tileCounter, 8 * sizeof(uint32_t)));
-  NBX_CUDA(h, cudaMalloc(&so.status, 3 * sort_pass_words(cap) * sizeof(uint32_t)));
-  q.cap = cap; // only once everything is there
+  so.hist = reinterpret_cast<uint32_t *>(base + hist);
+  so.tileCounter = reinterpret_cast<uint32_t *>(base + tiles);
+  so.status = reinterpret_cast<uint32_t *>(base + status);
+  q.cap = n;
   return NBX_OK;
 }
 
@@ -2147,26 +2171,27 @@ int nbx_accel_at(nbx_handle *h, const float *px, const float *py, uint32_t nq,
   if (!h->treeValid) return fail(h, NBX_ERR_STATE, "no tree built");
   for (uint32_t at = 0; at < nq; at += nbx_handle::kQueryChunk) {
     const uint32_t n = std::min(nq - at, nbx_handle::kQueryChunk);
-    // 8 bytes a point of the pinned body staging, 32 of the device staging's
-    // 36 a body, and the step's sort scratch: all free between calls (every
-    // user of the pinned staging synchronises; the device's is used in stream
-    // order)
+    // the body stagings (36 bytes a body, pinned and on the device) and the
+    // step's sort scratch are free between calls: every user of the pinned
+    // staging synchronises, the device's is used in stream order.  They take 8
+    // bytes a point and 16, and what is beyond takes the handle's own buffers
     float2 *host = reinterpret_cast<float2 *>(h->hPinned);
-    float2 *dev0 = reinterpret_cast<float2 *>(h->dAoS);
+    float2 *dev = reinterpret_cast<float2 *>(h->dAoS);
     SortScratch *sort = &h->sort;
     size_t cap = n;
-    if (n > h->n) {
-      const int rc = query_grow(h, n);
-      if (rc != NBX_OK) {
-        query_free(h);
-        return rc;
-      }
+    int rc = NBX_OK;
+    if (n > (uint64_t)h->n * sizeof(nbx_body) / sizeof(float2)) {
+      rc = query_grow_host(h, n);
       host = h->qs.host;
-      dev0 = h->qs.dev;
+    }
+    if (rc == NBX_OK && n > std::min<uint64_t>((uint64_t)h->n * 2, h->sort.capacity)) {
+      rc = query_grow(h, n);
+      dev = h->qs.dev;
       sort = &h->qs.sort;
       cap = h->qs.cap;
     }
-    // into pinned memory, with the points' box and whether the clamp-free law
+    if (rc != NBX_OK) return rc;
+    // into the staging, with the points' box and whether the clamp-free law
     // may be used at them
     const float lim = h->coordLimit;
     float x0 = FLT_MAX, x1 = -FLT_MAX, y0 = FLT_MAX, y1 = -FLT_MAX;
@@ -2183,15 +2208,12 @@ int nbx_accel_at(nbx_handle *h, const float *px, const float *py, uint32_t nq,
     const float w = x1 - x0, ht = y1 - y0;
     auto scale = [](float e) { return e > 0.0f && e <= FLT_MAX ? 4096.0f / e : 0.0f; };
     const float box[4] = {x0, y0, scale(w), scale(ht)};
-    float2 *dev[4];
-    for (int k = 0; k < 4; ++k) dev[k] = dev0 + (size_t)k * cap;
-    NBX_CUDA(h, cudaMemcpyAsync(dev[0], host, n * sizeof(float2), cudaMemcpyHostToDevice,
+    NBX_CUDA(h, cudaMemcpyAsync(dev, host, n * sizeof(float2), cudaMemcpyHostToDevice,
                                 h->stream));
     launch_query_forces(h->stream, h->state(), h->params.exact_math != 0,
-                        inside && forces_unclamped(h), *sort, dev[0], n, box, dev[1], dev[2],
-                        dev[3]);
+                        inside && forces_unclamped(h), *sort, dev, n, box, dev + cap);
     NBX_CUDA(h, cudaGetLastError());
-    NBX_CUDA(h, cudaMemcpyAsync(host, dev[3], n * sizeof(float2), cudaMemcpyDeviceToHost,
+    NBX_CUDA(h, cudaMemcpyAsync(host, dev, n * sizeof(float2), cudaMemcpyDeviceToHost,
                                 h->stream));
     NBX_CUDA(h, cudaStreamSynchronize(h->stream));
     for (uint32_t i = 0; i < n; ++i) {

@@ -1019,8 +1019,7 @@ __device__ __forceinline__ void store_acc(const DevState &S, uint32_t i, float x
 template <bool kExact, bool kCount, int kCorr, bool kClamp, bool kPairs>
 __device__ __forceinline__ void forces_walk(
     const DevState &S, float tSq, float eSq, unsigned long long *counts,
-    float bandSq, const float2 *__restrict__ query, uint32_t nQuery,
-    float2 *__restrict__ queryAcc, float4 (*sBody)[32]) {
+    float bandSq, float2 *query, uint32_t nQuery, float4 (*sBody)[32]) {
   const int lane = threadIdx.x & 31;
   const int w = threadIdx.x >> 5;
   const uint32_t warpsTotal = (gridDim.x * blockDim.x) >> 5;
@@ -1080,7 +1079,7 @@ __device__ __forceinline__ void forces_walk(
       }
     } else if (valid) {
       if (query) {
-        queryAcc[i] = make_float2(ax, ay);
+        query[i] = make_float2(ax, ay);
       } else {
         store_acc<kExact>(S, i, x, y, ax, ay);
       }
@@ -1105,12 +1104,11 @@ __global__ void __launch_bounds__(kBlock, kPairs && !kExact && !kCount && kCorr 
                                               : 2048 / kBlock)
     k_forces(DevState S, float tSq, float eSq,
              unsigned long long *counts = nullptr, float bandSq = 0.0f,
-             const float2 *__restrict__ query = nullptr, uint32_t nQuery = 0,
-             float2 *__restrict__ queryAcc = nullptr) {
+             float2 *query = nullptr, uint32_t nQuery = 0) {
   chain_begin();
   __shared__ float4 sBody[kBlock / 32][32];
   forces_walk<kExact, kCount, kCorr, kClamp, kPairs>(S, tSq, eSq, counts, bandSq, query, nQuery,
-                                                     queryAcc, sBody);
+                                                     sBody);
 }
 
 // The force pass with the learned correction, one warp per 32 bodies.  us by
@@ -1248,8 +1246,8 @@ __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
 constexpr int kQueryBlock = 128;
 template <GroupWalk kWalk>
 __global__ void __launch_bounds__(kQueryBlock, kGroupWarpsPerSM * 32 / kQueryBlock)
-    k_query_groups(DevState S, float tSq, float eSq, const float2 *__restrict__ query,
-                   uint32_t nQuery, uint32_t per, float2 *__restrict__ queryAcc) {
+    k_query_groups(DevState S, float tSq, float eSq, float2 *query, uint32_t nQuery,
+                   uint32_t per) {
   extern __shared__ uint4 sDyn[];
   const int lane = threadIdx.x & 31;
   WalkStage &st = reinterpret_cast<WalkStage *>(sDyn)[threadIdx.x >> 5];
@@ -1263,7 +1261,7 @@ __global__ void __launch_bounds__(kQueryBlock, kGroupWarpsPerSM * 32 / kQueryBlo
   float ax = 0.0f, ay = 0.0f;
   group_forces<kWalk>(S, tSq, eSq, 0.0f, q.x, q.y, 0u, __ballot_sync(0xffffffffu, mine),
                       st, ax, ay);
-  if (mine) queryAcc[i] = make_float2(ax, ay);
+  if (mine) query[i] = make_float2(ax, ay);
 }
 
 // Sort key of a query point: 12 + 12 interleaved bits of its place in the
@@ -1414,7 +1412,7 @@ void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, boo
 
 // Accelerations at nq arbitrary points from instance 0's last tree
 // (QuadTree::acceleration, QuadTree.cpp:264-389, for any query position):
-// points -> acc through the scratch arrays in order and accSorted.  A target's
+// points -> their sums, in place, through the scratch array sorted.  A target's
 // sums do not depend on its warp, so the points are first put in Morton order
 // of their box [x0, y0, 1 / cell sizes]: neighbours share a warp and its
 // walk.  groups: the clamp-free law may be used (every point within the
@@ -1426,13 +1424,12 @@ void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, boo
 // which a warp's walk is the union of 32 unrelated ones; 100 points 35 and 20
 // us instead of 373.
 void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool groups,
-                         SortScratch &sort, const float2 *points, uint32_t nq, const float box[4],
-                         float2 *sorted, float2 *accSorted, float2 *acc) {
+                         SortScratch &sort, float2 *points, uint32_t nq, const float box[4],
+                         float2 *sorted) {
   const uint32_t blocks = (nq + 255) / 256;
   const bool order = nq > 64; // fewer are a warp or two anyway
   const uint32_t *vals = nullptr;
-  const float2 *query = points;
-  float2 *out = acc;
+  float2 *query = points; // each target's point, then its sums
   if (order) {
     cudaMemsetAsync(sort.hist, 0, 3 * 256 * sizeof(uint32_t), s);
     k_query_keys<<<blocks < 592 ? blocks : 592, 256, 0, s>>>(points, nq, box[0], box[1], box[2],
@@ -1441,7 +1438,6 @@ void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool gro
     vals = sort.vals[buf];
     k_query_gather<<<blocks, 256, 0, s>>>(points, vals, nq, sorted);
     query = sorted;
-    out = accSorted;
   }
   if ((exact || groups) && group_walk_fits(S)) {
     uint32_t per = 32;
@@ -1451,15 +1447,15 @@ void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool gro
     const uint32_t warps = (nq + per - 1) / per;
     auto kernel = exact ? k_query_groups<kExactWalk> : k_query_groups<kPlainWalk>;
     kernel<<<(warps * 32 + kQueryBlock - 1) / kQueryBlock, kQueryBlock,
-             kQueryBlock / 32 * sizeof(WalkStage), s>>>(S, S.tSq, S.eSq, query, nq, per, out);
+             kQueryBlock / 32 * sizeof(WalkStage), s>>>(S, S.tSq, S.eSq, query, nq, per);
   } else {
     const uint32_t b = ((nq + 31) / 32 + kWarps - 1) / kWarps;
     if (exact)
-      k_forces<true><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, 0.0f, query, nq, out);
+      k_forces<true><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, 0.0f, query, nq);
     else
-      k_forces<false><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, 0.0f, query, nq, out);
+      k_forces<false><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, 0.0f, query, nq);
   }
-  if (order) k_query_scatter<<<blocks, 256, 0, s>>>(accSorted, vals, nq, acc);
+  if (order) k_query_scatter<<<blocks, 256, 0, s>>>(sorted, vals, nq, points);
 }
 
 // chained: the launch follows a kernel of the step's chain on s (chain_begin).

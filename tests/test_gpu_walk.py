@@ -163,3 +163,21 @@ def test_tree_sums(nbx, oracle, sizes, leaf):
         ox, oy = oracle.tree_forces(sb["px"], sb["py"], sb["mass"], tree, 0.5, 1.0)
         assert same_bits(g["ax"][at:at + len(p)], ox) and same_bits(g["ay"][at:at + len(p)], oy)
         at += len(p)
+
+
+@pytest.mark.parametrize("nq", [600, 601, 1350, 1351, 5000])
+def test_points_around_the_handles_own_room(nbx, nq):
+    """300 bodies' staging takes 1350 points on the host and 600 on the device;
+    more go through buffers of their own, also after smaller calls: the same
+    bits as in calls of 100."""
+    b = nbx.cold_square(300, 1)
+    p = np.random.default_rng(nq).uniform(-60, 60, (2, nq)).astype(np.float32)
+    sim = nbx.Simulation(b)
+    sim.phase("build")
+    few = [sim.accel_at(p[0, k:k + 100], p[1, k:k + 100]) for k in range(0, nq, 100)]
+    for _ in range(2):
+        ax, ay = sim.accel_at(p[0], p[1])
+        assert same_bits(ax, np.concatenate([f[0] for f in few]))
+        assert same_bits(ay, np.concatenate([f[1] for f in few]))
+        sim.accel_at(p[0, :50], p[1, :50])
+    sim.close()
