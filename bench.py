@@ -62,9 +62,9 @@ FLOP_PER_INTERACTION = 20.0
 # integrate 40, bounds 8, Morton 20, one sort pass 24, gather 56,
 # build + upward ~33, collision 88.
 ALG_BYTES_PER_BODY_STEP = 285.0 - 16.0  # the force pass's 16 B excluded
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_forces
-# launch on the two-disc 1M workload, from an ncu capture of its third launch.
-FORCE_TRAFFIC_BYTES = 23.705856e6
+# DRAM bytes (read + write) of one k_forces_groups launch on the two-disc 1M
+# workload, from an ncu capture of its fourth launch.
+FORCE_TRAFFIC_BYTES = 26.19e6
 
 
 def parse():
@@ -745,12 +745,12 @@ def run_b200(args):
                 "api": "nbx_step_io (pinned host bodies in and out)",
                 "ms_per_step_upload_step_download": e2e_sep_ms},
         "roofline": {
-            "kernel": "k_forces (warp-cooperative traversal)",
+            "kernel": "k_forces_groups (one walk per group of 32 bodies)",
             "bound": "fp32", "achieved": achieved, "peak": peak,
             "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
             "traffic": FORCE_TRAFFIC_BYTES if n == N_BODIES else None,
             "traffic_note": "dram__bytes_read.sum + dram__bytes_write.sum of one "
-                            "launch, ncu capture at step 3 (a constant)",
+                            "launch, ncu capture at step 4 (a constant)",
             "peak_note": "FP32 FMA peak measured live by a probe kernel "
                          "(MEASURED_PEAKS.json holds no FP32 figure)",
             "flops_per_launch": flops, "launch_ms": force_ms,

@@ -24,8 +24,9 @@
 //  * mass / centre-of-mass (and second moments) go up the tree with
 //    arrival counters: the fourth child to finish sums its parent in the
 //    fixed order c0+c1+c2+c3 of sumNode, so the sums are deterministic.
-// A second pass lays the nodes out in depth-first preorder for the force
-// traversal (force.cu).
+// Those arrays are made on request only.  A step makes the records of the
+// force traversal (force.cu), in depth-first preorder with the group walk's
+// records of four children, from the same codes (k_trav_tree, k_trav_top).
 #include "nbx_state.cuh"
 
 #include <float.h>
