@@ -289,7 +289,7 @@ __device__ __forceinline__ void root_frame_seg(const DevState &S, uint32_t sg) {
 // among at most kClusterSortMax bodies, whose keys are in keys32(scratch, 0),
 // every other body's key being nonUnit (the units go to the first places of
 // scratch.vals[1]).
-constexpr uint32_t kClusterMortonMax = 40000, kClusterSortMax = 65536;
+constexpr uint32_t kClusterMortonMax = 20480, kClusterSortMax = 65536;
 void cluster_sort_morton(cudaStream_t s, const DevState &S, SortScratch &scratch);
 void cluster_sort_units(cudaStream_t s, const DevState &S, SortScratch &scratch,
                         uint32_t nonUnit);

@@ -793,7 +793,9 @@ int radix_sort_u32(cudaStream_t s, SortScratch &sc, uint32_t n_max,
 // -> now, at 1000 bodies: 47 -> 14 / 33 -> 12, at 8000: 57 -> 20 / 37 -> 16, at
 // 32,000: 61 -> 43 / 40 -> 18, at 65,000: 63 -> 70 / 42 -> 22.  The eight SMs
 // take 0.8 us per 1000 elements, so the codes keep a launch per pass beyond
-// kClusterMortonMax; the units are few of the bodies.
+// kClusterMortonMax (a step here / with a launch per pass: 18,000 bodies 151 /
+// 153, 24,000 163 / 161, 30,011 170 / 163, 40,000 187 / 176); the units are few of
+// the bodies (at 18,000 bodies 153 / 160, at 65,536 197 / 201).
 namespace {
 
 namespace cg = cooperative_groups;
@@ -947,8 +949,8 @@ __global__ void __cluster_dims__(B, 1, 1) __launch_bounds__(T, 1)
       uint32_t peers = __ballot_sync(0xffffffffu, ok);
 #pragma unroll
       for (int bit = 0; bit < 8; ++bit) {
-        const uint32_t bb = __ballot_sync(0xffffffffu, (d >> bit) & 1u);
-        peers &= ((d >> bit) & 1u) ? bb : ~bb;
+        const uint32_t mine = (uint32_t)((int32_t)(d << (31 - bit)) >> 31); // as k_onesweep
+        peers &= ~(__ballot_sync(0xffffffffu, mine != 0u) ^ mine);
       }
       const uint32_t before = __popc(peers & ltmask);
       uint32_t b = 0;

@@ -34,7 +34,7 @@ def test_steps(nbx, oracle, name, n):
     sim.close()
 
 
-@pytest.mark.parametrize("n", [32769, 39999, 40000, 40001, 65536, 65537])
+@pytest.mark.parametrize("n", [20479, 20480, 20481, 32769, 39999, 40000, 40001, 65536, 65537])
 def test_orders(nbx, oracle, n):
     """Around the largest sizes of each variant: the Morton permutation and
     the pairs in resolution order."""
