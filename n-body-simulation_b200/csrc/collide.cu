@@ -202,14 +202,15 @@ constexpr uint32_t kStash = 16; // partners remembered per body by the count pas
 // at most 0.999 of a cell wide and the cell index is the exact floor), so a
 // body from any other cell fails the overlap test by itself.  The boxes are
 // read beside the indices (gridBox), so a candidate costs no dependent load.
-// All bounds of the nine buckets are loaded at once, the buckets that hold any
-// body are listed in shared memory (ranges: this thread's column) and their
-// bodies taken two at a time across the buckets' ends: bound by the latency
+// kListed: all bounds of the nine buckets are loaded at once, the buckets that
+// hold any body are listed in shared memory (ranges: this thread's column) and
+// their bodies taken two at a time across the buckets' ends: bound by the latency
 // of the chain (cell, bounds, bodies).  us of the count pass, bucket after
 // bucket with a body at a time / so: 10,000 bodies 22 / 13, 2^20 87 / 65, 2^22
 // 382 / 213 (four at a time 238: 48 registers for 40).
+// Otherwise bucket after bucket, without shared memory: see k_partners_fill.
 constexpr int kAtOnce = 2;
-template <class F>
+template <bool kListed, class F>
 __device__ __forceinline__ void for_each_cell_neighbour(const DevState &S, uint32_t i,
                                                         uint32_t sg, const float4 &bi,
                                                         uint32_t mask, uint2 *ranges, F &&f) {
@@ -217,6 +218,24 @@ __device__ __forceinline__ void for_each_cell_neighbour(const DevState &S, uint3
   uint32_t hs[9];
   cell_hash3x3(sg, c.x, c.y, mask, hs);
   const bool oneInstance = S.nseg == 1;
+  if (!kListed) {
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+      bool seen = false;
+#pragma unroll
+      for (int r = 0; r < q; ++r) seen |= hs[r] == hs[q];
+      if (seen) continue;
+      const uint32_t e0 = S.bucketStart[hs[q]], e1 = S.bucketStart[hs[q] + 1];
+      for (uint32_t e = e0; e < e1; ++e) {
+        const uint32_t j = S.grid[e];
+        const float4 bj = S.gridBox[e];
+        if (j == i) continue;
+        if (!oneInstance && S.segOf[j] != sg) continue;
+        if (boxes_overlap(bi, i, bj, j)) f(j);
+      }
+    }
+    return;
+  }
   uint32_t total = 0, listed = 0;
   uint2 range[9];
 #pragma unroll
@@ -277,7 +296,7 @@ __global__ void __launch_bounds__(kBlock) k_partners_count(DevState S) {
     uint32_t cnt = 0;
     uint32_t *stash = S.stash + (size_t)i * kStash;
     if (!(S.slot[i] & 0x80000000u)) {
-      for_each_cell_neighbour(S, i, sg, bi, mask, sRanges + threadIdx.x, [&](uint32_t j) {
+      for_each_cell_neighbour<true>(S, i, sg, bi, mask, sRanges + threadIdx.x, [&](uint32_t j) {
         if (cnt < kStash) stash[cnt] = j;
         ++cnt;
       });
@@ -347,16 +366,20 @@ __device__ __forceinline__ void flush_unit_hist(uint32_t (*sh)[256], uint32_t un
 
 // Fill pass: small bodies copy their stash (or search again past kStash
 // partners) into their CSR list and sort it by the partners' before()
-// order (up to four, nearly all lists, by rank with every load in flight: at
-// 2^22 bodies 102 -> 90 us, at 10,000 13 -> 11); large bodies add their large-large partners, and the count pass's
-// small-large pairs go into the large bodies' lists.  Every body's unit
-// key and its digit counts come out too.
+// order (up to four, nearly all lists of a sparse state, by rank with every load
+// in flight: at 2^22 bodies 133 -> 106 us, at 10,000 13 -> 11); large bodies add
+// their large-large partners, and the count pass's small-large pairs go into
+// the large bodies' lists.  Every body's unit key and its digit counts come out
+// too.
+// A dense state's long lists are sorted through L1, so this pass holds no shared
+// memory beside the histogram: with the second search's bucket ranges there (18 KB
+// a block) it took 13.5 ms instead of 9.5 on the collapsed cold square (2^22
+// bodies after 1990 steps, 26 million pairs) and 6.1 instead of 4.8 after 1800.
 __global__ void __launch_bounds__(kBlock)
     k_partners_fill(DevState S, uint32_t *__restrict__ keys, uint32_t *hist) {
   chain_begin();
   __shared__ uint32_t sh[3][256];
   __shared__ uint32_t sUnits;
-  __shared__ uint2 sRanges[9 * kBlock];
   for (int q = threadIdx.x; q < 3 * 256; q += blockDim.x) sh[q >> 8][q & 255] = 0;
   if (threadIdx.x == 0) sUnits = 0;
   __syncthreads();
@@ -419,8 +442,8 @@ __global__ void __launch_bounds__(kBlock)
       for (uint32_t a = 0; a < cnt; ++a) S.plist[base + a] = stash[a];
     } else {
       uint32_t w = 0;
-      for_each_cell_neighbour(S, i, sg, bi, mask, sRanges + threadIdx.x,
-                              [&](uint32_t j) { S.plist[base + w++] = j; });
+      for_each_cell_neighbour<false>(S, i, sg, bi, mask, nullptr,
+                                     [&](uint32_t j) { S.plist[base + w++] = j; });
       for (uint32_t k = 0; k < lCount; ++k) {
         const uint32_t j = S.largeList[lStart + k];
         if (boxes_overlap(bi, i, S.box[j], j)) S.plist[base + w++] = j;
