@@ -25,9 +25,12 @@
 // schedulers of 4: 86% of what an even split would give.
 //
 // Exact arithmetic, eps = 0 and a subnormal eps^2 run a loop that checks each
-// source's instance and skips j == i (k_naive; the reference skips it
-// explicitly; with eps > 0 it adds exactly zero), as does a block of
-// k_naive_pairs whose targets straddle instances.
+// source's instance and skips j == i (k_naive), as the reference does, and so
+// does a block of k_naive_pairs whose targets straddle instances.  Otherwise the
+// body itself adds m / eps^3 times a distance of zero, and a last tile's padding
+// a mass of zero at the origin: exactly zero both, unless m / eps^3 (eps^-3)
+// overflows -- m 1 below eps 1.4e-13, m 1e6 below 1.4e-11.  Then the sum is NaN,
+// and the block goes through the checked loop.
 #include "nbx_state.cuh"
 
 #include <float.h>
@@ -123,9 +126,8 @@ __global__ void __launch_bounds__(kNaiveThreads) k_naive_pairs(DevState S, float
   const float4 b = S.xym[min(i, S.n - 1u)];
   const float x = b.x, y = b.y;
   float ax = 0.0f, ay = 0.0f;
-  if (src.mixed) {
-    naive_checked<false>(S, src, i, x, y, eSq, tile, ax, ay);
-  } else {
+  bool checked = src.mixed;
+  if (!checked) {
     float *sx = reinterpret_cast<float *>(tile), *sy = sx + kTile, *sm = sy + kTile;
     constexpr int kPer = kTile / kNaiveThreads;
     float4 next[kPer];
@@ -172,7 +174,10 @@ __global__ void __launch_bounds__(kNaiveThreads) k_naive_pairs(DevState S, float
         }
       }
     }
+    checked = __syncthreads_or(ax != ax || ay != ay);
+    if (checked) ax = ay = 0.0f;
   }
+  if (checked) naive_checked<false>(S, src, i, x, y, eSq, tile, ax, ay);
   if (i >= S.n) return;
   add_attractor<false>(S.attr, x, y, ax, ay);
   S.acc[i] = make_float2(ax, ay);

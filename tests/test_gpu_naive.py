@@ -146,3 +146,32 @@ def test_direct_fp64_sums_own_instance(nbx, oracle):
         assert abs(ax[k] - rx[0]) <= 1e-12 * max(1.0, abs(rx[0]))
         assert abs(ay[k] - ry[0]) <= 1e-12 * max(1.0, abs(ry[0]))
     h.close()
+
+
+@pytest.mark.parametrize("n", [1, 5, 128, 255, 256, 257, 259, 600])
+@pytest.mark.parametrize("eps,heavy", [(1e-18, 1.0), (1e-15, 1.0), (1e-13, 1.0), (1e-11, 1e6),
+                                       (2e-11, 1e6), (1e-3, 1e36)])
+def test_naive_body_itself_adds_nothing(nbx, n, eps, heavy):
+    """A softening so small that m / eps^3 overflows: a body still adds nothing
+    to itself, nor does anything at the origin, alone and beside other
+    instances in its blocks."""
+    b = nbx.cold_square(n, 5)
+    b["mass"][n // 2] = heavy
+    b["px"][0], b["py"][0] = 0.0, 0.0
+    x, y, m = (b[k].astype(np.float64) for k in ("px", "py", "mass"))
+    dx, dy = x - x[:, None], y - y[:, None]
+    s = dx * dx + dy * dy + float(np.float32(eps)) ** 2
+    f = np.where(np.eye(n, dtype=bool), 0.0, m / (s * np.sqrt(s)))
+    ex, ey = (dx * f).sum(1), (dy * f).sum(1)
+    # n terms of about ten rounded operations each: (n + 16) half-ulps of the
+    # sum of their sizes
+    tol = (n + 16) * 2.0 ** -24 * (np.hypot(dx, dy) * f).sum(1) + 1e-30
+    others = nbx.cold_square(70, 9)
+    for sizes, bodies, at in (([n], b, 0), ([70, n, 70], np.concatenate([others, b, others]), 70)):
+        sim = nbx.Handle(sizes, force_law=1, epsilon=eps)
+        sim.upload(bodies)
+        sim.phase("attract")
+        g = sim.download()[at:at + n]
+        sim.close()
+        err = np.hypot(g["ax"] - ex, g["ay"] - ey)
+        assert (err <= tol).all(), (sizes, (err / tol).max())
