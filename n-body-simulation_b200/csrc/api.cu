@@ -46,7 +46,8 @@ void render_composite(cudaStream_t s, const float4 *v0, const float4 *v1,
                       uint32_t maxEntries, uint32_t *first, uint32_t *last,
                       const RenderParams &P, float4 *image);
 DevState launch_naive_gather(cudaStream_t s, const DevState &S);
-void launch_naive_forces(cudaStream_t s, const DevState &S, bool exact);
+void launch_naive_forces(cudaStream_t s, const DevState &S, bool exact, float maxMass);
+bool naive_overflows(float eSq, float maxMass);
 void mlp_harvest(cudaStream_t s, const DevState &S, const uint32_t *targets,
                  uint32_t nt, float theta, float band, float eps, uint2 *items,
                  uint32_t cap, uint32_t *count, float *rows);
@@ -552,6 +553,12 @@ bool forces_unclamped(const nbx_handle *h) {
          h->maxMass < 1.6e19f * fminf(1.0f, eSq);
 }
 
+// Whether an all-pairs step has the second kernel (naive_overflows).
+bool naive_again(const nbx_handle *h) {
+  return h->params.force_law == 1 &&
+         naive_overflows(h->params.epsilon * h->params.epsilon, h->maxMass);
+}
+
 // Ranges of the force pass for nbx_step_io: whole warps, at most
 // kIoChunks of them, none for fewer than 64K bodies (the copy is short).
 uint32_t io_chunks(const nbx_handle *h) {
@@ -606,7 +613,7 @@ DevState enqueue_step(nbx_handle *h, cudaStream_t s, DevState S) {
     S = launch_naive_gather(s, S);
     mark(s, "naive.gather");
     if (h->timedCapture) cudaEventRecordWithFlags(h->forceMark[0], s, cudaEventRecordExternal);
-    launch_naive_forces(s, S, h->params.exact_math != 0);
+    launch_naive_forces(s, S, h->params.exact_math != 0, h->maxMass);
     if (h->timedCapture) cudaEventRecordWithFlags(h->forceMark[1], s, cudaEventRecordExternal);
     mark(s, "forces");
     return S;
@@ -982,15 +989,16 @@ int nbx_upload_bodies(nbx_handle *h, const nbx_body *bodies, size_t n) {
   }
   NBX_CUDA(h, cudaStreamSynchronize(h->stream));
   const uint32_t massBits = *h->hWord;
-  // the force pass leaves out its FLT_MAX clamp when it cannot act; a
-  // change of that choice needs new step graphs
+  // the force pass leaves out its FLT_MAX clamp when it cannot act, and the
+  // all-pairs one its second kernel; a change of either choice needs new step
+  // graphs
   uint32_t coordLimitBits = 0;
   {
-    const bool before = forces_unclamped(h);
+    const bool before = forces_unclamped(h), own = naive_again(h);
     float mm = INFINITY; // a negative mass (or -0): keep the clamp
     if (!(massBits & 0x80000000u)) std::memcpy(&mm, &massBits, sizeof(mm));
     h->maxMass = mm;
-    if (forces_unclamped(h) != before) destroy_graphs(h);
+    if (forces_unclamped(h) != before || naive_again(h) != own) destroy_graphs(h);
     // every node sum of x * m stays below 1e36 and every distance below
     // 1.2e19 (its square finite) while all |x|, |y| < this limit
     float lim = 4e18f;
@@ -1521,7 +1529,7 @@ int nbx_phase(nbx_handle *h, int phase) {
   case NBX_PHASE_FORCES:
     if (h->params.force_law == 1) {
       if (!h->forceInput) return fail(h, NBX_ERR_STATE, "no force input gathered");
-      launch_naive_forces(s, S, h->params.exact_math != 0);
+      launch_naive_forces(s, S, h->params.exact_math != 0, h->maxMass);
       break;
     }
     if (!h->treeValid) return fail(h, NBX_ERR_STATE, "no tree built");
@@ -1536,7 +1544,7 @@ int nbx_phase(nbx_handle *h, int phase) {
       h->cur ^= 1;
       h->treeValid = false;
       h->forceInput = true;
-      launch_naive_forces(s, S, h->params.exact_math != 0);
+      launch_naive_forces(s, S, h->params.exact_math != 0, h->maxMass);
       break;
     }
     launch_step_zero(s, S, h->scan, h->sort, false);

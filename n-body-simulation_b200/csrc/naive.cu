@@ -29,8 +29,9 @@
 // does a block of k_naive_pairs whose targets straddle instances.  Otherwise the
 // body itself adds m / eps^3 times a distance of zero, and a last tile's padding
 // a mass of zero at the origin: exactly zero both, unless m / eps^3 (eps^-3)
-// overflows -- m 1 below eps 1.4e-13, m 1e6 below 1.4e-11.  Then the sum is NaN,
-// and the block goes through the checked loop.
+// overflows -- m 1 below eps 1.4e-13, m 1e6 below 1.4e-11.  Then the sum is NaN;
+// where the largest mass allows that, k_naive runs again over the blocks with a
+// NaN (a check in k_naive_pairs itself: 44 registers for 40, 1842 -> 1868 us).
 #include "nbx_state.cuh"
 
 #include <float.h>
@@ -98,10 +99,15 @@ __device__ __forceinline__ void naive_checked(const DevState &S, const Sources &
   }
 }
 
-template <bool kExact>
+// kAgain: only the blocks in which some sum is NaN.
+template <bool kExact, bool kAgain = false>
 __global__ void __launch_bounds__(kNaiveThreads) k_naive(DevState S, float eSq) {
   __shared__ float4 tile[kTile];
   const uint32_t i = blockIdx.x * kNaiveThreads + threadIdx.x;
+  if (kAgain) {
+    const float2 a = S.acc[min(i, S.n - 1u)];
+    if (!__syncthreads_or(a.x != a.x || a.y != a.y)) return;
+  }
   const Sources src = block_sources(S, i);
   const float4 b = S.xym[min(i, S.n - 1u)];
   float ax = 0.0f, ay = 0.0f;
@@ -126,8 +132,9 @@ __global__ void __launch_bounds__(kNaiveThreads) k_naive_pairs(DevState S, float
   const float4 b = S.xym[min(i, S.n - 1u)];
   const float x = b.x, y = b.y;
   float ax = 0.0f, ay = 0.0f;
-  bool checked = src.mixed;
-  if (!checked) {
+  if (src.mixed) {
+    naive_checked<false>(S, src, i, x, y, eSq, tile, ax, ay);
+  } else {
     float *sx = reinterpret_cast<float *>(tile), *sy = sx + kTile, *sm = sy + kTile;
     constexpr int kPer = kTile / kNaiveThreads;
     float4 next[kPer];
@@ -174,10 +181,7 @@ __global__ void __launch_bounds__(kNaiveThreads) k_naive_pairs(DevState S, float
         }
       }
     }
-    checked = __syncthreads_or(ax != ax || ay != ay);
-    if (checked) ax = ay = 0.0f;
   }
-  if (checked) naive_checked<false>(S, src, i, x, y, eSq, tile, ax, ay);
   if (i >= S.n) return;
   add_attractor<false>(S.attr, x, y, ax, ay);
   S.acc[i] = make_float2(ax, ay);
@@ -214,13 +218,26 @@ DevState launch_naive_gather(cudaStream_t s, const DevState &S) {
   return T;
 }
 
+// Whether a body's own term (or the padding's) can overflow in k_naive_pairs;
+// maxMass: of all bodies, or infinity where it is not known.
+bool naive_overflows(float eSq, float maxMass) {
+  const double m = maxMass < 1.0f ? 1.0 : maxMass; // NaN: not known
+  return !(m / ((double)eSq * sqrt((double)eSq)) < 1e38);
+}
+
 // All-pairs accelerations of the bodies in S.xym into S.acc.
-void launch_naive_forces(cudaStream_t s, const DevState &S, bool exact) {
+void launch_naive_forces(cudaStream_t s, const DevState &S, bool exact, float maxMass) {
   if (S.n == 0) return;
   const uint32_t blocks = (S.n + kNaiveThreads - 1) / kNaiveThreads;
-  if (exact) k_naive<true><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
-  else if (S.eSq >= FLT_MIN) k_naive_pairs<<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
-  else k_naive<false><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
+  if (exact) {
+    k_naive<true><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
+  } else if (S.eSq >= FLT_MIN) {
+    k_naive_pairs<<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
+    if (naive_overflows(S.eSq, maxMass))
+      k_naive<false, true><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
+  } else {
+    k_naive<false><<<blocks, kNaiveThreads, 0, s>>>(S, S.eSq);
+  }
 }
 
 } // namespace nbx

@@ -175,3 +175,21 @@ def test_naive_body_itself_adds_nothing(nbx, n, eps, heavy):
         sim.close()
         err = np.hypot(g["ax"] - ex, g["ay"] - ey)
         assert (err <= tol).all(), (sizes, (err / tol).max())
+
+
+def test_naive_masses_change_between_steps(nbx):
+    """Steps captured while no term could overflow, then bodies with which one
+    does: the same bits as from a handle that never saw the first ones."""
+    b = nbx.cold_square(600, 5)
+    h = naive_sim(nbx, b, epsilon=1e-11)
+    h.step(2)
+    b["mass"][7] = 1e6
+    h.upload(b)
+    h.step(1)
+    got = h.download()
+    h.close()
+    other = naive_sim(nbx, b, epsilon=1e-11)
+    other.step(1)
+    want = other.download()
+    other.close()
+    assert np.isfinite(got["ax"]).all() and same_bits(got, want)
