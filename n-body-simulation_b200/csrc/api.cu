@@ -345,13 +345,28 @@ int cuda_fail(nbx_handle *h, cudaError_t e, const char *what) {
     if (e_ != cudaSuccess) return cuda_fail((h), e_, #call);                 \
   } while (0)
 
-// The next piece of the handle's one device allocation: allocate() lays the
-// pieces out twice, first to add up their sizes (arena null), then to set the
-// pointers.  256-byte aligned, with as much again between pieces.
+// Where a piece of `bytes` goes in the handle's one device allocation, `used`
+// bytes of which are taken: large pieces start on 2 MB as allocations of their
+// own would (with all of them packed at 256 bytes the ordered resolution of
+// the collapsed cold square, 2^22 bodies after 1990 steps, took 26.5 ms instead
+// of 24.7), the others on 256 bytes.
+constexpr size_t kArenaLarge = 2u << 20;
+constexpr size_t arena_place(size_t used, size_t bytes) {
+  const size_t align = bytes >= kArenaLarge ? kArenaLarge : 256;
+  return (used + align - 1) & ~(align - 1);
+}
+static_assert(arena_place(1, kArenaLarge) == kArenaLarge && arena_place(257, 4) == 512 &&
+                  arena_place(3 * kArenaLarge, kArenaLarge) == 3 * kArenaLarge,
+              "large pieces on 2 MB");
+
+// The next piece: allocate() lays the pieces out twice, first to add up their
+// sizes (arena null), then to set the pointers, with 256 bytes or more between
+// two pieces.
 template <typename T> void carve(nbx_handle *h, T *&p, size_t count) {
-  const size_t bytes = (std::max<size_t>(count, 1) * sizeof(T) + 511) & ~(size_t)255;
-  p = h->arena ? reinterpret_cast<T *>(h->arena + h->arenaUsed) : nullptr;
-  h->arenaUsed += bytes;
+  const size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  const size_t at = arena_place(h->arenaUsed, bytes);
+  p = h->arena ? reinterpret_cast<T *>(h->arena + at) : nullptr;
+  h->arenaUsed = at + bytes + 256;
 }
 
 uint32_t next_pow2(uint64_t v) {
