@@ -800,6 +800,19 @@ __global__ void __launch_bounds__(kBlock, kFull ? 2 : 3)
         S.spanParent[span_slot(p, d)] = parent;
       }
     }
+    // bodies in leaves too deep for the group walk: one addition a warp where it
+    // has one instance
+    const uint32_t deep = leaf && d > walk_depth(S.tSq) ? e - i : 0u;
+    const uint32_t deepLanes = __ballot_sync(0xffffffffu, deep != 0);
+    if (deepLanes != 0) {
+      const uint32_t one = __shfl_sync(0xffffffffu, sg, __ffs(deepLanes) - 1);
+      if (__all_sync(0xffffffffu, deep == 0 || sg == one)) {
+        const uint32_t sum = __reduce_add_sync(0xffffffffu, deep);
+        if (lane == 0) add_deep(S.seg[one], sum);
+      } else if (deep != 0) {
+        add_deep(S.seg[sg], deep);
+      }
+    }
     // the spanning nodes' list
     const uint32_t spanning = __ballot_sync(0xffffffffu, spans);
     if (spanning) {

@@ -1046,7 +1046,7 @@ __device__ __forceinline__ void forces_walk(
       }
       const SegDev &G = S.seg[query ? 0u : S.segOf[i]];
       if (G.travCount > 0) cur = G.travBase;
-      wide = G.wide != 0u;
+      wide = (G.flags & kSegWide) != 0u;
     }
     float ax = 0.0f, ay = 0.0f;
     uint32_t nFar = 0, nNear = 0, nVisit = 0, nIter = 0, nChunk = 0;
@@ -1090,7 +1090,7 @@ __device__ __forceinline__ void forces_walk(
 // The force pass.  kClamp = false is the clamp-free law (see law_factor),
 // which the host picks only for non-negative masses below its bound; a
 // warp holding a target whose instance reaches beyond the coordinate limit
-// stored at upload (the build's SegDev::wide), where distances could
+// stored at upload (the build's kSegWide), where distances could
 // overflow, takes the clamped walk instead.  Launch bounds: a full SM of
 // kBlock-thread blocks (2048 threads: at most 32 registers) for every walk
 // but the paired plain walk's: 1536 threads per SM (40 registers),
@@ -1147,74 +1147,94 @@ __global__ void __launch_bounds__(kLearnedBlock, 768 / kLearnedBlock)
 }
 
 // Sums of a group walk for the targets of `lanes` (places (x, y), a valid
-// one on every lane) in instance sg: walk_group, the cursor walk where that
-// does not fit, and, for an instance that reaches beyond the coordinate limit,
-// the clamped one (exact arithmetic always clamps), as in k_forces.
-template <GroupWalk kWalk>
-__device__ __forceinline__ void group_forces(const DevState &S, float tSq, float eSq,
-                                             float bandSq, float x, float y, uint32_t sg,
-                                             uint32_t lanes, WalkStage &st,
-                                             float &ax, float &ay) {
+// one on every lane) in instance sg, and, for an instance that reaches beyond the
+// coordinate limit, the clamped cursor walk's (exact arithmetic always clamps),
+// as in k_forces.  Returns the targets whose walk does not fit (kGated: or is left
+// to k_forces_deep): nothing is summed for them, and walk_rest does.
+template <GroupWalk kWalk, bool kGated = false>
+__device__ __forceinline__ uint32_t group_forces(const DevState &S, float tSq, float eSq,
+                                                 float bandSq, float x, float y, uint32_t sg,
+                                                 uint32_t lanes, WalkStage &st,
+                                                 float &ax, float &ay) {
   constexpr bool kExact = kWalk == kExactWalk;
   constexpr int kCorr = kWalk == kQuadWalk ? 2 : 0;
   const int lane = threadIdx.x & 31;
   const SegDev &G = S.seg[sg];
-  if (G.travCount == 0) return; // no tree (capacity)
-  float4 *staged = reinterpret_cast<float4 *>(&st);
-  static_assert(sizeof(WalkStage) >= 32 * sizeof(float4), "holds a leaf's staged bodies");
-  uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
-  if (G.wide) {
+  if (G.travCount == 0) return 0; // no tree (capacity)
+  if (kGated && G.flags == kSegDeep) return lanes;
+  if (G.flags & kSegWide) {
+    uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
     walk_targets<kExact, false, kCorr, true>(S, tSq, eSq, bandSq, x, y,
-                                             (lanes >> lane) & 1u ? G.travBase : kDone, staged,
-                                             ax, ay, c0, c1, c2, c3, c4);
-    return;
+                                             (lanes >> lane) & 1u ? G.travBase : kDone,
+                                             reinterpret_cast<float4 *>(&st), ax, ay, c0, c1, c2,
+                                             c3, c4);
+    return 0;
   }
   // A group whose walk does not fit goes in two at the widest step along its
   // targets, if that is most of the group's extent (neighbours in Morton
-  // order across the gap between two discs, say).
-  uint32_t piece = lanes;
-  while (piece) {
+  // order across the gap between two discs, say).  Only once, since each try
+  // costs a third of a walk and a cusp has such steps at every scale.
+  uint32_t left = lanes, piece = lanes;
+  for (bool whole = true;; whole = false) {
     const bool in = (piece >> lane) & 1u;
     const int lead = __ffs(piece) - 1;
     const float leadX = __shfl_sync(0xffffffffu, x, lead);
     const float leadY = __shfl_sync(0xffffffffu, y, lead);
     const float px = in ? x : leadX, py = in ? y : leadY;
-    if (!walk_group<kWalk>(S, tSq, eSq, bandSq, px, py, sg, piece, st, ax, ay)) {
-      __syncwarp();
-      const float nx = __shfl_down_sync(0xffffffffu, px, 1);
-      const float ny = __shfl_down_sync(0xffffffffu, py, 1);
-      const bool next = in && lane < 31 && ((piece >> (lane + 1)) & 1u);
-      const float step = next ? fabsf(nx - px) + fabsf(ny - py) : 0.0f;
-      const float widest = warp_max(step);
-      const float extent = warp_max(px) - warp_min(px) + warp_max(py) - warp_min(py);
-      const uint32_t at = __ballot_sync(0xffffffffu, step == widest);
-      if (widest > 0.5f * extent) {
-        piece &= (at & (0u - at)) * 2u - 1u; // the lanes up to the step
-        continue;
-      }
-      const uint32_t root = in ? G.travBase : kDone;
-      float wx = 0.0f, wy = 0.0f;
-      if (kWalk == kPlainWalk) {
-        float *sX = reinterpret_cast<float *>(staged);
-        walk_plain_x2(S, tSq, eSq, x, y, root, sX, sX + 32, sX + 64, wx, wy);
-      } else {
-        walk_targets<kExact, false, kCorr, kExact>(S, tSq, eSq, bandSq, x, y, root, staged, wx,
-                                                   wy, c0, c1, c2, c3, c4);
-      }
-      if (in) {
-        ax = wx;
-        ay = wy;
-      }
-    }
+    const bool fits = walk_group<kWalk>(S, tSq, eSq, bandSq, px, py, sg, piece, st, ax, ay);
     __syncwarp();
-    piece = lanes & ~(piece | (piece - 1u)); // the targets after this piece
+    if (fits) {
+      left &= ~piece;
+      if (left == 0) return 0;
+      piece = left;
+      continue;
+    }
+    if (!whole) return left;
+    const float nx = __shfl_down_sync(0xffffffffu, px, 1);
+    const float ny = __shfl_down_sync(0xffffffffu, py, 1);
+    const bool next = in && lane < 31 && ((piece >> (lane + 1)) & 1u);
+    const float step = next ? fabsf(nx - px) + fabsf(ny - py) : 0.0f;
+    const float widest = warp_max(step);
+    const float extent = warp_max(px) - warp_min(px) + warp_max(py) - warp_min(py);
+    const uint32_t at = __ballot_sync(0xffffffffu, step == widest);
+    if (!(widest > 0.5f * extent)) return left;
+    piece &= (at & (0u - at)) * 2u - 1u; // the lanes up to the step
+  }
+}
+
+// The targets `left` by group_forces, with a cursor per lane.
+template <GroupWalk kWalk>
+__device__ __forceinline__ void walk_rest(const DevState &S, float tSq, float eSq, float bandSq,
+                                          float x, float y, uint32_t sg, uint32_t left,
+                                          WalkStage &st, float &axOut, float &ayOut) {
+  constexpr bool kExact = kWalk == kExactWalk;
+  constexpr int kCorr = kWalk == kQuadWalk ? 2 : 0;
+  static_assert(sizeof(WalkStage) >= 32 * sizeof(float4), "holds a leaf's staged bodies");
+  const bool in = (left >> (threadIdx.x & 31)) & 1u;
+  const uint32_t root = in ? S.seg[sg].travBase : kDone;
+  float ax = 0.0f, ay = 0.0f;
+  if (kWalk == kPlainWalk) {
+    float *sX = reinterpret_cast<float *>(&st);
+    walk_plain_x2(S, tSq, eSq, x, y, root, sX, sX + 32, sX + 64, ax, ay);
+  } else {
+    uint32_t c0 = 0, c1 = 0, c2 = 0, c3 = 0, c4 = 0;
+    walk_targets<kExact, false, kCorr, kExact>(S, tSq, eSq, bandSq, x, y, root,
+                                               reinterpret_cast<float4 *>(&st), ax, ay, c0, c1,
+                                               c2, c3, c4);
+  }
+  if (in) {
+    axOut = ax;
+    ayOut = ay;
   }
 }
 
 // A force pass, one group of targets per warp: the default one (leaf_pairs 1),
-// exact arithmetic, or the quadrupole term.
+// exact arithmetic, or the quadrupole term.  Targets that do not fit are walked
+// with a cursor per lane.  That takes twice the time here that it takes at
+// k_forces' occupancy, so with kGated k_forces_deep does the whole pass where many
+// are not likely to fit.
 constexpr int kGroupWarpsPerSM = 20;
-template <int kBlock, GroupWalk kWalk>
+template <int kBlock, GroupWalk kWalk, bool kGated>
 __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
                                               ? kGroupWarpsPerSM * 32 / kBlock : 1)
     k_forces_groups(DevState S, float tSq, float eSq, float bandSq) {
@@ -1234,11 +1254,42 @@ __global__ void __launch_bounds__(kBlock, kGroupWarpsPerSM * 32 / kBlock > 0
     const uint32_t i = mine ? first + lane : first;
     const float4 b = S.xym[i];
     float ax = 0.0f, ay = 0.0f;
-    group_forces<kWalk>(S, tSq, eSq, bandSq, b.x, b.y, sg,
-                        __ballot_sync(0xffffffffu, mine), st, ax, ay);
+    const uint32_t left = group_forces<kWalk, kGated>(S, tSq, eSq, bandSq, b.x, b.y, sg,
+                                              __ballot_sync(0xffffffffu, mine), st, ax, ay);
+    if (left != 0) {
+      if (kGated && G.flags == kSegDeep) continue;
+      walk_rest<kWalk>(S, tSq, eSq, bandSq, b.x, b.y, sg, left, st, ax, ay);
+    }
     if (mine) store_acc<kWalk == kExactWalk>(S, i, b.x, b.y, ax, ay);
     __syncwarp();
   }
+}
+
+// The instances that k_forces_groups<.., true> leaves, with a cursor per lane.
+constexpr int kDeepBlock = 256;
+__global__ void __launch_bounds__(kDeepBlock, 1536 / kDeepBlock)
+    k_forces_deep(DevState S, float tSq, float eSq) {
+  chain_begin();
+  if (S.nseg == 1 && S.seg[0].flags != kSegDeep) return;
+  __shared__ float sBody[kDeepBlock / 32][96];
+  const uint32_t end = S.forceEnd ? min(S.forceEnd, S.n) : S.n;
+  const uint32_t i = S.forceBegin + blockIdx.x * kDeepBlock + threadIdx.x;
+  float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  uint32_t root = kDone;
+  bool mine = false;
+  if (i < end) {
+    const SegDev &G = S.seg[S.segOf[i]];
+    mine = G.flags == kSegDeep;
+    if (mine) {
+      b = S.xym[i];
+      root = G.travCount > 0 ? G.travBase : kDone;
+    }
+  }
+  if (!__any_sync(0xffffffffu, mine)) return;
+  float *sX = sBody[threadIdx.x >> 5];
+  float ax = 0.0f, ay = 0.0f;
+  walk_plain_x2(S, tSq, eSq, b.x, b.y, root, sX, sX + 32, sX + 64, ax, ay);
+  if (mine) store_acc<false>(S, i, b.x, b.y, ax, ay);
 }
 
 // The same sums at query points (instance 0's tree), `per` consecutive points
@@ -1259,8 +1310,9 @@ __global__ void __launch_bounds__(kQueryBlock, kGroupWarpsPerSM * 32 / kQueryBlo
   const uint32_t i = (uint32_t)first + (mine ? lane : 0);
   const float2 q = query[i];
   float ax = 0.0f, ay = 0.0f;
-  group_forces<kWalk>(S, tSq, eSq, 0.0f, q.x, q.y, 0u, __ballot_sync(0xffffffffu, mine),
-                      st, ax, ay);
+  const uint32_t left = group_forces<kWalk>(S, tSq, eSq, 0.0f, q.x, q.y, 0u,
+                                            __ballot_sync(0xffffffffu, mine), st, ax, ay);
+  if (left != 0) walk_rest<kWalk>(S, tSq, eSq, 0.0f, q.x, q.y, 0u, left, st, ax, ay);
   if (mine) query[i] = make_float2(ax, ay);
 }
 
@@ -1361,8 +1413,9 @@ uint32_t force_targets(const DevState &S) {
   return e > S.forceBegin ? e - S.forceBegin : 0u;
 }
 
-// Whether groups' walks nearly always fit their scratch (one that does not
-// is walked with a cursor per lane in the same kernel, at few warps per SM):
+// Whether groups' walks nearly always fit their scratch, for bodies spread
+// evenly (what does not fit is walked with a cursor per lane at few warps per SM; the
+// kernels see uneven states themselves, walk_depth):
 // a group opens about 3 log4(n / L) / theta^2 records and its leaves hold
 // about 2.3 L (1 + 1 / theta)^2 bodies, n the mean instance (measured at theta
 // 0.25 to 0.5 and leaf capacities 4 to 64).  2^20 bodies, L 16, us with / without: theta 0.5
@@ -1375,21 +1428,26 @@ bool group_walk_fits(const DevState &S) {
   return 0.5f * log2f(fmaxf(n / L, 1.0f)) <= 40.0f * S.tSq && L * near * near <= 330.0f;
 }
 
-template <int kBlock, GroupWalk kWalk>
+// Above so many groups the default pass has k_forces_deep behind it, for states in
+// which many groups do not fit.  Where none does not it costs 1 us at 60,000
+// bodies and 8 at 2^20 (force pass 618 -> 624).  Plummer's density, us without
+// groups / with, without k_forces_deep / with it: 60,000 bodies theta 0.4 213 / 274 /
+// 216; 2^20 theta 0.5 1239 / 2040 / 1221, 2^22 5242 / 10210 / 5138; a cusp (density as
+// r^-1.8): 100,000 theta 0.5 432 / 480 / 433, 2^20 1660 / 1700 / 1652.
+constexpr uint32_t kGateGroups = 1024;
+
+template <int kBlock, GroupWalk kWalk, bool kGated = false>
 void launch_groups(cudaStream_t s, const DevState &S, int blocks, float band, bool chained) {
   constexpr int smem = kBlock / 32 * (int)sizeof(WalkStage);
+  constexpr auto kernel = k_forces_groups<kBlock, kWalk, kGated>;
   if (smem > 48 * 1024) // above what a launch may ask for by default
-    cudaFuncSetAttribute(k_forces_groups<kBlock, kWalk>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (blocks <= 0) {
     const uint32_t warps = (S.tgEnd ? S.tgEnd : S.nGroups) - S.tgBegin, per = kBlock / 32;
     blocks = (int)std::max(1u, (warps + per - 1) / per);
   }
-  if (chained)
-    launch_after(s, k_forces_groups<kBlock, kWalk>, blocks, kBlock, smem, S, S.tSq, S.eSq,
-                 band * band);
-  else
-    k_forces_groups<kBlock, kWalk><<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq, band * band);
+  if (chained) launch_after(s, kernel, blocks, kBlock, smem, S, S.tSq, S.eSq, band * band);
+  else kernel<<<blocks, kBlock, smem, s>>>(S, S.tSq, S.eSq, band * band);
 }
 
 // The default plain walk with kBlock threads per block and the paired or
@@ -1403,7 +1461,13 @@ void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, boo
     const uint32_t b = (warps + per - 1) / per;
     blocks = (int)(b ? b : 1);
   }
-  if (pairs && groups) launch_groups<kBlock, kPlainWalk>(s, S, whole ? 0 : blocks, 0.0f, chained);
+  if (pairs && groups && S.nGroups > kGateGroups) {
+    launch_groups<kBlock, kPlainWalk, true>(s, S, whole ? 0 : blocks, 0.0f, chained);
+    const uint32_t deep = std::max(1u, (force_targets(S) + kDeepBlock - 1u) / kDeepBlock);
+    if (chained) launch_after(s, k_forces_deep, deep, kDeepBlock, 0, S, S.tSq, S.eSq);
+    else k_forces_deep<<<deep, kDeepBlock, 0, s>>>(S, S.tSq, S.eSq);
+  } else if (pairs && groups)
+    launch_groups<kBlock, kPlainWalk>(s, S, whole ? 0 : blocks, 0.0f, chained);
   else if (pairs)
     k_forces<false, false, 0, false, kBlock, true><<<blocks, kBlock, 0, s>>>(S, S.tSq, S.eSq);
   else

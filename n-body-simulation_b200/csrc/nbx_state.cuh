@@ -7,16 +7,20 @@
 
 namespace nbx {
 
+// Flags of a segment: bodies reach beyond the clamp guard's coordinate limit;
+// so many of them lie in leaves deeper than walk_depth (SegDev::deep) that the
+// default force pass does the segment without the group walk.
+constexpr uint32_t kSegWide = 1u, kSegDeep = 2u;
+
 // Per-segment record in device memory.
 struct SegDev {
   uint32_t start, count;       // body range [start, start+count)
   float cell, invCell, smallW; // collision grid cell; boxes wider than
                                // smallW go to the large list
-  uint32_t wide;               // written every step: bodies reach beyond the
-                               // clamp guard's coordinate limit
+  uint32_t flags;              // written every step: kSegWide, kSegDeep
   // written every step
   float cx, cy, size; // root square (Quad::newContaining)
-  uint32_t pad1;
+  uint32_t deep;      // bodies in leaves deeper than walk_depth
   MortonFrame frame;  // quantisation constants (binary64 bit patterns)
   uint32_t nodeBase;  // first node of this segment's tree (breadth-first
                       // arrays, the reference's numbering)
@@ -71,7 +75,7 @@ constexpr int kLevelSlots = 34; // depths 0..32 plus an end slot
 // leave out the law's FLT_MAX clamp only while every distance it forms
 // stays finite: the upload stores the largest coordinate allowed here
 // (float bits), and each build marks the instances whose bodies reach
-// beyond it (SegDev::wide), for the force pass to keep the clamp there.
+// beyond it (kSegWide), for the force pass to keep the clamp there.
 constexpr int kCtrCoordLimit = 15;
 constexpr int kCtrSpans = 11; // spanning nodes of the build (DevState::spanList)
 constexpr int kCtrBoundsDone = 7; // blocks of the bounds pass done (self-resetting)
@@ -244,6 +248,23 @@ __device__ __forceinline__ uint64_t body_code(float4 p, const MortonFrame &f) {
          spread_bits(quantise_fp64(p.x, __longlong_as_double((long long)f.x0), sc));
 }
 
+// Depth of a leaf beyond which the group walk (force.cu) hardly ever fits its
+// scratch: a walk opens about as many records at every level.  Leaf depths at which half
+// the groups fit, theta 0.4 / 0.45 / 0.5 / 0.6: a cusp (density as r^-1.8) 11 / 13
+// / 16 / 19, Plummer's density 14 / 16 / 17 to 18 / over 20; bodies spread evenly lie
+// at depth 9 (2^20) or 10 (2^22).
+__device__ __forceinline__ int walk_depth(float tSq) {
+  return (int)(36.0f * sqrtf(tSq) - 1.5f);
+}
+
+// Adds bodies of a segment in deeper leaves.  kSegDeep from an eighth of its bodies
+// on: a cursor takes about twice the time at the group walk's occupancy, and
+// groups save a fifth.
+__device__ __forceinline__ void add_deep(SegDev &G, uint32_t bodies) {
+  const uint32_t limit = G.count / 8u, before = atomicAdd(&G.deep, bodies);
+  if (before <= limit && before + bodies > limit) atomicOr(&G.flags, kSegDeep);
+}
+
 __device__ __forceinline__ float key_to_float(uint32_t k) {
   return u2f((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
 }
@@ -276,7 +297,8 @@ __device__ __forceinline__ void root_frame_seg(const DevState &S, uint32_t sg) {
   // clamp guard: bodies beyond the upload's coordinate limit (NaN-safe)
   const float lim = __uint_as_float(S.counters[kCtrCoordLimit]);
   const float reach = fmaxf(fmaxf(fabsf(minX), fabsf(maxX)), fmaxf(fabsf(minY), fabsf(maxY)));
-  G.wide = (k0 != 0xffffffffu && !(reach < lim)) ? 1u : 0u;
+  G.flags = (k0 != 0xffffffffu && !(reach < lim)) ? kSegWide : 0u;
+  G.deep = 0u; // counted by the build
   b[0] = 0xffffffffu;
   b[1] = 0u;
   b[2] = 0xffffffffu;
