@@ -390,6 +390,8 @@ int allocate(nbx_handle *h) {
   const uint32_t nodes = S.nodeCapacity;
   const uint32_t sortCap = 2 * n + 64;
   h->groupFirst.clear();
+  S.largest = 0;
+  for (uint32_t c : h->segCount) S.largest = std::max(S.largest, c);
   S.nGroups = (n + 31) / 32; // one instance: group g starts at 32 g
   if (ns > 1) {
     for (uint32_t s = 0; s < ns; ++s)

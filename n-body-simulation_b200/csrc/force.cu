@@ -1415,17 +1415,19 @@ uint32_t force_targets(const DevState &S) {
 
 // Whether groups' walks nearly always fit their scratch, for bodies spread
 // evenly (what does not fit is walked with a cursor per lane at few warps per SM; the
-// kernels see uneven states themselves, walk_depth):
-// a group opens about 3 log4(n / L) / theta^2 records and its leaves hold
-// about 2.3 L (1 + 1 / theta)^2 bodies, n the mean instance (measured at theta
-// 0.25 to 0.5 and leaf capacities 4 to 64).  2^20 bodies, L 16, us with / without: theta 0.5
-// 610 / 717, 0.45 673 / 812, 0.4 (refused) 1113 / 935; L 64 at theta 0.5
-// (refused) 3700 / 874.  30,000 bodies at theta 0.5: 39 / 88.
+// kernels see uneven states themselves, walk_depth): a group opens about
+// 3 log4(n / L) / theta^2 records and its leaves hold about 2.3 L (1 + 1 / theta)^2
+// bodies, n the largest instance.  Time without groups / with, discs and squares
+// of 10,000 to 2^22 bodies, theta 0.28 to 0.45, leaf capacities 4 and 16, by
+// log4(n / L) / theta^2: up to 48 from 1.16 to 3.3, at 50 from 0.71 (30,000 bodies, L 4,
+// theta 0.36) to 2.5, from 60 on down to 0.44.  L 64 at theta 0.5 (refused), 2^20
+// bodies: 874 us / 3700.  An instance of 2^20 bodies and 200 of 1000, theta 0.33: 1411
+// us / 2720 (9841 before what does not fit was walked at once).
 bool group_walk_fits(const DevState &S) {
-  const float L = (float)S.leafCapacity, n = (float)S.n / (float)S.nseg, t = sqrtf(S.tSq);
+  const float L = (float)S.leafCapacity, n = (float)S.largest, t = sqrtf(S.tSq);
   if (!(t > 0.0f)) return false;
   const float near = 1.0f + 1.0f / t;
-  return 0.5f * log2f(fmaxf(n / L, 1.0f)) <= 40.0f * S.tSq && L * near * near <= 330.0f;
+  return 0.5f * log2f(fmaxf(n / L, 1.0f)) <= 48.0f * S.tSq && L * near * near <= 330.0f;
 }
 
 // Above so many groups the default pass has k_forces_deep behind it, for states in

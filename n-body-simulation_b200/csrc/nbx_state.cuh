@@ -188,6 +188,7 @@ struct DevState {
   // the order of its sums, is the same in an ensemble and on its own
   uint32_t *groupFirst; // first body of each group (nseg > 1; else 32 g)
   uint32_t nGroups;
+  uint32_t largest;        // bodies of the largest instance
   uint32_t tgBegin, tgEnd; // groups of [forceBegin, forceEnd)
   float4 *tM; // {Ixx, Iyy, Ixy, size} for the learned correction
   float2 *tC; // square centre, for the learned correction

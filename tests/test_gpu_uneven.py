@@ -81,3 +81,8 @@ def test_groups_that_do_not_fit_cost_little(nbx, name, n, theta):
     b = [system(nbx, name, n)]
     assert force_ms(nbx, b, theta=theta) < 2.0 * force_ms(nbx, b, theta=theta, leaf_pairs=0)
 
+
+def test_a_large_instance_among_small_ones(nbx):
+    """Whether groups fit is a matter of the instance that holds the bodies."""
+    parts = [nbx.uniform_disc(1 << 20, 0)] + [nbx.uniform_disc(1000, k) for k in range(200)]
+    assert force_ms(nbx, parts, theta=0.33) < 1.5 * force_ms(nbx, parts, theta=0.33, leaf_pairs=0)
