@@ -3,6 +3,8 @@
 #pragma once
 #include "nbx_internal.cuh"
 
+#include <cstddef>
+
 #include <float.h>
 
 namespace nbx {
@@ -14,13 +16,14 @@ constexpr uint32_t kSegWide = 1u, kSegDeep = 2u;
 
 // Per-segment record in device memory.
 struct SegDev {
-  uint32_t start, count;       // body range [start, start+count)
+  uint32_t start, count; // body range [start, start+count)
+  // written every step (one store resets both)
+  uint32_t flags; // kSegWide, kSegDeep
+  uint32_t deep;  // bodies in leaves deeper than walk_depth
   float cell, invCell, smallW; // collision grid cell; boxes wider than
                                // smallW go to the large list
-  uint32_t flags;              // written every step: kSegWide, kSegDeep
   // written every step
   float cx, cy, size; // root square (Quad::newContaining)
-  uint32_t deep;      // bodies in leaves deeper than walk_depth
   MortonFrame frame;  // quantisation constants (binary64 bit patterns)
   uint32_t nodeBase;  // first node of this segment's tree (breadth-first
                       // arrays, the reference's numbering)
@@ -30,6 +33,10 @@ struct SegDev {
   uint32_t travCount; // nodes in the traversal layout (non-empty nodes)
   uint32_t travBase;  // first record of this segment's traversal layout
 };
+
+static_assert(offsetof(SegDev, flags) % 8 == 0 && alignof(SegDev) == 8 &&
+                  offsetof(SegDev, deep) == offsetof(SegDev, flags) + 4,
+              "flags and deep are one 8-byte word");
 
 // A node of the force traversal, in depth-first preorder: a = {comX, comY,
 // mass, size*size}, b = {next, open, start, end}: next = the slot after the
@@ -298,8 +305,8 @@ __device__ __forceinline__ void root_frame_seg(const DevState &S, uint32_t sg) {
   // clamp guard: bodies beyond the upload's coordinate limit (NaN-safe)
   const float lim = __uint_as_float(S.counters[kCtrCoordLimit]);
   const float reach = fmaxf(fmaxf(fabsf(minX), fabsf(maxX)), fmaxf(fabsf(minY), fabsf(maxY)));
-  G.flags = (k0 != 0xffffffffu && !(reach < lim)) ? kSegWide : 0u;
-  G.deep = 0u; // counted by the build
+  *reinterpret_cast<uint2 *>(&G.flags) =
+      make_uint2((k0 != 0xffffffffu && !(reach < lim)) ? kSegWide : 0u, 0u);
   b[0] = 0xffffffffu;
   b[1] = 0u;
   b[2] = 0xffffffffu;
