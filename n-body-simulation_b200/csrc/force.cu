@@ -1430,6 +1430,22 @@ bool group_walk_fits(const DevState &S) {
   return 0.5f * log2f(fmaxf(n / L, 1.0f)) <= 48.0f * S.tSq && L * near * near <= 330.0f;
 }
 
+// Whether the default force pass gains by groups where they fit: at a large theta
+// the walk is short, and a group's ~12 dependent batches cost more than a cursor's
+// steps as soon as warps queue for the GPU.  Force pass of a disc, a square and
+// bodies in clumps of clumps, us with a cursor / in groups: 100,000 bodies theta 1
+// 51 / 46, 52 / 44, 47 / 48; 200,000 theta 0.85 88 / 85, 86 / 83, 71 / 81, theta 1 76 / 77,
+// 72 / 75, 61 / 77, theta 2 of the disc 24 / 36; 400,000 theta 0.7 178 / 163, 174 / 159,
+// 145 / 155, theta 1 129 / 132, 125 / 130, 106 / 134; 2^20 theta 0.7 434 / 411, 410 / 411,
+// 340 / 388, theta 0.85 360 / 374, 342 / 374, 284 / 359; 2^22 theta 0.7 of the disc
+// 1732 / 1663.  Smaller leaves make longer walks: the disc, 200,000, theta 1, leaf
+// capacity 1 123 / 100, 4 94 / 82, 8 84 / 78, 32 73 / 79, 64 85 / 98.
+bool group_walk_pays(const DevState &S) {
+  return S.nGroups <= 148u * kGroupWarpsPerSM ||
+         sqrtf(S.tSq) <= 0.715f * powf(fmaxf(1048576.0f / (float)S.n, 1.0f), 0.2f) *
+                             powf(16.0f / (float)S.leafCapacity, 0.1f);
+}
+
 // Above so many groups the default pass has k_forces_deep behind it, for states in
 // which many groups do not fit.  Where none does not it costs 1 us at 60,000
 // bodies and 8 at 2^20 (force pass 618 -> 624).  Plummer's density, us without
@@ -1531,7 +1547,7 @@ void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
   if (corr == 0 && !exact && noClamp) {
     // the group walk where its records nearly always fit, with 128 threads a
     // block by default (see group_walk_fits), else a cursor per lane
-    const bool groups = pairs && group_walk_fits(S);
+    const bool groups = pairs && group_walk_fits(S) && group_walk_pays(S);
     if (threads == 0) threads = groups ? 128 : 256;
     if (threads == 128) launch_plain<128>(s, S, blocks, pairs, groups, chained);
     else if (threads == 512) launch_plain<512>(s, S, blocks, pairs, groups, chained);

@@ -86,3 +86,12 @@ def test_a_large_instance_among_small_ones(nbx):
     """Whether groups fit is a matter of the instance that holds the bodies."""
     parts = [nbx.uniform_disc(1 << 20, 0)] + [nbx.uniform_disc(1000, k) for k in range(200)]
     assert force_ms(nbx, parts, theta=0.33) < 1.5 * force_ms(nbx, parts, theta=0.33, leaf_pairs=0)
+
+
+def test_groups_that_do_not_pay(nbx):
+    """Short walks of many bodies: a large theta, bodies on a line."""
+    n = 1 << 20
+    b = nbx.cold_square(n, 1)
+    b["px"] = np.random.default_rng(1).uniform(-3e3, 3e3, n)
+    b["py"], b["radius"] = 0.0, 1e-3
+    assert force_ms(nbx, [b], theta=1.3) < 1.5 * force_ms(nbx, [b], theta=1.3, leaf_pairs=0)
