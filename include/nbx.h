@@ -280,8 +280,10 @@ int nbx_nbs2_flush(nbx_handle *h);
  * nothing sets -- the same loop, limit and status bit as the ordered
  * resolution's and the radix sort's waits -- so that the next nbx_sync
  * returns NBX_ERR_TIMEOUT (about a second later) and the handle stays usable
- * afterwards.  No counterpart in the reference, whose waits are
- * unbounded. */
+ * afterwards.  It also leaves the tree's records as a build on codes that such
+ * a wait left unsorted may: a force pass before the next build is made of
+ * nonsense, but stays in bounds.  No counterpart in the reference, whose waits
+ * are unbounded. */
 int nbx_debug_expire_wait(nbx_handle *h);
 
 /* --- FP64 checks --- */

@@ -400,7 +400,6 @@ int allocate(nbx_handle *h) {
     S.nGroups = (uint32_t)h->groupFirst.size();
   }
   const size_t spans = ((size_t)nodes / 256 + 1) * (kMaxDepth + 1);
-  size_t cleared = 0; // the pieces after it are written before they are read
   auto layout = [&] {
 #define A(ptr, count) carve(h, ptr, count)
   A(S.seg, ns);
@@ -498,8 +497,7 @@ int allocate(nbx_handle *h) {
   A(h->mlpGrad, kMlpParams + 1);
   A(h->mlpW, 1);
   A(S.attr, 2);
-  cleared = h->arenaUsed;
-  A(S.tQ, (size_t)n + ns); // written by every build
+  A(S.tQ, (size_t)n + ns);
   A(S.tQM, (size_t)n + ns);
 #undef A
   };
@@ -509,7 +507,7 @@ int allocate(nbx_handle *h) {
   NBX_CUDA(h, cudaMalloc(&h->arena, h->arenaUsed));
   h->arenaUsed = 0;
   layout();
-  NBX_CUDA(h, cudaMemset(h->arena, 0, cleared));
+  NBX_CUDA(h, cudaMemset(h->arena, 0, h->arenaUsed));
   NBX_CUDA(h, cudaMemset(S.spanKids, 0xff, spans * sizeof(uint4)));
   NBX_CUDA(h, cudaMemcpy(S.attr, h->attrHost, sizeof(h->attrHost), cudaMemcpyHostToDevice));
   if (!h->groupFirst.empty())
@@ -1500,6 +1498,9 @@ int nbx_debug_expire_wait(nbx_handle *h) {
   NBX_CUDA(h, cudaMemsetAsync(flag, 0, sizeof(uint32_t), h->stream));
   k_expire_wait<<<1, 32, 0, h->stream>>>(flag, h->base.status);
   NBX_CUDA(h, cudaGetLastError());
+  // links that lead nowhere, below children of size 1.6e-10
+  const DevState &S = h->base;
+  NBX_CUDA(h, cudaMemsetAsync(S.tQ, 0x2f, ((size_t)S.n + S.nseg) * sizeof(QuadRec), h->stream));
   return NBX_OK;
 }
 

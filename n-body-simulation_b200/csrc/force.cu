@@ -601,7 +601,7 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
       float w[2] = {0.0f, 0.0f};
       uint32_t link[2] = {kQuadLeaf, kQuadLeaf}, mask = 0;
       if (have) {
-        const QuadRec *q = tQ + min(st.rec[slot], lastRec);
+        const QuadRec *q = tQ + st.rec[slot];
         mask = st.who[slot];
         X2 = __ldg(reinterpret_cast<const f2x *>(&q->x) + half);
         Y2 = __ldg(reinterpret_cast<const f2x *>(&q->y) + half);
@@ -704,7 +704,7 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
       for (int j = 0; j < 2; ++j)
         if (inner[j]) {
           if (at < kSlots) {
-            st.rec[at] = link[j];
+            st.rec[at] = min(link[j], lastRec); // defensive bound
             st.who[at] = open[j];
           }
           info[j] |= (at & 255u) | kInfoInner;

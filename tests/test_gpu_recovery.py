@@ -1,0 +1,36 @@
+"""After a bounded device wait has given up: what it leaves behind stays in
+bounds and spoils no later call."""
+import numpy as np
+import pytest
+
+from conftest import same_bits
+
+pytestmark = pytest.mark.gpu
+
+TIMEOUT = 5
+
+
+def expire(nbx, h):
+    h._c(nbx.lib().nbx_debug_expire_wait(h.h))
+    with pytest.raises(nbx.NbxError) as e:
+        h.sync()
+    assert e.value.code == TIMEOUT
+
+
+@pytest.mark.parametrize("sizes", [[20], [300], [5000], [300, 1, 700]])
+def test_records_that_lead_nowhere(nbx, sizes):
+    """Children that every body opens, with links far beyond the records: the
+    group walk gives up within its scratch and the cursor walk, whose records are
+    whole, gives every body its sum."""
+    b = np.concatenate([nbx.cold_square(n, 1) for n in sizes])
+    b["px"] *= np.float32(1e-13)  # the records' children are then far too near
+    b["py"] *= np.float32(1e-13)
+    h = nbx.Handle(sizes, collisions=0)
+    h.upload(b)
+    h.phase("attract")
+    want = h.download()
+    expire(nbx, h)
+    h.phase("forces")
+    got = h.download()
+    h.close()
+    assert np.isfinite(got["ax"]).all() and same_bits(got, want)
