@@ -375,6 +375,22 @@ uint32_t next_pow2(uint64_t v) {
   return (uint32_t)std::min<uint64_t>(p, 1ull << 31);
 }
 
+// Places of the spanning nodes (DevState::spanList).
+size_t span_slots(const DevState &S) {
+  return ((size_t)S.nodeCapacity / 256 + 1) * (kMaxDepth + 1);
+}
+
+// Empties them, as a build expects them.  It leaves them so itself, unless its codes
+// were not sorted: a wait in the sort gave up.
+int empty_spans(nbx_handle *h, cudaStream_t s) {
+  const DevState &S = h->base;
+  const size_t spans = span_slots(S);
+  NBX_CUDA(h, cudaMemsetAsync(S.spanArrive, 0, spans * sizeof(uint32_t), s));
+  NBX_CUDA(h, cudaMemsetAsync(S.spanArriveTop, 0, spans * sizeof(uint32_t), s));
+  NBX_CUDA(h, cudaMemsetAsync(S.spanKids, 0xff, spans * sizeof(uint4), s));
+  return NBX_OK;
+}
+
 int allocate(nbx_handle *h) {
   DevState &S = h->base;
   const uint32_t n = h->n, ns = h->nseg;
@@ -399,7 +415,7 @@ int allocate(nbx_handle *h) {
         h->groupFirst.push_back(h->segStart[s] + b);
     S.nGroups = (uint32_t)h->groupFirst.size();
   }
-  const size_t spans = ((size_t)nodes / 256 + 1) * (kMaxDepth + 1);
+  const size_t spans = span_slots(S);
   auto layout = [&] {
 #define A(ptr, count) carve(h, ptr, count)
   A(S.seg, ns);
@@ -508,7 +524,7 @@ int allocate(nbx_handle *h) {
   h->arenaUsed = 0;
   layout();
   NBX_CUDA(h, cudaMemset(h->arena, 0, h->arenaUsed));
-  NBX_CUDA(h, cudaMemset(S.spanKids, 0xff, spans * sizeof(uint4)));
+  if (const int rc = empty_spans(h, nullptr)) return rc; // on the stream of the memset
   NBX_CUDA(h, cudaMemcpy(S.attr, h->attrHost, sizeof(h->attrHost), cudaMemcpyHostToDevice));
   if (!h->groupFirst.empty())
     NBX_CUDA(h, cudaMemcpy(S.groupFirst, h->groupFirst.data(), S.nGroups * sizeof(uint32_t),
@@ -807,6 +823,7 @@ int check_status(nbx_handle *h) {
   NBX_CUDA(h, cudaStreamSynchronize(h->stream));
   if (!bits) return NBX_OK;
   NBX_CUDA(h, cudaMemsetAsync(h->base.status, 0, 4, h->stream));
+  if (const int rc = empty_spans(h, h->stream)) return rc;
   NBX_CUDA(h, cudaStreamSynchronize(h->stream));
   if (bits & kStatusSpinLimit) return fail(h, NBX_ERR_TIMEOUT, "a bounded device wait gave up");
   if (bits & (kStatusTreeCapacity | kStatusPairCapacity | kStatusLargeCapacity))
@@ -1501,6 +1518,11 @@ int nbx_debug_expire_wait(nbx_handle *h) {
   // links that lead nowhere, below children of size 1.6e-10
   const DevState &S = h->base;
   NBX_CUDA(h, cudaMemsetAsync(S.tQ, 0x2f, ((size_t)S.n + S.nseg) * sizeof(QuadRec), h->stream));
+  // and remainders of nodes that were never completed
+  const size_t spans = span_slots(S);
+  NBX_CUDA(h, cudaMemsetAsync(S.spanArrive, 1, spans * sizeof(uint32_t), h->stream));
+  NBX_CUDA(h, cudaMemsetAsync(S.spanArriveTop, 1, spans * sizeof(uint32_t), h->stream));
+  NBX_CUDA(h, cudaMemsetAsync(S.spanKids, 0, spans * sizeof(uint4), h->stream));
   return NBX_OK;
 }
 

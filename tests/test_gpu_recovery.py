@@ -34,3 +34,30 @@ def test_records_that_lead_nowhere(nbx, sizes):
     got = h.download()
     h.close()
     assert np.isfinite(got["ax"]).all() and same_bits(got, want)
+
+
+@pytest.mark.parametrize("sizes", [[3000], [100001], [9000, 1, 20000]])
+@pytest.mark.parametrize("form", [{}, {"use_mlp": 2, "mlp_band": 0.4, "theta": 0.7}])
+def test_remainders_of_a_tree(nbx, sizes, form):
+    """Arrivals that an unsorted build left at nodes it never completed: later builds
+    of the same handle start from nothing, with the bodies it has and with others."""
+    b = np.concatenate([nbx.cold_square(n, 1) for n in sizes])
+    fresh = []
+    for bodies in (b, b[::-1].copy()):
+        h = nbx.Handle(sizes, collisions=0, **form)
+        h.upload(bodies)
+        h.step(3)
+        fresh.append(h.download())
+        h.close()
+    h = nbx.Handle(sizes, collisions=0, **form)
+    h.upload(b)
+    h.step(1)
+    h.sync()
+    expire(nbx, h)
+    h.step(2)
+    assert same_bits(h.download(), fresh[0])
+    expire(nbx, h)
+    h.upload(b[::-1].copy())
+    h.step(3)
+    assert same_bits(h.download(), fresh[1])
+    h.close()
