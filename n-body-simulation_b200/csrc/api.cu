@@ -2263,7 +2263,11 @@ int nbx_accel_at(nbx_handle *h, const float *px, const float *py, uint32_t nq,
     NBX_CUDA(h, cudaGetLastError());
     NBX_CUDA(h, cudaMemcpyAsync(host, dev, n * sizeof(float2), cudaMemcpyDeviceToHost,
                                 h->stream));
+    // the waits of the points' sort may have given up
+    NBX_CUDA(h, cudaMemcpyAsync(h->hWord, h->base.status, sizeof(uint32_t),
+                                cudaMemcpyDeviceToHost, h->stream));
     NBX_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (*h->hWord & kStatusSpinLimit) return check_status(h);
     for (uint32_t i = 0; i < n; ++i) {
       ax[at + i] = host[i].x;
       ay[at + i] = host[i].y;

@@ -1346,13 +1346,13 @@ __global__ void __launch_bounds__(256)
     k_query_gather(const float2 *__restrict__ from, const uint32_t *__restrict__ order,
                    uint32_t n, float2 *__restrict__ to) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) to[i] = from[order[i]];
+  if (i < n) to[i] = from[min(order[i], n - 1u)]; // defensive bound
 }
 __global__ void __launch_bounds__(256)
     k_query_scatter(const float2 *__restrict__ from, const uint32_t *__restrict__ order,
                     uint32_t n, float2 *__restrict__ to) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) to[order[i]] = from[i];
+  if (i < n && order[i] < n) to[order[i]] = from[i]; // defensive bound
 }
 
 // FMA throughput probe: 8 independent chains per thread.

@@ -61,3 +61,23 @@ def test_remainders_of_a_tree(nbx, sizes, form):
     h.step(3)
     assert same_bits(h.download(), fresh[1])
     h.close()
+
+
+@pytest.mark.parametrize("nq", [1, 64, 65, 5000])
+def test_points_after_an_expired_wait(nbx, nq):
+    """Accelerations at points, sorted or not, are not handed out as good when a
+    wait gave up, and are good again after the next build."""
+    b = nbx.cold_square(1000, 1)
+    p = np.random.default_rng(nq).uniform(-60, 60, (2, nq)).astype(np.float32)
+    h = nbx.Handle([1000])
+    h.upload(b)
+    h.phase("build")
+    want = h.accel_at(p[0], p[1])
+    h._c(nbx.lib().nbx_debug_expire_wait(h.h))
+    with pytest.raises(nbx.NbxError) as e:
+        h.accel_at(p[0], p[1])
+    assert e.value.code == TIMEOUT
+    h.upload(b)
+    h.phase("build")
+    assert all(same_bits(a, w) for a, w in zip(h.accel_at(p[0], p[1]), want))
+    h.close()
