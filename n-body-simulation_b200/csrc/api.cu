@@ -2212,13 +2212,22 @@ static int query_grow(nbx_handle *h, uint32_t n) {
   return NBX_OK;
 }
 
+// Points of nbx_accel_at's next chunk, from point `at` of nq on.
+static constexpr uint32_t query_chunk(uint32_t at, uint32_t nq) {
+  return nq - at < nbx_handle::kQueryChunk ? nq - at : nbx_handle::kQueryChunk;
+}
+// the last chunk ends the largest call (a step of whole chunks would wrap to 0)
+static_assert(0xfff00000u + query_chunk(0xfff00000u, 0xffffffffu) == 0xffffffffu &&
+                  query_chunk(0u, 0xffffffffu) == nbx_handle::kQueryChunk,
+              "at + query_chunk(at, nq) <= nq");
+
 int nbx_accel_at(nbx_handle *h, const float *px, const float *py, uint32_t nq,
                  float *ax, float *ay) {
   if (!h || (nq && (!px || !py || !ax || !ay))) return NBX_ERR_ARG;
   cudaSetDevice(h->device);
   if (!h->treeValid) return fail(h, NBX_ERR_STATE, "no tree built");
-  for (uint32_t at = 0; at < nq; at += nbx_handle::kQueryChunk) {
-    const uint32_t n = std::min(nq - at, nbx_handle::kQueryChunk);
+  for (uint32_t at = 0, n; at < nq; at += n) {
+    n = query_chunk(at, nq);
     // the body stagings (36 bytes a body, pinned and on the device) and the
     // step's sort scratch are free between calls: every user of the pinned
     // staging synchronises, the device's is used in stream order.  They take 8
