@@ -1573,6 +1573,7 @@ int nbx_phase(nbx_handle *h, int phase) {
       break;
     }
     if (!h->treeValid) return fail(h, NBX_ERR_STATE, "no tree built");
+    if (!h->momentsValid) S.tQM = nullptr; // not of this tree
     launch_forces(s, S, h->params.exact_math != 0, h->params.force_blocks,
                   h->mlpLoaded ? h->mlpW : nullptr, h->params.mlp_band,
                   h->params.use_mlp, forces_unclamped(h), h->params.force_block,

@@ -534,7 +534,7 @@ __device__ __forceinline__ uint32_t quad_record(const DevState &S, uint32_t at, 
   Q.w = make_float4(w[0], w[1], w[2], w[3]);
   *reinterpret_cast<uint4 *>(&Q.child[0]) = make_uint4(c[0].x, c[0].y, c[1].x, c[1].y);
   *reinterpret_cast<uint4 *>(&Q.child[2]) = make_uint4(c[2].x, c[2].y, c[3].x, c[3].y);
-  if (kFull) {
+  if (kFull && S.tQM) {
 #pragma unroll
     for (uint32_t q = 0; q < 4; ++q)
       if ((have >> q) & 1u) S.tQM[at].m[q] = make_float4(cm[q].x, cm[q].y, cm[q].z, ca[q].w);

@@ -855,7 +855,7 @@ __device__ __forceinline__ bool walk_group(const DevState &S, float tSq, float e
           // the node of the chain that the target accepts: the largest one that
           // passes (each is exactly a quarter of the last)
           float w = M.w;
-          while (w >= dSq * tSq && on) w *= 0.25f;
+          for (int up = 0; up <= kMaxDepth && on && w >= dSq * tSq; ++up) w *= 0.25f;
           const bool band = on && w >= dSq * bandSq;
           if (__ballot_sync(0xffffffffu, band)) {
             float qx, qy;
@@ -1561,12 +1561,12 @@ void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
   // term, theta 0.65, band 0.4: 10,000 66 / 53, 30,000 84 / 66, 100,000 121 / 135,
   // 2^20 746 / 967: scalar sums and terms of every lane's, unlike the plain
   // walk's pairs, are all they have to offer once there are warps enough.
-  if (S.n <= 65536u && group_walk_fits(S)) {
+  if (S.n <= kOrderedGroupsMax && group_walk_fits(S)) {
     if (corr == 0 && exact) {
       launch_groups<128, kExactWalk>(s, S, blocks, 0.0f, chained);
       return;
     }
-    if (corr == 2 && noClamp) {
+    if (corr == 2 && noClamp && S.tQM) {
       launch_groups<128, kQuadWalk>(s, S, blocks, band, chained);
       return;
     }

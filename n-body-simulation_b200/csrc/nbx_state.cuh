@@ -74,6 +74,9 @@ struct alignas(32) QuadMom {
   float4 m[4];
 };
 constexpr uint32_t kQuadLeaf = 0x80000000u;
+// Bodies up to which exact arithmetic and the quadrupole term walk in groups
+// (launch_forces).
+constexpr uint32_t kOrderedGroupsMax = 65536;
 
 constexpr int kMaxDepth = 32;   // TreeKernels.cuh:29
 constexpr int kLevelSlots = 34; // depths 0..32 plus an end slot
@@ -186,7 +189,8 @@ struct DevState {
   // traversal layout (preorder)
   TravNode *tN; // preorder traversal records (32 bytes, one load each)
   QuadRec *tQ;  // records of the group walks (n + nseg)
-  QuadMom *tQM; // their moments, where the build computes them
+  QuadMom *tQM; // their moments, where the build computes them (null where they
+                // are not there to be read)
   float4 *tUp; // per traversal record, upward pass: {weighted sums x, y,
                // bottom size^2, link bits}; shares the breadth-first arrays'
                // storage (comX ..)
