@@ -514,7 +514,8 @@ int allocate(nbx_handle *h) {
   A(h->mlpW, 1);
   A(S.attr, 2);
   A(S.tQ, (size_t)n + ns);
-  A(S.tQM, (size_t)n + ns);
+  if (n <= kOrderedGroupsMax) A(S.tQM, (size_t)n + ns);
+  else S.tQM = nullptr;
 #undef A
   };
   h->arena = nullptr;

@@ -190,7 +190,7 @@ struct DevState {
   TravNode *tN; // preorder traversal records (32 bytes, one load each)
   QuadRec *tQ;  // records of the group walks (n + nseg)
   QuadMom *tQM; // their moments, where the build computes them (null where they
-                // are not there to be read)
+                // are not there to be read, as beyond kOrderedGroupsMax bodies)
   float4 *tUp; // per traversal record, upward pass: {weighted sums x, y,
                // bottom size^2, link bits}; shares the breadth-first arrays'
                // storage (comX ..)

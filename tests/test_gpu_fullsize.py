@@ -167,3 +167,15 @@ def test_collisions_bit_exact_at_scale(nbx, oracle):
         ref, _ = oracle.collide(st)
         assert same_bits(out, ref), (label, int((out != ref).sum()), depth)
         sim.close()
+
+
+def test_memory_of_a_large_handle(nbx):
+    """A large handle holds no group moments, which only the quadrupole term of few
+    bodies reads: at most 2,600 bytes a body."""
+    import torch
+    n = 1 << 21
+    free = torch.cuda.mem_get_info()[0]
+    h = nbx.Handle([n])
+    held = free - torch.cuda.mem_get_info()[0]
+    h.close()
+    assert held < 2550 * n, held / n
