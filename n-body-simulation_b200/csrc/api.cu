@@ -35,6 +35,8 @@ void launch_step_zero(cudaStream_t s, const DevState &S, ScanScratch &scan, Sort
 void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
                    const MlpDev *mlp, float band, int corr, bool noClamp, int threads,
                    bool pairs, bool chained);
+int force_blocks_per_sm(const DevState &S, bool exact, int corr, bool noClamp, int threads,
+                        bool pairs);
 void render_vertices(cudaStream_t s, const float4 *pv, const float2 *mr, uint32_t n,
                      const RenderParams &P, float4 *v0, float4 *v1, uint32_t *tiles,
                      double4 *partial, unsigned long long *total, float *stats);
@@ -2337,18 +2339,15 @@ int nbx_autotune(nbx_handle *h, int allowLeaf, uint32_t steps, nbx_params *best,
     leafWidths = {1, 0};
   }
   struct Trial {
-    int leaf, threads, pairs, grid;
+    int leaf, threads, pairs, halves;
   };
   std::vector<Trial> trials;
   for (int leaf : leaves)
     for (int threads : blockShapes)
       for (int pairs : leafWidths) {
-        // grids: one warp per 32 bodies, or a half, one or two full SMs'
-        // worth of resident blocks per SM (the group walk's launch bounds
-        // hold 1024 threads per SM, the single-body walk's 2048)
-        const int perSm = (pairs ? 1024 : 2048) / (threads > 0 ? threads : 128);
-        for (int grid : {0, sms * perSm / 2, sms * perSm, sms * perSm * 2})
-          trials.push_back({leaf, threads, pairs, grid});
+        // grids: one warp per 32 bodies, or half as many blocks as the GPU holds
+        // at a time, all of them, or twice as many
+        for (int halves : {0, 1, 2, 4}) trials.push_back({leaf, threads, pairs, halves});
       }
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
@@ -2359,11 +2358,15 @@ int nbx_autotune(nbx_handle *h, int allowLeaf, uint32_t steps, nbx_params *best,
     for (const Trial &tr : trials) {
       nbx_params p = start;
       p.leaf_capacity = tr.leaf;
-      p.force_blocks = tr.grid;
       p.force_block = tr.threads;
       p.leaf_pairs = tr.pairs;
       h->params = p;
       sync_params(h);
+      const int perSm = force_blocks_per_sm(h->base, p.exact_math != 0, p.use_mlp,
+                                            forces_unclamped(h), p.force_block,
+                                            p.leaf_pairs != 0);
+      p.force_blocks = tr.halves ? std::max(1, sms * perSm * tr.halves / 2) : 0;
+      h->params = p;
       destroy_graphs(h);
       restore();
       if ((rc = nbx_step(h, 1)) != NBX_OK) break;

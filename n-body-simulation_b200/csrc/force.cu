@@ -1540,6 +1540,20 @@ void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool gro
   if (order) k_query_scatter<<<blocks, 256, 0, s>>>(sorted, vals, nq, points);
 }
 
+// Blocks of launch_forces' kernel that an SM holds, by the kernels' launch bounds.
+int force_blocks_per_sm(const DevState &S, bool exact, int corr, bool noClamp, int threads,
+                        bool pairs) {
+  const bool fits = group_walk_fits(S);
+  if (corr == 0 && !exact && noClamp) {
+    const bool groups = pairs && fits && group_walk_pays(S);
+    if (threads == 0) threads = groups ? 128 : 256;
+    return std::max(1, (groups ? kGroupWarpsPerSM * 32 : pairs ? 1536 : 2048) / threads);
+  }
+  if (S.n <= kOrderedGroupsMax && fits && ((corr == 0 && exact) || (corr == 2 && noClamp)))
+    return kGroupWarpsPerSM * 32 / 128;
+  return corr == 1 ? 768 / kLearnedBlock : 2048 / kForceBlock;
+}
+
 // chained: the launch follows a kernel of the step's chain on s (chain_begin).
 void launch_forces(cudaStream_t s, const DevState &S, bool exact, int blocks,
                    const MlpDev *mlp, float band, int corr, bool noClamp, int threads,

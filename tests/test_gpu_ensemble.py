@@ -147,3 +147,15 @@ def test_ensemble_step_io(nbx):
         ens.step_io_ptr(pinned.data_ptr(), pinned.data_ptr(), n)
         assert same_bits(hb, expect[k]), k
     ens.close()
+
+
+@pytest.mark.parametrize("n", [10000, 200000])
+def test_autotune_tries_whole_grids(nbx, n):
+    """The block counts tried are none given, or half, one or two times what the
+    GPU's 148 SMs hold at a time: 640 threads an SM in groups, 2048 without."""
+    h = nbx.Handle([n], theta=0.5)
+    h.upload(nbx.uniform_disc(n, 0))
+    best = h.autotune(steps=3)
+    h.close()
+    held = 148 * ((640 if best["leaf_pairs"] else 2048) // best["force_block"])
+    assert best["force_blocks"] in (0, held // 2, held, 2 * held)
