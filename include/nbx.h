@@ -78,11 +78,13 @@ typedef struct nbx_params {
                              src/cuda/CudaNaive.cu:17-57); no tree is built,
                              use_mlp must be 0 */
   int32_t force_block;    /* threads per block of the default force walk:
-                             128, 256 or 512 (0 = 128) */
+                             128, 256 or 512 (0: 128 where it walks in groups,
+                             else 256) */
   int32_t leaf_pairs;     /* default force walk: 1 walks the tree once per
-                             group of 32 bodies and sums the group's terms
-                             with paired FP32 instructions, 0 one record and
-                             one body at a time (default 1); the same terms
+                             group of 32 bodies where such groups fit and pay
+                             (else with a cursor per body) and sums with
+                             paired FP32 instructions, 0 one record and one
+                             body at a time (default 1); the same terms
                              either way, summed in another order */
 } nbx_params;
 

@@ -9,15 +9,15 @@
 // The default force pass walks the tree once per group of 32 bodies over
 // records of four children (walk_group), and so do queries, and exact
 // arithmetic and the quadrupole term of few bodies.  Many of those, the
-// learned correction (walk_learned), the clamped law, counting and whatever
-// does not fit a group's scratch keep a cursor per lane (walk_targets), so that
-// a body's terms are summed in the reference's order: along a lane's walk of the depth-first preorder layout (build.cu)
-// the position only increases (descend = +1, skip = +subtree size), so the
-// warp always serves the smallest position any lane is waiting at.  The
-// node's record is read once per warp (one broadcast load through L1;
-// staging 32-node tiles in shared memory measured 9-11% slower for the extra
-// per-iteration bookkeeping); a leaf's bodies are staged in shared memory
-// with one coalesced load.
+// learned correction (walk_learned), the clamped law, counting, short walks of many
+// bodies (group_walk_pays), uneven states (k_forces_deep) and whatever does not
+// fit a group's scratch keep a cursor per lane (walk_targets, walk_plain_x2): along
+// a lane's walk of the depth-first preorder layout (build.cu) the position only
+// increases (descend = +1, skip = +subtree size), so the warp always serves the
+// smallest position any lane is waiting at.  The node's record is read once
+// per warp (one broadcast load through L1; staging 32-node tiles in shared memory
+// measured 9-11% slower for the extra per-iteration bookkeeping); a leaf's bodies
+// are staged in shared memory with one coalesced load.
 //
 // kExact = true evaluates every float operation as the reference writes
 // it (no FMA contraction, IEEE reciprocal): the result is bit-identical to
@@ -506,6 +506,7 @@ struct alignas(16) WalkStage {
   };
   uint8_t batch[kSlots];             // first slot of each batch
 };
+static_assert(sizeof(WalkStage) == 9520, "20 warps: 190 KB of an SM's 228");
 static_assert(kSlots <= 256 && kSlots * 4 < 1024 && kPairs < 4096 && kPairs <= kTerms,
               "packed fields");
 constexpr uint32_t kItemLeaf = 1024u;

@@ -692,10 +692,10 @@ void sort_fix_low_bits32(cudaStream_t s, SortScratch &sc, int buf, uint32_t n,
   uint32_t b = (n + 255) / 256;
   if (b > 148u * 16u) b = 148u * 16u;
   CodeLow lk{codes};
-  launch_after(s, k_fix_runs32<decltype(lk)>, b, 256, 0, keys32(sc, buf), sc.vals[buf], n, lk, false, 0u, longRuns,
-                                 runCount, cap, err);
-  launch_after(s, k_long_runs32<decltype(lk)>, 148, 256, 0, keys32(sc, buf), sc.vals[buf], keys32(sc, buf ^ 1),
-                                     sc.vals[buf ^ 1], n, lk, longRuns, runCount, cap);
+  launch_after(s, k_fix_runs32<decltype(lk)>, b, 256, 0, keys32(sc, buf), sc.vals[buf], n, lk,
+               false, 0u, longRuns, runCount, cap, err);
+  launch_after(s, k_long_runs32<decltype(lk)>, 148, 256, 0, keys32(sc, buf), sc.vals[buf],
+               keys32(sc, buf ^ 1), sc.vals[buf ^ 1], n, lk, longRuns, runCount, cap);
 }
 
 void sort_fix_units(cudaStream_t s, SortScratch &sc, int buf, uint32_t n, const float4 *box,
@@ -706,10 +706,10 @@ void sort_fix_units(cudaStream_t s, SortScratch &sc, int buf, uint32_t n, const 
   uint32_t b = (n + 255) / 256;
   if (b > 148u * 16u) b = 148u * 16u;
   BoxMinX lk{box};
-  launch_after(s, k_fix_runs32<decltype(lk)>, b, 256, 0, keys32(sc, buf), sc.vals[buf], n, lk, true, skip, longRuns,
-                                 runCount, cap, err);
-  launch_after(s, k_long_runs32<decltype(lk)>, 148, 256, 0, keys32(sc, buf), sc.vals[buf], keys32(sc, buf ^ 1),
-                                     sc.vals[buf ^ 1], n, lk, longRuns, runCount, cap);
+  launch_after(s, k_fix_runs32<decltype(lk)>, b, 256, 0, keys32(sc, buf), sc.vals[buf], n, lk,
+               true, skip, longRuns, runCount, cap, err);
+  launch_after(s, k_long_runs32<decltype(lk)>, 148, 256, 0, keys32(sc, buf), sc.vals[buf],
+               keys32(sc, buf ^ 1), sc.vals[buf ^ 1], n, lk, longRuns, runCount, cap);
 }
 
 size_t sort_tiles(uint32_t n_max) {
