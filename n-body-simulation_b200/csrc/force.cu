@@ -1441,8 +1441,11 @@ bool group_walk_fits(const DevState &S) {
 // 340 / 388, theta 0.85 360 / 374, 342 / 374, 284 / 359; 2^22 theta 0.7 of the disc
 // 1732 / 1663.  Smaller leaves make longer walks: the disc, 200,000, theta 1, leaf
 // capacity 1 123 / 100, 4 94 / 82, 8 84 / 78, 32 73 / 79, 64 85 / 98.
+// In nbx_step_io (recOut) they are taken all the same: the pass hides behind the
+// copies, and the first range ends sooner (2^20 bodies of two discs, theta 1: 2016 /
+// 1976 us a call).
 bool group_walk_pays(const DevState &S) {
-  return S.nGroups <= 148u * kGroupWarpsPerSM ||
+  return S.nGroups <= 148u * kGroupWarpsPerSM || S.recOut ||
          sqrtf(S.tSq) <= 0.715f * powf(fmaxf(1048576.0f / (float)S.n, 1.0f), 0.2f) *
                              powf(16.0f / (float)S.leafCapacity, 0.1f);
 }
@@ -1481,10 +1484,13 @@ void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, boo
     blocks = (int)(b ? b : 1);
   }
   if (pairs && groups && S.nGroups > kGateGroups) {
-    launch_groups<kBlock, kPlainWalk, true>(s, S, whole ? 0 : blocks, 0.0f, chained);
+    // Behind the groups in a chain, before them in nbx_step_io's ranges: a
+    // range's records leave when its last kernel ends, and behind the groups that
+    // one waited for room among the other ranges' blocks (2^20 bodies: 44 us a call).
     const uint32_t deep = std::max(1u, (force_targets(S) + kDeepBlock - 1u) / kDeepBlock);
+    if (!chained) k_forces_deep<<<deep, kDeepBlock, 0, s>>>(S, S.tSq, S.eSq);
+    launch_groups<kBlock, kPlainWalk, true>(s, S, whole ? 0 : blocks, 0.0f, chained);
     if (chained) launch_after(s, k_forces_deep, deep, kDeepBlock, 0, S, S.tSq, S.eSq);
-    else k_forces_deep<<<deep, kDeepBlock, 0, s>>>(S, S.tSq, S.eSq);
   } else if (pairs && groups)
     launch_groups<kBlock, kPlainWalk>(s, S, whole ? 0 : blocks, 0.0f, chained);
   else if (pairs)
