@@ -15,10 +15,10 @@ barrier + synchronize on both sides, max over ranks.  With N GPUs each rank
 advances its own replica (the single simulation does not shard), so the
 whole-job value is N x bodies / step time ("scaling": "weak").
 
-e2e: the same metric through the C ABI as a drop-in Simulation::step with a
-host-owned body array (nbx_step_io, the call the drop-in makes): per step
-the 36-byte Body records go host -> device (pinned), one step runs, and they
-come back device -> host, the copy back overlapped with the force pass's
+e2e: the same metric through the C ABI with a host-owned body array
+(nbx_step_io, the call the drop-in Simulation::step makes; here on pinned
+memory, as a program has that pins its vector): per step the 36-byte Body
+records go host -> device, one step runs, and they come back device -> host, the copy back overlapped with the force pass's
 later target ranges.  The same loop through three calls (upload, step,
 download) is reported beside it.
 

@@ -301,7 +301,7 @@ struct nbx_handle {
   struct {
     uint32_t hostCap = 0, cap = 0;
     float2 *host = nullptr; // points, then accelerations
-    float2 *dev = nullptr;  // [2][cap]: points, then sums; sorted, then their sums
+    float2 *dev = nullptr;  // [2][cap]: sorted, then their sums; points, then sums
     SortScratch sort;       // in dev's allocation
   } qs;
   // splat renderer buffers, grown on demand
@@ -2195,7 +2195,7 @@ static int query_grow(nbx_handle *h, uint32_t n) {
     return at;
   };
   const size_t words = n * sizeof(uint32_t);
-  const size_t points = next(2 * (size_t)n * sizeof(float2));
+  const size_t points = next((2 * (size_t)n + 1) * sizeof(float2));
   const size_t keys[2] = {next(words), next(words)}, vals[2] = {next(words), next(words)};
   const size_t hist = next(8 * 256 * sizeof(uint32_t)), tiles = next(8 * sizeof(uint32_t));
   const size_t status = next(3 * sort_pass_words(n) * sizeof(uint32_t));
@@ -2236,22 +2236,24 @@ int nbx_accel_at(nbx_handle *h, const float *px, const float *py, uint32_t nq,
     // step's sort scratch are free between calls: every user of the pinned
     // staging synchronises, the device's is used in stream order.  They take 8
     // bytes a point and 16, and what is beyond takes the handle's own buffers
+    const size_t back = n + (n > kQueryUnsorted ? 1 : 0); // the status behind the sums
     float2 *host = reinterpret_cast<float2 *>(h->hPinned);
-    float2 *dev = reinterpret_cast<float2 *>(h->dAoS);
+    float2 *sorted = reinterpret_cast<float2 *>(h->dAoS);
     SortScratch *sort = &h->sort;
     size_t cap = n;
     int rc = NBX_OK;
-    if (n > (uint64_t)h->n * sizeof(nbx_body) / sizeof(float2)) {
-      rc = query_grow_host(h, n);
+    if (back > (uint64_t)h->n * sizeof(nbx_body) / sizeof(float2)) {
+      rc = query_grow_host(h, (uint32_t)back);
       host = h->qs.host;
     }
     if (rc == NBX_OK && n > std::min<uint64_t>((uint64_t)h->n * 2, h->sort.capacity)) {
       rc = query_grow(h, n);
-      dev = h->qs.dev;
+      sorted = h->qs.dev;
       sort = &h->qs.sort;
       cap = h->qs.cap;
     }
     if (rc != NBX_OK) return rc;
+    float2 *dev = sorted + cap;
     // into the staging, with the points' box and whether the clamp-free law
     // may be used at them
     const float lim = h->coordLimit;
@@ -2272,15 +2274,16 @@ int nbx_accel_at(nbx_handle *h, const float *px, const float *py, uint32_t nq,
     NBX_CUDA(h, cudaMemcpyAsync(dev, host, n * sizeof(float2), cudaMemcpyHostToDevice,
                                 h->stream));
     launch_query_forces(h->stream, h->state(), h->params.exact_math != 0,
-                        inside && forces_unclamped(h), *sort, dev, n, box, dev + cap);
+                        inside && forces_unclamped(h), *sort, dev, n, box, sorted);
     NBX_CUDA(h, cudaGetLastError());
-    NBX_CUDA(h, cudaMemcpyAsync(host, dev, n * sizeof(float2), cudaMemcpyDeviceToHost,
+    NBX_CUDA(h, cudaMemcpyAsync(host, dev, back * sizeof(float2), cudaMemcpyDeviceToHost,
                                 h->stream));
-    // the waits of the points' sort may have given up
-    NBX_CUDA(h, cudaMemcpyAsync(h->hWord, h->base.status, sizeof(uint32_t),
-                                cudaMemcpyDeviceToHost, h->stream));
     NBX_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (*h->hWord & kStatusSpinLimit) return check_status(h);
+    if (back > n) { // the waits of the points' sort may have given up
+      uint32_t status;
+      std::memcpy(&status, host + n, sizeof(status));
+      if (status & kStatusSpinLimit) return check_status(h);
+    }
     for (uint32_t i = 0; i < n; ++i) {
       ax[at + i] = host[i].x;
       ay[at + i] = host[i].y;

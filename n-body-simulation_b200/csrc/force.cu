@@ -1342,7 +1342,9 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// to[i] = from[order[i]], and back: to[order[i]] = from[i].
+// to[i] = from[order[i]], and back: to[order[i]] = from[i], with the status that
+// the sort may have raised behind the last place (one copy takes both to the
+// host: a copy of its own 3 us a call).
 __global__ void __launch_bounds__(256)
     k_query_gather(const float2 *__restrict__ from, const uint32_t *__restrict__ order,
                    uint32_t n, float2 *__restrict__ to) {
@@ -1351,8 +1353,9 @@ __global__ void __launch_bounds__(256)
 }
 __global__ void __launch_bounds__(256)
     k_query_scatter(const float2 *__restrict__ from, const uint32_t *__restrict__ order,
-                    uint32_t n, float2 *__restrict__ to) {
+                    uint32_t n, const uint32_t *status, float2 *__restrict__ to) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) to[n] = make_float2(__uint_as_float(*status), 0.0f);
   if (i < n && order[i] < n) to[order[i]] = from[i]; // defensive bound
 }
 
@@ -1455,7 +1458,7 @@ bool group_walk_pays(const DevState &S) {
 // bodies and 8 at 2^20 (force pass 618 -> 624).  Plummer's density, us without
 // groups / with, without k_forces_deep / with it: 60,000 bodies theta 0.4 213 / 274 /
 // 216; 2^20 theta 0.5 1239 / 2040 / 1221, 2^22 5242 / 10210 / 5138; a cusp (density as
-// r^-1.8): 100,000 theta 0.5 432 / 480 / 433, 2^20 1660 / 1700 / 1652.
+// r^-1.6): 100,000 theta 0.5 432 / 480 / 433, 2^20 1660 / 1700 / 1652.
 constexpr uint32_t kGateGroups = 1024;
 
 template <int kBlock, GroupWalk kWalk, bool kGated = false>
@@ -1501,7 +1504,8 @@ void launch_plain(cudaStream_t s, const DevState &S, int blocks, bool pairs, boo
 
 // Accelerations at nq arbitrary points from instance 0's last tree
 // (QuadTree::acceleration, QuadTree.cpp:264-389, for any query position):
-// points -> their sums, in place, through the scratch array sorted.  A target's
+// points -> their sums, in place, through the scratch array sorted; beyond
+// kQueryUnsorted points the status follows the sums (k_query_scatter).  A target's
 // sums do not depend on its warp, so the points are first put in Morton order
 // of their box [x0, y0, 1 / cell sizes]: neighbours share a warp and its
 // walk.  groups: the clamp-free law may be used (every point within the
@@ -1516,7 +1520,7 @@ void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool gro
                          SortScratch &sort, float2 *points, uint32_t nq, const float box[4],
                          float2 *sorted) {
   const uint32_t blocks = (nq + 255) / 256;
-  const bool order = nq > 64; // fewer are a warp or two anyway
+  const bool order = nq > kQueryUnsorted;
   const uint32_t *vals = nullptr;
   float2 *query = points; // each target's point, then its sums
   if (order) {
@@ -1544,7 +1548,7 @@ void launch_query_forces(cudaStream_t s, const DevState &S, bool exact, bool gro
     else
       k_forces<false><<<b, kForceBlock, 0, s>>>(S, S.tSq, S.eSq, nullptr, 0.0f, query, nq);
   }
-  if (order) k_query_scatter<<<blocks, 256, 0, s>>>(sorted, vals, nq, points);
+  if (order) k_query_scatter<<<blocks, 256, 0, s>>>(sorted, vals, nq, S.status, points);
 }
 
 // Blocks of launch_forces' kernel that an SM holds, by the kernels' launch bounds.

@@ -209,6 +209,9 @@ struct DevState {
   float4 *attr;
 };
 
+// Points of nbx_accel_at that are not sorted first: a warp or two anyway.
+constexpr uint32_t kQueryUnsorted = 64;
+
 // Camera and draw settings of the splat renderer (render.cu).
 struct RenderParams {
   float camX, camY, scale, halfW, halfH;
@@ -262,7 +265,7 @@ __device__ __forceinline__ uint64_t body_code(float4 p, const MortonFrame &f) {
 
 // Depth of a leaf beyond which the group walk (force.cu) hardly ever fits its
 // scratch: a walk opens about as many records at every level.  Leaf depths at which half
-// the groups fit, theta 0.4 / 0.45 / 0.5 / 0.6: a cusp (density as r^-1.8) 11 / 13
+// the groups fit, theta 0.4 / 0.45 / 0.5 / 0.6: a cusp (density as r^-1.6) 11 / 13
 // / 16 / 19, Plummer's density 14 / 16 / 17 to 18 / over 20; bodies spread evenly lie
 // at depth 9 (2^20) or 10 (2^22).
 __device__ __forceinline__ int walk_depth(float tSq) {

@@ -63,19 +63,22 @@ def test_remainders_of_a_tree(nbx, sizes, form):
     h.close()
 
 
-@pytest.mark.parametrize("nq", [1, 64, 65, 5000])
+@pytest.mark.parametrize("nq", [1, 64, 65, 600, 601, 5000])
 def test_points_after_an_expired_wait(nbx, nq):
-    """Accelerations at points, sorted or not, are not handed out as good when a
-    wait gave up, and are good again after the next build."""
-    b = nbx.cold_square(1000, 1)
+    """Accelerations at points that were sorted (more than 64) are not handed out as
+    good when a wait gave up; of fewer the status stays for the next call that
+    reports it.  All are good again after the next build."""
+    b = nbx.cold_square(300, 1)
     p = np.random.default_rng(nq).uniform(-60, 60, (2, nq)).astype(np.float32)
-    h = nbx.Handle([1000])
+    h = nbx.Handle([300])
     h.upload(b)
     h.phase("build")
     want = h.accel_at(p[0], p[1])
     h._c(nbx.lib().nbx_debug_expire_wait(h.h))
     with pytest.raises(nbx.NbxError) as e:
         h.accel_at(p[0], p[1])
+        assert nq <= 64
+        h.sync()
     assert e.value.code == TIMEOUT
     h.upload(b)
     h.phase("build")
