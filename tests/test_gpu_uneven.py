@@ -95,3 +95,27 @@ def test_groups_that_do_not_pay(nbx):
     b["px"] = np.random.default_rng(1).uniform(-3e3, 3e3, n)
     b["py"], b["radius"] = 0.0, 1e-3
     assert force_ms(nbx, [b], theta=1.3) < 1.5 * force_ms(nbx, [b], theta=1.3, leaf_pairs=0)
+
+
+@pytest.mark.parametrize("n,theta", [(40000, 0.5), (300001, 0.5), (300001, 1.0)])
+def test_every_kind_of_step(nbx, n, theta):
+    """Plain, timed and host-body steps (whose force pass runs in ranges, without the
+    step's chain of launches) of a cusp give the same bits."""
+    import torch
+    b = system(nbx, "cusp", n)
+    got = []
+    for kind in ("step", "step_timed", "io"):
+        h = nbx.Handle([n], theta=theta, collisions=0, dt=1e-4)
+        h.upload(b)
+        if kind == "io":
+            buf = torch.empty((n, 9), dtype=torch.float32, pin_memory=True)
+            out = buf.numpy().view(np.uint8).reshape(-1).view(b.dtype)
+            out[:] = b
+            for _ in range(2):
+                h.step_io_ptr(buf.data_ptr(), buf.data_ptr(), n)
+            got.append(out.copy())
+        else:
+            getattr(h, kind)(2)
+            got.append(h.download())
+        h.close()
+    assert same_bits(got[0], got[1]) and same_bits(got[0], got[2])
