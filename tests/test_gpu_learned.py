@@ -100,3 +100,41 @@ def test_sums_do_not_depend_on_the_warp(nbx, first, n):
         got.append(h.download()[-n:])
         h.close()
     assert same_bits(got[0]["ax"], got[1]["ax"]) and same_bits(got[0]["ay"], got[1]["ay"])
+
+
+@pytest.mark.parametrize("n", [1, 33, 3001])
+@pytest.mark.parametrize("theta,band", [(0.7, 0.7), (0.7, 1.5), (1.0, 1.0)])
+def test_a_band_that_no_accepted_cell_reaches(nbx, oracle, n, theta, band):
+    b = nbx.cold_square(n, 3)
+    _, _, _, sb, tree = oracle.morton_build(b, 16)
+    want, size, doubt = constant_forces(sb, tree, theta, band)
+    w = np.zeros(1442, F)
+    w[B3:] = T0, T1
+    sim = nbx.Simulation(b, theta=theta, use_mlp=1, mlp_band=band)
+    sim.mlp_set_params(w)
+    sim.phase("attract")
+    g = sim.download()
+    sim.set_params(mlp_band=band * 100)
+    sim.phase("attract")
+    far = sim.download()
+    sim.close()
+    # as in test_corrected_cells
+    tol = (n + 16) * 2.0 ** -24 * size + doubt + 1e-30
+    err = np.hypot(g["ax"] - want[:, 0], g["ay"] - want[:, 1])
+    assert (err <= tol).all(), (err / tol).max()
+    assert same_bits(far["ax"], g["ax"]) and same_bits(far["ay"], g["ay"])
+
+
+def test_no_rounds_without_corrections(nbx):
+    """With no cell in the band the pass costs no more than a walk (the rounds with
+    a few rows took 1.1 times as long as with none)."""
+    ms = []
+    for band in (0.7, 0.69):
+        h = nbx.Handle([1 << 20], theta=0.7, use_mlp=1, mlp_band=band, collisions=0, dt=1e-6)
+        h.mlp_set_params(np.zeros(1442, F))
+        h.upload(nbx.uniform_disc(1 << 20, 0))
+        h.step(2)
+        h.sync()
+        ms.append(np.median([h.profile_step()["forces"] for _ in range(6)][1:]))
+        h.close()
+    assert ms[0] < 0.8 * ms[1]
