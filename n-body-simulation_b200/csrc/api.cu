@@ -348,17 +348,18 @@ int cuda_fail(nbx_handle *h, cudaError_t e, const char *what) {
   } while (0)
 
 // Where a piece of `bytes` goes in the handle's one device allocation, `used`
-// bytes of which are taken: large pieces start on 2 MB as allocations of their
-// own would (with all of them packed at 256 bytes the ordered resolution of
-// the collapsed cold square, 2^22 bodies after 1990 steps, took 26.5 ms instead
-// of 24.7), the others on 256 bytes.
-constexpr size_t kArenaLarge = 2u << 20;
+// bytes of which are taken: pieces of 64 MB and more start on 2 MB as allocations
+// of their own would (with all of them packed at 256 bytes the ordered resolution of
+// the collapsed cold square, 2^22 bodies after 1990 steps, took 26.5 ms instead of
+// 24.8), the others on 256 bytes (from 2 MB on on 2 MB the step of two discs of 2^20
+// takes 0.4% more).
+constexpr size_t kArenaLarge = 64u << 20, kArenaAlign = 2u << 20;
 constexpr size_t arena_place(size_t used, size_t bytes) {
-  const size_t align = bytes >= kArenaLarge ? kArenaLarge : 256;
+  const size_t align = bytes >= kArenaLarge ? kArenaAlign : 256;
   return (used + align - 1) & ~(align - 1);
 }
-static_assert(arena_place(1, kArenaLarge) == kArenaLarge && arena_place(257, 4) == 512 &&
-                  arena_place(3 * kArenaLarge, kArenaLarge) == 3 * kArenaLarge,
+static_assert(arena_place(1, kArenaLarge) == kArenaAlign && arena_place(257, 4) == 512 &&
+                  arena_place(3 * kArenaAlign, kArenaLarge) == 3 * kArenaAlign,
               "large pieces on 2 MB");
 
 // The next piece: allocate() lays the pieces out twice, first to add up their
